@@ -65,8 +65,9 @@ typedef struct tbfs_options {
                                   the barrier that ends level k-1, so the
                                   others' bounded waits expire and the call
                                   returns TBFS_ERR_TIMEOUT; 0 = off          */
-  float alpha;               /* TD->BU when frontier edges > unexplored/alpha */
-  float beta;                /* BU->TD when frontier size < n/beta           */
+  float alpha;               /* bottom-up when frontier edges > unexplored/alpha
+                                (with path counts: alpha * 0.35)             */
+  float beta;                /* no BU->TD while frontier size > n/beta       */
   void *stream;              /* cudaStream_t; NULL = legacy default stream   */
   int64_t timeout_ns;        /* grid-barrier wait budget; <=0 = 2 s          */
   /* Per-level trace (host memory, may be NULL): record d holds
@@ -75,15 +76,14 @@ typedef struct tbfs_options {
    *  0, -1} closes the run.  Capacity counts records (4 int64 each). */
   int64_t *level_trace;
   int32_t level_trace_cap;
-  /* Path counts of a level found bottom-up are finished one level later,
-   * either by pulling over that level's lists or by pushing from the
-   * previous level's lists; pull is used unless it reads more than
-   * pull_ratio times as many list entries as push.  <= 0: default 1. */
+  /* Kept for callers that set it; no effect: a bottom-up level counts its
+   * paths in the pass that finds it. */
   float pull_ratio;
   /* Engine shape of the single-source traversal (tbfs_autotune sets both):
    * the most list entries a lane handles per round of a push or pull (1..6;
-   * 0 = 6), and CTAs per SM of the persistent launch (0 = as many as fit,
-   * or 2 on graphs whose out-lists all have at most 16 entries). */
+   * 0 = 6), and units of 256 threads per SM of the persistent launch (1..4;
+   * 0 = 3, 4 on large graphs regrouped by degree, 2 on graphs whose out-lists
+   * all have at most 16 entries). */
   int32_t max_ept;
   int32_t ctas_per_sm;
 } tbfs_options;
@@ -99,9 +99,7 @@ typedef struct tbfs_stats {
 } tbfs_stats;
 
 /* Defaults: AUTO, want_sigma = 1, host outputs, alpha = 15, beta = 2,
- * pull_ratio = 1 (near the best of RMAT scale 18-22 and Erdos-Renyi scale 22
- * with path counts; Beamer's beta = 18 kept bottom-up levels after the
- * frontier had begun to shrink, 14-43 % slower on those graphs). */
+ * pull_ratio = 1. */
 void tbfs_options_init(tbfs_options *opt);
 
 /* Upload a CSC adjacency (col_ptr[n+1], row_idx[nnz], int32, 0-based).
@@ -274,7 +272,7 @@ tbfs_status tbfs_graph_degree_stats(tbfs_graph *g, int32_t kind, tbfs_degree_sta
                                     int64_t *dist, int64_t dist_cap);
 
 /* Autotuner: picks the single-source engine's shape (max_ept, ctas_per_sm)
- * and then alpha, beta and pull_ratio for g by timing traversals from the k
+ * and then alpha and beta for g by timing traversals from the k
  * sample roots (device events; the shape over a small grid at opt's
  * direction parameters, then every combination of a grid of those at the
  * chosen shape) and writes them into *opt, leaving its other fields as they

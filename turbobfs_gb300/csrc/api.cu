@@ -111,7 +111,9 @@ static void graph_free(tbfs_graph *g) {
   tbfs::dev_free(g->cp);
   tbfs::dev_free(g->ic);
   tbfs::dev_free(g->queues);
-  tbfs::dev_free(g->hot); /* bitmaps, S_work, sigma_work */
+  tbfs::dev_free(g->hot); /* sigma_odd, sigma_work, S_work, bitmaps */
+  tbfs::dev_free(g->hubs);
+  tbfs::dev_free(g->tile);
   tbfs::dev_free(g->inv);
   tbfs::dev_free(g->perm);
   tbfs::dev_free(g->ctl);
@@ -149,18 +151,20 @@ static tbfs_status need_device() {
 /* allocations shared by both constructors, after cp/ic/rp/jr are set */
 static tbfs_status graph_finish(tbfs_graph *g) {
   const size_t n = (size_t)g->n;
-  CUDA_TRY(tbfs::dev_alloc(&g->queues, 9 * n * sizeof(int)));
+  CUDA_TRY(tbfs::dev_alloc(&g->queues, 6 * n * sizeof(int)));
   /* the arrays the traversal gathers from at random -- path counts, depths,
    * frontier bitmaps -- in one block */
-  const size_t sig_b = g->inv ? n * sizeof(unsigned long long) : 0;
+  const size_t odd_b = (n * sizeof(unsigned long long) + 255) / 256 * 256;
+  const size_t sig_b = g->inv ? odd_b : 0;
   const size_t S_b = g->inv ? (n * sizeof(int) + 255) / 256 * 256 : 0;
-  const size_t bm_b = 4 * ((n + 31) / 32) * sizeof(unsigned);
-  CUDA_TRY(tbfs::dev_alloc(&g->hot, sig_b + S_b + bm_b));
+  const size_t bm_b = 3 * ((n + 31) / 32) * sizeof(unsigned);
+  CUDA_TRY(tbfs::dev_alloc(&g->hot, odd_b + sig_b + S_b + bm_b));
+  g->sigma_odd = reinterpret_cast<unsigned long long *>(g->hot);
   if (g->inv) {
-    g->sigma_work = reinterpret_cast<unsigned long long *>(g->hot);
-    g->S_work = reinterpret_cast<int *>(g->hot + sig_b);
+    g->sigma_work = reinterpret_cast<unsigned long long *>(g->hot + odd_b);
+    g->S_work = reinterpret_cast<int *>(g->hot + odd_b + sig_b);
   }
-  g->bitmaps = reinterpret_cast<unsigned *>(g->hot + sig_b + S_b);
+  g->bitmaps = reinterpret_cast<unsigned *>(g->hot + odd_b + sig_b + S_b);
   CUDA_TRY(tbfs::dev_alloc(&g->ctl, sizeof(BfsCtl)));
   CUDA_TRY(cudaMallocHost(&g->ctl_host, sizeof(BfsCtl)));
   memset(g->ctl_host, 0, sizeof(BfsCtl));
@@ -181,6 +185,12 @@ static tbfs_status graph_finish(tbfs_graph *g) {
       if (e != cudaSuccess) return cuda_fail(e, "out-degree bound", __LINE__);
     }
     g->short_lists = max_out <= tbfs::kShortList;
+    CUDA_TRY(tbfs::dev_alloc(&g->tile, ((size_t)tbfs::tile_count(g->n, g->nnz) + 1) * sizeof(int)));
+    CUDA_TRY(tbfs::fill_tiles(g->cp, g->n, g->nnz, g->tile, 0));
+    if (maxd > tbfs::kHubLen) {
+      CUDA_TRY(tbfs::dev_alloc(&g->hubs, (2 + tbfs::hub_segments_cap(g->nnz)) * sizeof(int)));
+      CUDA_TRY(tbfs::hub_segments(g->cp, g->n, g->hubs, g->hubs + 2, 0));
+    }
   }
   return TBFS_OK;
 }
@@ -661,12 +671,18 @@ static BfsParams make_params(tbfs_graph *g, int32_t root, const tbfs_options &o,
   p.sigma_out = o.want_sigma ? sigma : nullptr;
   p.S = g->inv ? g->S_work : S;
   p.sigma = o.want_sigma ? (g->inv ? g->sigma_work : sigma) : nullptr;
-  for (int b = 0; b < 3; ++b) {
+  p.sigma_odd = g->sigma_odd;
+  for (int b = 0; b < 2; ++b) {
     p.q[b] = g->queues + (size_t)(0 + b) * g->n;
-    p.e[b] = g->queues + (size_t)(3 + b) * g->n;
-    p.a[b] = g->queues + (size_t)(6 + b) * g->n;
+    p.e[b] = g->queues + (size_t)(2 + b) * g->n;
+    p.a[b] = g->queues + (size_t)(4 + b) * g->n;
   }
-  for (int b = 0; b < 4; ++b) p.fb[b] = g->bitmaps + (size_t)b * ((g->n + 31) / 32);
+  p.hub_count = g->hubs;
+  p.hub_seg = g->hubs ? g->hubs + 2 : nullptr;
+  p.tile = g->tile;
+  p.nnz = g->nnz;
+  p.hub_len = g->hubs ? (unsigned)tbfs::kHubLen : ~0u;
+  for (int b = 0; b < 3; ++b) p.fb[b] = g->bitmaps + (size_t)b * ((g->n + 31) / 32);
   p.ctl = g->ctl;
   p.out_edges_total = g->out_edges_total;
   p.timeout_ns = o.timeout_ns > 0 ? o.timeout_ns : 2000000000LL;
@@ -676,7 +692,6 @@ static BfsParams make_params(tbfs_graph *g, int32_t root, const tbfs_options &o,
   p.symmetric = g->separate_out ? 0 : 1;
   p.alpha = o.alpha;
   p.beta = o.beta;
-  p.pull_ratio = o.pull_ratio;
   p.inject_barrier_skip = o.inject_barrier_skip > 0 ? o.inject_barrier_skip : 0;
   p.trace = nullptr;
   p.trace_cap = 0;

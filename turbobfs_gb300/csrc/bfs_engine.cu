@@ -15,21 +15,26 @@
  * F_{d+1} either
  *   top-down : edge-balanced push over the out-edges of F_d; an unvisited
  *              target is claimed with atomicCAS(S, -1, d+1) and appended to
- *              the next queue, or
- *   bottom-up: every unvisited vertex scans its in-list and stops at the
- *              first in-neighbour with S == d (early exit).
+ *              the next queue, and (with path counts) every edge that lands
+ *              on a vertex at depth d+1 adds sigma[u] to it; or
+ *   bottom-up: every unvisited vertex scans its in-list.  Depths only: it
+ *              stops at the first in-neighbour in F_d (frontier bitmap).
+ *              With path counts: it sums its in-neighbours' counts, which
+ *              discovers and counts in one pass (pull_item).
  *
  * Path counts.  sigma[v] = sum of sigma[u] over the entries u->v with
- * S[u] = S[v]-1 (each such entry is a "parent edge").  The engine computes
- * sigma(F_{d+1}) wherever it is cheapest:
- *   - during a top-down discovery from F_d whose counts are final: every
- *     parent edge of F_{d+1} is examined by the push anyway, so each edge
- *     that lands on a vertex claimed at depth d+1 adds sigma[u] to it
- *     (no extra list reads);
- *   - otherwise (F_{d+1} was found bottom-up, which stops early) in the next
- *     phase, by either pulling over the lists of F_{d+1} or pushing from the
- *     lists of F_d -- whichever frontier has fewer edges.  The three most
- *     recent queues are kept, so F_d is still available then.
+ * S[u] = S[v]-1.  The counts of even and odd depths are kept in two arrays,
+ * both zero where nothing was counted.  An in-neighbour of a vertex still
+ * unvisited in phase d has depth d, or is unvisited itself: nothing above
+ * level d can reach it first.  So the sum over ALL in-neighbours of the array
+ * of d's parity is exactly the sum over the parents (a neighbour found in
+ * this phase is counted in the other array), and it is nonzero exactly when
+ * the vertex has a parent: a bottom-up level needs one gather per list entry
+ * and no frontier test.  This holds while no count has wrapped to zero; once
+ * an overflow is recorded the parents are found by their depth instead.
+ * Before, a bottom-up level stopped at the first parent and the next phase
+ * read the lists again for the counts (a push of 52 M entries with 40 M L2
+ * reductions on RMAT-22's heaviest level).
  * Counts are exact in uint64 arithmetic; any sum that reaches 2^63 sets
  * ctl->sigma_overflow (overflow is reported, never rounded).
  *
@@ -40,15 +45,16 @@
  * every lane handles kEPT consecutive edges per round, so that many list
  * reads, then that many depth gathers, are in flight per lane.  On graphs
  * whose out-lists are all short (kShortList entries at most) the kernel
- * instance bfs_persistent_kernel<true> cuts small top-down levels into
+ * instances bfs_persistent_kernel<true, .> cut small top-down levels into
  * items of kShortEntries whole queue entries instead, which need no owner
  * search (the chain of dependent L2 round trips is what a small level
  * costs); other graphs run the instance compiled without that path.
  *
- * Direction rule (device side; Beamer, Asanovic, Patterson, "Direction-
- * optimizing breadth-first search", SC 2012): leave top-down when the
- * frontier's out-edges exceed (unexplored edges)/alpha; return to top-down
- * when the frontier shrinks below n/beta.  The comparisons are in fp32:
+ * Direction rule (device side; after Beamer, Asanovic, Patterson,
+ * "Direction-optimizing breadth-first search", SC 2012): a level runs
+ * bottom-up when alpha times the frontier's out-edges exceed the unexplored
+ * edges plus the cost of visiting every vertex's word; a frontier of more
+ * than n/beta vertices does not leave bottom-up.  The comparisons are in fp32:
  * every thread evaluates them at every level, and fp64 issues slowly on
  * this part (in fp64 they cost about 0.7 us per level).
  *
@@ -70,36 +76,21 @@
 #ifndef TBFS_EPT
 #define TBFS_EPT 6
 #endif
-#ifndef TBFS_BLOCK
-#define TBFS_BLOCK 256
-#endif
-#ifndef TBFS_MIN_BLOCKS
-#define TBFS_MIN_BLOCKS 4 /* 4 CTAs of 256 per SM: 64 registers (a small spill) */
-#endif
-#ifndef TBFS_SHORT_LEVELS
-#define TBFS_SHORT_LEVELS 1 /* small top-down levels of short-list graphs: items of whole queue entries */
-#endif
 #ifndef TBFS_SHORT_CAS_FIRST
 #define TBFS_SHORT_CAS_FIRST 1 /* aligned items claim with the CAS alone */
 #endif
-#ifndef TBFS_SPREAD_ITEMS
-#define TBFS_SPREAD_ITEMS 1 /* static work items round-robin over the CTAs */
-#endif
-#ifndef TBFS_RED_PUSH
-#define TBFS_RED_PUSH 1 /* pushes without the overflow check where a bound rules overflow out */
-#endif
-
 namespace tbfs {
 namespace {
 
 using dev::FULL;
 using dev::add_chk;
-using dev::smem_add_split;
 using dev::global_ns;
 using dev::grid_barrier;
 using dev::warp_find_owner;
-constexpr int kBlock = TBFS_BLOCK;
-constexpr int kWarps = kBlock / 32;
+constexpr int kBlock = 1024;       /* threads of a full CTA, one CTA per SM */
+constexpr long long kLargeEntries = 48 << 20;
+constexpr int kBlockStep = 256;    /* threads per unit of ctas_per_sm */
+constexpr int kFilterBits = 1 << 18; /* frontier filter in shared memory (32 KB) */
 constexpr int kWin = 128;          /* queue entries staged per warp window */
 constexpr int kEPT = TBFS_EPT;     /* most consecutive edges per lane/round */
 /* queue entries per item of a small level of a short-list graph: at most
@@ -108,18 +99,28 @@ constexpr unsigned kShortEntries = 8;
 constexpr float kBuWordCost = 4.0f; /* a bitmap word of a bottom-up level, in list entries */
 enum { DIR_TD = 0, DIR_BU = 1 };
 
-/* what an expansion does with path counts */
-enum SigMode {
-  SIG_NONE = 0,     /* depths only                                          */
-  SIG_PULL = 1,     /* entries gather sigma from neighbours at depth d-1    */
-  SIG_PUSH_NEW = 2, /* entries add their sigma to targets claimed at d+1    */
-  SIG_PUSH_AT = 3   /* entries add their sigma to targets at depth `tgt`    */
-};
+/* A bottom-up level with path counts scans every unvisited vertex's whole
+ * list where one without stops at the first parent, so it must beat the push
+ * by more: alpha is scaled by this (15 -> 5.25).  RMAT-22, a level of 21.3 M
+ * out-edges with 107 M unexplored: top-down 417 us, bottom-up 301; of 9.9 M
+ * with 118 M: top-down 247. */
+constexpr float kSigmaAlpha = 0.35f;
+/* unexplored entries from which a bottom-up level with path counts is cut
+ * into items of equal cost (a few hundred entries per warp) ... */
+constexpr float kHeavyEntries = 3e5f;
+constexpr float kHeavyShare = 0.25f; /* ... and of all entries: else words of
+                                        visited hubs make most of the items */
+/* entries per frontier vertex from which a frontier filter pays: every CTA
+ * reads the whole queue to fill its own */
+constexpr float kFilterGain = 300.0f;
+/* what leaving bottom-up costs a traversal with path counts besides a pass over
+ * the depths (a barrier and the round trips around it), in list entries */
+constexpr float kLeaveCost = 4e5f;
 
-struct WarpWin {
-  /* PULL: accumulator of the entry; PUSH: the entry's sigma -- as low and
-   * high words in separate arrays, so that neighbouring entries fall in
-   * different banks */
+/* Shared memory of a warp that expands: a window of queue entries. */
+struct ExpandWin {
+  /* sigma of the entry as low and high words in separate arrays, so that
+   * neighbouring entries fall in different banks */
   unsigned lo[kWin], hi[kWin];
   int v[kWin];                  /* vertex of the entry                      */
   int a[kWin];                  /* list index of its first window edge      */
@@ -190,19 +191,17 @@ __device__ __forceinline__ bool bit_of(const unsigned *bm, int v) {
   return (bm[(unsigned)v >> 5] >> ((unsigned)v & 31u)) & 1u;
 }
 
-/* One warp expands the flattened out-edge range [E0, E1) of queue Q.
- * DISC: claim unvisited targets at depth d+1 into `nx` (and bitmap nb).
- * SIG: see SigMode (PULL is valid only when in-lists == out-lists; the push
- * modes walk the out-lists, which hold exactly the parent edges of their
- * targets).  Without DISC, membership of a neighbour in the level the mode
- * needs (d-1 for PULL, tgt for PUSH_AT) is read from bitmap tb, one bit per
- * vertex, instead of from S. */
-template <bool DISC, int SIG, bool CHK = true, bool ALIGNED = false>
-__device__ __forceinline__ void expand_chunk(const BfsParams &p, int d, int tgt, const Queue &Q,
+/* One warp expands the flattened out-edge range [E0, E1) of queue Q: claims
+ * unvisited targets at depth d+1 into `nx` (depths only: and bitmap nb).
+ * SIG: every edge whose target is at depth d+1 afterwards adds its source's
+ * count (src) to the target's (dst); CHK: each add is checked for overflow. */
+template <bool SIG, bool CHK = true, bool ALIGNED = false>
+__device__ __forceinline__ void expand_chunk(const BfsParams &p, int d, const Queue &Q,
                                              unsigned E0, unsigned E1, unsigned ept,
-                                             const NextQueue &nx, const unsigned *tb,
-                                             unsigned *nb, WarpWin &w, bool &ovf,
-                                             unsigned first = 0, unsigned count = 0) {
+                                             const NextQueue &nx,
+                                             const unsigned long long *src,
+                                             unsigned long long *dst, unsigned *nb, ExpandWin &w,
+                                             bool &ovf, unsigned first = 0, unsigned count = 0) {
   const int lane = threadIdx.x & 31;
   /* ALIGNED item: entries [first, first + count), all their edges, one
    * window; E0 = 0 and E1 = ~0u, so the window offsets below are the
@@ -222,12 +221,8 @@ __device__ __forceinline__ void expand_chunk(const BfsParams &p, int d, int tgt,
       w.v[k] = v;
       w.a[k] = __ldcg(Q.a + i) + (int)(b - eb);
       w.s[k] = bc - pos;
-      if (SIG == SIG_PULL) {
-        w.lo[k] = 0u;
-        w.hi[k] = 0u;
-      }
-      if ((SIG == SIG_PUSH_NEW || SIG == SIG_PUSH_AT) && !aligned) {
-        const unsigned long long x = p.sigma[v];
+      if (SIG && !aligned) {
+        const unsigned long long x = src[v];
         w.lo[k] = (unsigned)x;
         w.hi[k] = (unsigned)(x >> 32);
       }
@@ -280,17 +275,16 @@ __device__ __forceinline__ void expand_chunk(const BfsParams &p, int d, int tgt,
       /* an aligned item reads its entries' path counts with the list
        * entries instead of staging them first: one round trip fewer */
       unsigned long long xs[kEPT];
-      if (aligned && SIG == SIG_PUSH_NEW) {
+      if (aligned && SIG) {
 #pragma unroll
-        for (int j = 0; j < kEPT; ++j) xs[j] = ((valid >> j) & 1u) ? p.sigma[w.v[kk[j]]] : 0ull;
+        for (int j = 0; j < kEPT; ++j) xs[j] = ((valid >> j) & 1u) ? src[w.v[kk[j]]] : 0ull;
       }
-      int su[kEPT];   /* DISC: depth of the neighbour                        */
-      unsigned in = 0; /* bit j: neighbour j is in the level the sigma mode needs */
+      int su[kEPT]; /* depth of the target */
       /* an aligned item may claim with the CAS alone: its return value is
        * the depth the plain read would have given */
       constexpr bool cas_first = aligned && TBFS_SHORT_CAS_FIRST;
       int ad[kEPT], dg[kEPT];
-      if (DISC && cas_first) {
+      if (cas_first) {
 #pragma unroll
         for (int j = 0; j < kEPT; ++j) {
           su[j] = -2;
@@ -302,100 +296,57 @@ __device__ __forceinline__ void expand_chunk(const BfsParams &p, int d, int tgt,
             dg[j] = __ldg(p.rp + u[j] + 1) - ad[j];
           }
         }
-      } else if (DISC) {
+      } else {
 #pragma unroll
         for (int j = 0; j < kEPT; ++j) su[j] = ((valid >> j) & 1u) ? p.S[u[j]] : -2;
-        if (SIG == SIG_PULL) {
+      }
+      unsigned hit = 0; /* targets at depth d+1 after this edge */
+      unsigned take = 0;
+      if (cas_first) {
 #pragma unroll
-          for (int j = 0; j < kEPT; ++j)
-            if (su[j] == d - 1) in |= 1u << j;
+        for (int j = 0; j < kEPT; ++j) {
+          if (su[j] == -1) take |= 1u << j;
+          else if (su[j] == d + 1) hit |= 1u << j;
         }
       } else {
-        unsigned wd[kEPT];
 #pragma unroll
         for (int j = 0; j < kEPT; ++j) {
-          su[j] = -2;
-          wd[j] = ((valid >> j) & 1u) ? tb[(unsigned)u[j] >> 5] : 0u;
+          if (su[j] == -1) {
+            const int old = atomicCAS(p.S + u[j], -1, d + 1);
+            if (old == -1) take |= 1u << j;
+            else if (old == d + 1) hit |= 1u << j;
+          } else if (su[j] == d + 1) {
+            hit |= 1u << j;
+          }
         }
-#pragma unroll
-        for (int j = 0; j < kEPT; ++j)
-          if ((wd[j] >> ((unsigned)u[j] & 31u)) & 1u) in |= 1u << j;
       }
-      unsigned hit = 0; /* PUSH_NEW: targets at depth d+1 after this edge */
-      if (DISC) {
-        unsigned take = 0;
-        if (cas_first) {
+      hit |= take;
 #pragma unroll
-          for (int j = 0; j < kEPT; ++j) {
-            if (su[j] == -1) take |= 1u << j;
-            else if (su[j] == d + 1) hit |= 1u << j;
-          }
-        } else {
-#pragma unroll
-          for (int j = 0; j < kEPT; ++j) {
-            if (su[j] == -1) {
-              const int old = atomicCAS(p.S + u[j], -1, d + 1);
-              if (old == -1) take |= 1u << j;
-              else if (old == d + 1) hit |= 1u << j;
-            } else if (su[j] == d + 1) {
-              hit |= 1u << j;
-            }
-          }
+      for (int j = 0; j < kEPT; ++j) {
+        if (!cas_first) {
+          ad[j] = 0;
+          dg[j] = 0;
         }
-        hit |= take;
-#pragma unroll
-        for (int j = 0; j < kEPT; ++j) {
+        if ((take >> j) & 1u) {
           if (!cas_first) {
-            ad[j] = 0;
-            dg[j] = 0;
+            ad[j] = __ldg(p.rp + u[j]);
+            dg[j] = __ldg(p.rp + u[j] + 1) - ad[j];
           }
-          if ((take >> j) & 1u) {
-            if (!cas_first) {
-              ad[j] = __ldg(p.rp + u[j]);
-              dg[j] = __ldg(p.rp + u[j] + 1) - ad[j];
-            }
-            atomicOr(nb + ((unsigned)u[j] >> 5), 1u << ((unsigned)u[j] & 31u));
-          }
+          if (!SIG) atomicOr(nb + ((unsigned)u[j] >> 5), 1u << ((unsigned)u[j] & 31u));
         }
-        warp_append<kEPT>(take, u, dg, ad, nx.q, nx.e, nx.a, nx.ctr);
       }
-      if (SIG == SIG_PUSH_NEW || SIG == SIG_PUSH_AT) {
+      warp_append<kEPT>(take, u, dg, ad, nx.q, nx.e, nx.a, nx.ctr);
+      if (SIG) {
 #pragma unroll
         for (int j = 0; j < kEPT; ++j) {
-          const bool add = SIG == SIG_PUSH_NEW ? ((hit >> j) & 1u) != 0 : ((in >> j) & 1u) != 0;
-          if (add) {
+          if ((hit >> j) & 1u) {
             const unsigned long long x =
-                aligned && SIG == SIG_PUSH_NEW
-                    ? xs[j]
-                    : ((unsigned long long)w.hi[kk[j]] << 32) | (unsigned long long)w.lo[kk[j]];
-            if (CHK) add_chk(atomicAdd(p.sigma + u[j], x), x, ovf);
-            else atomicAdd(p.sigma + u[j], x); /* result unused: a reduction, no round trip */
+                aligned ? xs[j]
+                        : ((unsigned long long)w.hi[kk[j]] << 32) | (unsigned long long)w.lo[kk[j]];
+            if (CHK) add_chk(atomicAdd(dst + u[j], x), x, ovf);
+            else atomicAdd(dst + u[j], x); /* result unused: a reduction, no round trip */
           }
         }
-      }
-      if (SIG == SIG_PULL) {
-        unsigned long long c[kEPT]; /* path counts of the parents only */
-#pragma unroll
-        for (int j = 0; j < kEPT; ++j) c[j] = ((in >> j) & 1u) ? p.sigma[u[j]] : 0ull;
-        unsigned long long run = 0;
-        int rk = kk[0];
-#pragma unroll
-        for (int j = 0; j < kEPT; ++j) {
-          if (kk[j] != rk) {
-            if (run) smem_add_split(&w.lo[rk], &w.hi[rk], run, ovf);
-            rk = kk[j];
-            run = 0;
-          }
-          run = add_chk(run, c[j], ovf);
-        }
-        if (run) smem_add_split(&w.lo[rk], &w.hi[rk], run, ovf);
-      }
-    }
-    __syncwarp();
-    if (SIG == SIG_PULL) {
-      for (unsigned k = lane; k < nw; k += 32) {
-        const unsigned long long x = ((unsigned long long)w.hi[k] << 32) | (unsigned long long)w.lo[k];
-        if (x) add_chk(atomicAdd(p.sigma + w.v[k], x), x, ovf);
       }
     }
     __syncwarp();
@@ -428,86 +379,439 @@ __device__ __forceinline__ ExpandPlan plan_expand(unsigned qe, unsigned nwarps, 
   return pl;
 }
 
-/* the expansions a phase can run (template instances of expand_chunk) */
-enum ExpandKind {
-  EX_NONE = 0,
-  EX_DISC = 1,          /* discovery, depths only                 */
-  EX_DISC_PUSH_NEW = 2, /* discovery + counts pushed to new targets */
-  EX_DISC_PULL = 3,     /* discovery + counts of the entries pulled */
-  EX_PUSH_AT = 4,       /* counts pushed to targets at depth tgt    */
-  EX_PULL = 5           /* counts of the entries pulled             */
-};
-
+/* a top-down level: queue, how it is cut, where its counts come from and go */
 struct ExpandTask {
-  int kind, tgt;
   Queue Q;
-  const unsigned *tb;
   ExpandPlan pl;
-  bool chk; /* pushes check every add for overflow */
+  const unsigned long long *src;
+  unsigned long long *dst;
+  bool chk;                /* check every add for overflow */
 };
 
+template <bool SIG>
 __device__ __forceinline__ void run_expand_item(const BfsParams &p, int d, const ExpandTask &t,
                                                 unsigned c, const NextQueue &nx, unsigned *nb,
-                                                WarpWin &w, bool &ovf) {
+                                                ExpandWin &w, bool &ovf) {
   const unsigned E0 = c * t.pl.ch;
   const unsigned E1 = E0 + t.pl.ch < t.Q.qe ? E0 + t.pl.ch : t.Q.qe;
-  switch (t.kind) {
-    case EX_DISC:
-      expand_chunk<true, SIG_NONE>(p, d, t.tgt, t.Q, E0, E1, t.pl.ept, nx, t.tb, nb, w, ovf);
-      break;
-    case EX_DISC_PUSH_NEW:
-      if (t.chk)
-        expand_chunk<true, SIG_PUSH_NEW>(p, d, t.tgt, t.Q, E0, E1, t.pl.ept, nx, t.tb, nb, w, ovf);
-      else
-        expand_chunk<true, SIG_PUSH_NEW, false>(p, d, t.tgt, t.Q, E0, E1, t.pl.ept, nx, t.tb, nb,
-                                                w, ovf);
-      break;
-    case EX_DISC_PULL:
-      expand_chunk<true, SIG_PULL>(p, d, t.tgt, t.Q, E0, E1, t.pl.ept, nx, t.tb, nb, w, ovf);
-      break;
-    case EX_PUSH_AT:
-      if (t.chk)
-        expand_chunk<false, SIG_PUSH_AT>(p, d, t.tgt, t.Q, E0, E1, t.pl.ept, nx, t.tb, nb, w, ovf);
-      else
-        expand_chunk<false, SIG_PUSH_AT, false>(p, d, t.tgt, t.Q, E0, E1, t.pl.ept, nx, t.tb, nb,
-                                                w, ovf);
-      break;
-    case EX_PULL:
-      expand_chunk<false, SIG_PULL>(p, d, t.tgt, t.Q, E0, E1, t.pl.ept, nx, t.tb, nb, w, ovf);
-      break;
-    default:
-      break;
-  }
+  if (!SIG || t.chk)
+    expand_chunk<SIG>(p, d, t.Q, E0, E1, t.pl.ept, nx, t.src, t.dst, nb, w, ovf);
+  else
+    expand_chunk<SIG, false>(p, d, t.Q, E0, E1, t.pl.ept, nx, t.src, t.dst, nb, w, ovf);
 }
 
 /* One item of a small top-down level of a short-list graph: queue entries
  * [first, first + kShortEntries) with all their edges (ALIGNED expand_chunk:
  * no owner search). */
-__device__ __forceinline__ void run_short_item(const BfsParams &p, int d, const ExpandTask &t, unsigned first,
-                    unsigned max_ept, const NextQueue &nx, unsigned *nb, WarpWin &w, bool &ovf) {
+template <bool SIG>
+__device__ __forceinline__ void run_short_item(const BfsParams &p, int d, const ExpandTask &t,
+                                               unsigned first, unsigned max_ept,
+                                               const NextQueue &nx, unsigned *nb, ExpandWin &w,
+                                               bool &ovf) {
   const unsigned ept = max_ept < 4u ? max_ept : 4u;
-  if (t.kind == EX_DISC)
-    expand_chunk<true, SIG_NONE, true, true>(p, d, 0, t.Q, 0u, ~0u, ept, nx, t.tb, nb, w, ovf,
-                                             first, kShortEntries);
-  else if (t.chk)
-    expand_chunk<true, SIG_PUSH_NEW, true, true>(p, d, 0, t.Q, 0u, ~0u, ept, nx, t.tb, nb, w,
-                                                 ovf, first, kShortEntries);
+  if (!SIG || t.chk)
+    expand_chunk<SIG, true, true>(p, d, t.Q, 0u, ~0u, ept, nx, t.src, t.dst, nb, w, ovf, first,
+                                  kShortEntries);
   else
-    expand_chunk<true, SIG_PUSH_NEW, false, true>(p, d, 0, t.Q, 0u, ~0u, ept, nx, t.tb, nb, w,
-                                                  ovf, first, kShortEntries);
+    expand_chunk<SIG, false, true>(p, d, t.Q, 0u, ~0u, ept, nx, t.src, t.dst, nb, w, ovf, first,
+                                   kShortEntries);
 }
 
-/* Bottom-up discovery.  A warp takes kBuWords consecutive 32-vertex words
- * per iteration; lane i owns vertex 32*word+i of each, so the depth checks,
+/* ---- bottom-up levels ----
+ * With path counts, a bottom-up level only counts what it finds (per lane, added up once per
+ * warp at the end of the phase): a following bottom-up level needs no queue,
+ * and a top-down one collects it from the depths (collect_queue).  Appending
+ * during the level, and one work counter for items of two words, cost two
+ * atomics on one address per 64 vertices, which L2 takes at ~0.75 G/s: 84 us
+ * for a level of RMAT-22 with next to nothing to do. */
+struct Found {
+  unsigned n, e; /* vertices, their out-edges */
+};
+
+/* 32-vertex words a warp looks at together */
+constexpr int kBuWords = 8;
+
+/* queue of level d from the depths */
+constexpr int kCollectWords = 8;
+__device__ __forceinline__ void collect_queue(const BfsParams &p, int d, int *q, int *e, int *a,
+                                              unsigned warp, unsigned nwarps) {
+  const unsigned lane = threadIdx.x & 31, nwords = ((unsigned)p.n + 31u) >> 5;
+  for (unsigned word = warp * kCollectWords; word < nwords; word += nwarps * kCollectWords) {
+    int v[kCollectWords], dg[kCollectWords], ad[kCollectWords];
+    unsigned take = 0;
+#pragma unroll
+    for (int j = 0; j < kCollectWords; ++j) {
+      v[j] = (int)((word + j) * 32u + lane);
+      if (v[j] < p.n && p.S[v[j]] == d) take |= 1u << j;
+    }
+    if (!__any_sync(FULL, take != 0u)) continue;
+#pragma unroll
+    for (int j = 0; j < kCollectWords; ++j) {
+      dg[j] = ad[j] = 0;
+      if ((take >> j) & 1u) {
+        ad[j] = __ldg(p.rp + v[j]);
+        dg[j] = __ldg(p.rp + v[j] + 1) - ad[j];
+      }
+    }
+    warp_append<kCollectWords>(take, v, dg, ad, q, e, a, &p.ctl->collect);
+  }
+}
+
+/* Where a bottom-up level finds the counts of level d. */
+struct Counts {
+  const unsigned long long *src;
+  /* frontier filter in the CTA's shared memory: bit u % kFilterBits set for
+   * every u in F_d; null where it would not pay */
+  const unsigned *filter;
+  bool by_depth; /* counts may be zero: parents are found by their depth d */
+  int d;
+};
+
+/* exact sum of counts: 64 bits and the carries out of them */
+struct Sum {
+  unsigned lo, hi, c;
+};
+
+__device__ __forceinline__ void sum_add(Sum &s, unsigned lo, unsigned hi, unsigned c) {
+  asm("add.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, %4;\n\taddc.u32 %2, %2, %5;"
+      : "+r"(s.lo), "+r"(s.hi), "+r"(s.c)
+      : "r"(lo), "r"(hi), "r"(c));
+}
+
+/* Entries [lo, hi) of a list by the whole warp: the exact sum of their counts,
+ * and whether there is a parent among them. */
+__device__ __forceinline__ void sum_exact(const BfsParams &p, const Counts &c, unsigned lo,
+                                          unsigned hi, Sum &s, bool &par) {
+  s = {0u, 0u, 0u};
+  par = false;
+  for (unsigned k = lo + (threadIdx.x & 31); k < hi; k += 32u) {
+    const int u = __ldg(p.ic + k);
+    const unsigned long long x = c.src[u];
+    sum_add(s, (unsigned)x, (unsigned)(x >> 32), 0u);
+    if (c.by_depth && p.S[u] == c.d) par = true;
+  }
+  __syncwarp();
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned l = __shfl_xor_sync(FULL, s.lo, o), h = __shfl_xor_sync(FULL, s.hi, o);
+    const unsigned y = __shfl_xor_sync(FULL, s.c, o);
+    sum_add(s, l, h, y);
+  }
+  par = c.by_depth ? __any_sync(FULL, par) : (s.lo | s.hi | s.c) != 0u;
+}
+
+/* Fast sums keep 32 bits: exact while every count is below 2^20 (a list they
+ * are used for has at most kHubLen entries); `big` collects the other bits, and
+ * a list that shows any is summed again exactly. */
+constexpr unsigned kBigCount = ~((1u << 20) - 1u);
+static_assert(kHubLen <= 1 << 12, "fast sums must fit 32 bits");
+
+/* the counts of u[0..U) (-1: none) as 32 bits; big collects the other bits */
+template <bool FILTER, int U>
+__device__ __forceinline__ void get_fast(const Counts &c, const int (&u)[U], unsigned (&y)[U],
+                                         unsigned &big) {
+  unsigned long long x[U];
+  bool on[U];
+#pragma unroll
+  for (int j = 0; j < U; ++j) on[j] = u[j] >= 0;
+  if (FILTER) {
+    unsigned f[U];
+#pragma unroll
+    for (int j = 0; j < U; ++j) f[j] = c.filter[((unsigned)u[j] >> 5) & (kFilterBits / 32u - 1u)];
+#pragma unroll
+    for (int j = 0; j < U; ++j) on[j] = on[j] && (__funnelshift_r(f[j], f[j], (unsigned)u[j]) & 1u);
+  }
+#pragma unroll
+  for (int j = 0; j < U; ++j) {
+    x[j] = 0ull;
+    if (on[j]) x[j] = c.src[u[j]];
+  }
+#pragma unroll
+  for (int j = 0; j < U; ++j) {
+    y[j] = (unsigned)x[j];
+    big |= (unsigned)(x[j] >> 32) | (y[j] & kBigCount);
+  }
+}
+
+template <bool FILTER, int U>
+__device__ __forceinline__ void add_fast(const Counts &c, const int (&u)[U], unsigned &acc,
+                                         unsigned &big) {
+  unsigned y[U];
+  get_fast<FILTER, U>(c, u, y, big);
+#pragma unroll
+  for (int j = 0; j < U; ++j) acc += y[j];
+}
+
+/* Bottom-up discovery with path counts over the vertices [v_lo, v_hi), in
+ * groups of 128 (four to a lane), by the length of an unvisited vertex's list:
+ * the lane reads up to kOwn entries alone, two of each of its four lists a
+ * step; 8 lanes read a list of up to kHalf, the next lists' entries
+ * requested before these entries' counts arrive; the whole warp reads a longer
+ * one, one pass ahead.  Lists over p.hub_len are left to pull_segment.
+ * What bounds a level is latency (a list entry from DRAM and a count from L2
+ * are each 700-1500 cycles away with 8 warps per scheduler) and, next to it,
+ * instructions.  RMAT-22's heaviest level (76.6 M entries; 5 % in lists of up to
+ * 8 entries, 20 % up to 32, 70 % over 64) took 1150 us with groups of one
+ * width by the mean length (three quarters of the lanes idle), 376 with the
+ * lists laid end to end (100 instructions per 32 entries to find an entry's
+ * list and split the sums), 300-355 with 96-bit sums and lists sorted by
+ * length in shared memory, 300 word by word without the lookahead, 252 so
+ * (against 75 for an early-exit scan and 324 for a push of the counts after
+ * it). */
+constexpr unsigned kOwn = 8, kHalf = 48;
+constexpr int kWords = 4; /* words of a group */
+static_assert(kWords * 32 <= kWin, "a group's vertices must fit the window");
+
+template <bool FILTER>
+__device__ __forceinline__ void pull_range(const BfsParams &p, Found &fd, const Counts &c,
+                                           unsigned long long *dst, int v_lo, int v_hi,
+                                           ExpandWin &w, bool &ovf) {
+  const unsigned lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
+  for (; v_lo < v_hi; v_lo += 32 * kWords) {
+    unsigned lo[kWords], hi[kWords]; /* lists the lane reads alone; else hi = lo */
+    unsigned mids = 0u, longs = 0u, other = 0u, on = 0u;
+    {
+#pragma unroll
+      for (int j = 0; j < kWords; ++j) {
+        const int v = v_lo + 32 * j + (int)lane;
+        if (v < v_hi && p.S[v] == -1) on |= 1u << j;
+      }
+#pragma unroll
+      for (int j = 0; j < kWords; ++j) {
+        const int v = v_lo + 32 * j + (int)lane;
+        lo[j] = hi[j] = 0u;
+        if ((on >> j) & 1u) {
+          lo[j] = (unsigned)__ldg(p.cp + v);
+          hi[j] = (unsigned)__ldg(p.cp + v + 1);
+        }
+      }
+      bool any = false;
+#pragma unroll
+      for (int j = 0; j < kWords; ++j) {
+        unsigned len = hi[j] - lo[j];
+        if (len > p.hub_len) len = 0u;
+        if (len == 0u) {
+          hi[j] = lo[j];
+          on &= ~(1u << j);
+        }
+        any |= len != 0u;
+        /* to the window: the lists for 8 lanes from the front of v[], those
+         * for a warp from its back, both by slot; bounds in lo[], hi[] */
+        const bool exact = c.by_depth || len > (unsigned)kHubLen;
+        const bool is_l = len > kHalf && !exact, is_m = len > kOwn && len <= kHalf && !exact;
+        const unsigned mm = __ballot_sync(FULL, is_m), ml = __ballot_sync(FULL, is_l);
+        if (((on >> j) & 1u) && (len > kOwn || exact)) {
+          other |= 1u << j;
+          w.lo[32 * j + lane] = lo[j];
+          w.hi[32 * j + lane] = hi[j];
+          w.s[32 * j + lane] = 0u;
+          w.a[32 * j + lane] = exact ? 1 : 0; /* big */
+          if (is_m) w.v[mids + __popc(mm & lt)] = 32 * j + (int)lane;
+          if (is_l) w.v[kWin - 1u - longs - __popc(ml & lt)] = 32 * j + (int)lane;
+          hi[j] = lo[j];
+        }
+        mids += __popc(mm);
+        longs += __popc(ml);
+      }
+      if (!__any_sync(FULL, any)) continue;
+    }
+    __syncwarp();
+    if (longs) {
+      /* passes of 128 entries, requested one ahead */
+      unsigned i = kWin - longs, k = 0u; /* next request: list, first entry */
+      auto request = [&](int (&u)[4], int &slot, bool &last) {
+        slot = -1;
+        if (i >= (unsigned)kWin) return;
+        slot = w.v[i];
+        const unsigned b = w.lo[slot] + k, e = w.hi[slot];
+        const int *a = p.ic + b + lane;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) u[j] = b + lane + 32u * j < e ? __ldg(a + 32 * j) : -1;
+        k += 128u;
+        last = b + 128u >= e;
+        if (last) {
+          ++i;
+          k = 0u;
+        }
+      };
+      int u0[4], u1[4], s0, s1;
+      bool l0 = false, l1 = false;
+      request(u0, s0, l0);
+      unsigned a = 0u, b = 0u;
+      while (s0 >= 0) {
+        request(u1, s1, l1);
+        add_fast<FILTER, 4>(c, u0, a, b);
+        if (l0) {
+          a = __reduce_add_sync(FULL, a);
+          b = __reduce_or_sync(FULL, b);
+          if (lane == 0) {
+            w.s[s0] = a;
+            w.a[s0] = (int)b;
+          }
+          a = b = 0u;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) u0[j] = u1[j];
+        s0 = s1;
+        l0 = l1;
+      }
+    }
+    if (mids) {
+      constexpr int U = kHalf / 8;
+      int u[U], t[U];
+      auto request = [&](unsigned i) {
+        i += lane >> 3;
+        const int slot = w.v[i < mids ? i : 0u];
+        const unsigned b = w.lo[slot] + (lane & 7u), e = i < mids ? w.hi[slot] : 0u;
+        const int *a = p.ic + b;
+#pragma unroll
+        for (int j = 0; j < U; ++j) u[j] = b + 8u * j < e ? __ldg(a + 8 * j) : -1;
+      };
+      request(0u);
+      for (unsigned i = 0u; i < mids; i += 4u) {
+#pragma unroll
+        for (int j = 0; j < U; ++j) t[j] = u[j];
+        if (i + 4u < mids) request(i + 4u);
+        unsigned a = 0u, b = 0u;
+        add_fast<FILTER, U>(c, t, a, b);
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) {
+          a += __shfl_xor_sync(FULL, a, o);
+          b |= __shfl_xor_sync(FULL, b, o);
+        }
+        if ((lane & 7u) == 0u && i + (lane >> 3) < mids) {
+          const int slot = w.v[i + (lane >> 3)];
+          w.s[slot] = a;
+          w.a[slot] = (int)b;
+        }
+      }
+    }
+    unsigned acc[kWords], big = 0u; /* big: bit j for the lane's list j */
+    unsigned most = 0u;
+#pragma unroll
+    for (int j = 0; j < kWords; ++j) {
+      acc[j] = 0u;
+      const unsigned n = hi[j] - lo[j];
+      most = most > n ? most : n;
+    }
+    most = __reduce_max_sync(FULL, most);
+    for (unsigned t = 0u; t < most; t += 2u) {
+      int u[2 * kWords];
+#pragma unroll
+      for (int j = 0; j < kWords; ++j) {
+        const unsigned k = lo[j] + t;
+        u[2 * j] = k < hi[j] ? __ldg(p.ic + k) : -1;
+        u[2 * j + 1] = k + 1u < hi[j] ? __ldg(p.ic + k + 1u) : -1;
+      }
+      unsigned b = 0u, x[2 * kWords];
+      get_fast<FILTER, 2 * kWords>(c, u, x, b);
+#pragma unroll
+      for (int j = 0; j < kWords; ++j) acc[j] += x[2 * j] + x[2 * j + 1];
+      if (b) big = ~0u; /* any of the lane's: all its lists again */
+    }
+    __syncwarp();
+    /* vertices with a parent: depth and count */
+#pragma unroll
+    for (int j = 0; j < kWords; ++j) {
+      const int v = v_lo + 32 * j + (int)lane;
+      const bool here = (on >> j) & 1u;
+      unsigned b = lo[j], e = hi[j], x = acc[j], s_hi = 0u;
+      bool redo = here && big != 0u;
+      if ((other >> j) & 1u) {
+        b = w.lo[32 * j + lane];
+        e = w.hi[32 * j + lane];
+        x = w.s[32 * j + lane];
+        redo = w.a[32 * j + lane] != 0;
+      }
+      bool found = x != 0u;
+      for (unsigned m = __ballot_sync(FULL, redo); m; m &= m - 1u) {
+        const int l = __ffs(m) - 1;
+        Sum s;
+        bool par;
+        sum_exact(p, c, __shfl_sync(FULL, b, l), __shfl_sync(FULL, e, l), s, par);
+        if ((int)lane == l) {
+          x = s.lo;
+          s_hi = s.hi;
+          found = par;
+          if (s.c | (s.hi >> 31)) ovf = true;
+        }
+      }
+      if (here && found) {
+        p.S[v] = c.d + 1;
+        dst[v] = ((unsigned long long)s_hi << 32) | x;
+        fd.n += 1u;
+        fd.e += p.symmetric ? e - b : (unsigned)(__ldg(p.rp + v + 1) - __ldg(p.rp + v));
+      }
+    }
+    __syncwarp();
+  }
+}
+
+/* entries [lo, hi) of the list of v by the whole warp */
+__device__ __forceinline__ void pull_segment(const BfsParams &p, Found &fd, const Counts &c,
+                                             unsigned long long *dst, int v, int lo, int hi,
+                                             bool &ovf) {
+  const unsigned lane = threadIdx.x & 31;
+  unsigned acc = 0u, big = c.by_depth ? 1u : 0u;
+  if (!c.by_depth) {
+    for (unsigned k = (unsigned)lo + lane; k - lane < (unsigned)hi; k += 256u) {
+      int u[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) u[j] = k + 32u * j < (unsigned)hi ? __ldg(p.ic + k + 32 * j) : -1;
+      add_fast<false, 8>(c, u, acc, big);
+    }
+  }
+  Sum s = {__reduce_add_sync(FULL, acc), 0u, 0u};
+  bool par = s.lo != 0u;
+  if (__any_sync(FULL, big != 0u)) sum_exact(p, c, (unsigned)lo, (unsigned)hi, s, par);
+  if (lane == 0 && par) {
+    const unsigned long long x = ((unsigned long long)s.hi << 32) | s.lo;
+    add_chk(atomicAdd(dst + v, x), x, ovf);
+    if (s.c) ovf = true;
+    if (atomicCAS(p.S + v, -1, c.d + 1) == -1) {
+      fd.n += 1u;
+      fd.e += (unsigned)(__ldg(p.rp + v + 1) - __ldg(p.rp + v));
+    }
+  }
+}
+
+/* The same for 32 segments of the graph's hub list, kHubLen entries of a longer
+ * list each, by the whole warp: i0, i0 + step, ...: neighbours in the list are
+ * mostly of one vertex, so that a warp taking 32 in a row would read a whole
+ * list alone (87 us of a level whose other work took 70).  Segments of a vertex meet
+ * in its count by atomics; the one whose claim of the depth succeeds counts
+ * the vertex as found. */
+__device__ __forceinline__ void pull_segments(const BfsParams &p, Found &fd, const Counts &c,
+                                              unsigned long long *dst, unsigned i0, unsigned step,
+                                              unsigned n_seg, bool &ovf) {
+  const int lane = threadIdx.x & 31;
+  int vs = 0, los = 0, his = 0;
+  bool on = false;
+  const unsigned i = i0 + (unsigned)lane * step;
+  if (i < n_seg) {
+    vs = __ldg(p.hub_seg + 2 * i);
+    los = __ldg(p.hub_seg + 2 * i + 1);
+    const int sv = __ldcg(p.S + vs); /* -1, or d+1 by another segment of this phase */
+    on = sv == -1 || sv == c.d + 1;
+    if (on) his = __ldg(p.cp + vs + 1);
+  }
+  for (unsigned m = __ballot_sync(FULL, on); m; m &= m - 1u) {
+    const int l = __ffs(m) - 1;
+    const int v = __shfl_sync(FULL, vs, l), lo = __shfl_sync(FULL, los, l);
+    const int end = __shfl_sync(FULL, his, l), hi = end - lo < kHubLen ? end : lo + kHubLen;
+    pull_segment(p, fd, c, dst, v, lo, hi, ovf);
+  }
+}
+
+/* Bottom-up discovery, depths only.  A warp takes nw <= kBuWords consecutive
+ * 32-vertex words (fewer on small graphs, so that every warp has some); lane i owns vertex 32*word+i of each, so the depth checks,
  * list bounds and the first gathers of all kBuWords vertices are in flight
  * together.  An unvisited vertex scans its in-list until the first
  * neighbour in F_d (bitmap cb); the scan advances every still-searching
  * vertex of the lane by one entry per step.  The warp owns its words of the
  * next level's bitmap nb and writes them whole. */
-constexpr int kBuWords = 8;
-
-__device__ void bu_tile(const BfsParams &p, int d, const NextQueue &nx, const unsigned *cb,
-                        unsigned *nb, unsigned tile) {
+__device__ __forceinline__ void bu_tile(const BfsParams &p, int d, const NextQueue &nx, const unsigned *cb,
+                        unsigned *nb, unsigned word, unsigned nw) {
   const int lane = threadIdx.x & 31;
   const unsigned nwords = ((unsigned)p.n + 31u) >> 5;
   {
@@ -515,10 +819,10 @@ __device__ void bu_tile(const BfsParams &p, int d, const NextQueue &nx, const un
     unsigned search = 0; /* bit j: vertex j unvisited and still searching */
 #pragma unroll
     for (int j = 0; j < kBuWords; ++j) {
-      v[j] = (int)((tile * kBuWords + j) * 32u + (unsigned)lane);
+      v[j] = (int)((word + j) * 32u + (unsigned)lane);
       k[j] = 0;
       ke[j] = 0;
-      if (v[j] < p.n && p.S[v[j]] == -1) search |= 1u << j;
+      if ((unsigned)j < nw && v[j] < p.n && p.S[v[j]] == -1) search |= 1u << j;
     }
 #pragma unroll
     for (int j = 0; j < kBuWords; ++j)
@@ -561,38 +865,64 @@ __device__ void bu_tile(const BfsParams &p, int d, const NextQueue &nx, const un
     }
 #pragma unroll
     for (int j = 0; j < kBuWords; ++j) {
-      const unsigned word = __ballot_sync(FULL, (found >> j) & 1u);
-      const unsigned wi = tile * kBuWords + j;
-      if (lane == 0 && wi < nwords) nb[wi] = word;
+      const unsigned bits = __ballot_sync(FULL, (found >> j) & 1u);
+      if (lane == 0 && (unsigned)j < nw && word + j < nwords) nb[word + j] = bits;
     }
     warp_append<kBuWords>(found, v, dg, ad, nx.q, nx.e, nx.a, nx.ctr);
   }
 }
 
-template <bool SHORT>
-__global__ void __launch_bounds__(kBlock, TBFS_MIN_BLOCKS) bfs_persistent_kernel(const BfsParams p) {
-  __shared__ WarpWin s_win[kWarps];
-  WarpWin &win = s_win[threadIdx.x >> 5];
+template <bool SHORT, bool SIG>
+__global__ void __launch_bounds__(kBlock, 1) bfs_persistent_kernel(const BfsParams p) {
+  /* a window per warp, then the frontier filter (instance <false, true>) */
+  extern __shared__ __align__(16) unsigned char s_dyn[];
+  ExpandWin *s_win = reinterpret_cast<ExpandWin *>(s_dyn);
+  ExpandWin &win = s_win[threadIdx.x >> 5];
+  unsigned *s_filter =
+      !SHORT && p.filter ? reinterpret_cast<unsigned *>(s_win + (blockDim.x >> 5)) : nullptr;
   const unsigned gtid = blockIdx.x * blockDim.x + threadIdx.x;
   const unsigned nthreads = gridDim.x * blockDim.x;
   const unsigned nwarps = nthreads >> 5;
   BfsCtl *ctl = p.ctl;
-  const bool want_sigma = p.sigma != nullptr;
+  constexpr bool want_sigma = SIG;
   const int root = p.inv ? __ldg(p.inv + p.root) : p.root; /* internal numbering */
 
-  /* init: S = -1, sigma = 0, root at depth 0 with one path; F_0 = {root} in
-   * bitmap 0, the other bitmaps empty */
-  for (unsigned i = gtid; i < (unsigned)p.n; i += nthreads) {
-    p.S[i] = (int)i == root ? 0 : -1;
-    if (want_sigma) p.sigma[i] = (int)i == root ? 1ull : 0ull;
+  /* init: S = -1, counts 0, root at depth 0 with one path; depths only:
+   * F_0 = {root} in bitmap 0, the other bitmaps empty.  With path counts (a
+   * pass over the results ends the traversal) a vertex without in-list is
+   * kNoList until then, so that bottom-up levels need not look at it again:
+   * 43 % of RMAT-22's vertices. */
+  constexpr int kNoList = -2;
+  if (want_sigma) {
+    for (unsigned i0 = gtid; i0 < (unsigned)p.n; i0 += 4u * nthreads) {
+      int len[4];
+#pragma unroll
+      for (unsigned j = 0; j < 4u; ++j) {
+        const unsigned i = i0 + j * nthreads;
+        len[j] = i < (unsigned)p.n ? __ldg(p.cp + i + 1) - __ldg(p.cp + i) : 0;
+      }
+#pragma unroll
+      for (unsigned j = 0; j < 4u; ++j) {
+        const unsigned i = i0 + j * nthreads;
+        if (i < (unsigned)p.n) {
+          p.S[i] = (int)i == root ? 0 : len[j] ? -1 : kNoList;
+          p.sigma[i] = (int)i == root ? 1ull : 0ull;
+          p.sigma_odd[i] = 0ull;
+        }
+      }
+    }
+  } else {
+    for (unsigned i = gtid; i < (unsigned)p.n; i += nthreads) p.S[i] = (int)i == root ? 0 : -1;
   }
   const unsigned nwords = ((unsigned)p.n + 31u) >> 5;
-  for (unsigned i = gtid; i < nwords; i += nthreads) {
-    p.fb[0][i] = i == ((unsigned)root >> 5) ? 1u << ((unsigned)root & 31u) : 0u;
-    p.fb[1][i] = 0u;
-    p.fb[2][i] = 0u;
-    p.fb[3][i] = 0u;
+  if (!want_sigma) {
+    for (unsigned i = gtid; i < nwords; i += nthreads) {
+      p.fb[0][i] = i == ((unsigned)root >> 5) ? 1u << ((unsigned)root & 31u) : 0u;
+      p.fb[1][i] = 0u;
+      p.fb[2][i] = 0u;
+    }
   }
+  const unsigned n_hub = want_sigma && p.hub_count ? (unsigned)__ldg(p.hub_count) : 0u;
   if (gtid == 0) {
     const int a = __ldg(p.rp + root);
     p.q[0][0] = root;
@@ -605,9 +935,8 @@ __global__ void __launch_bounds__(kBlock, TBFS_MIN_BLOCKS) bfs_persistent_kernel
 
   int d = 0, dir = DIR_TD, td = 0, bu = 0;
   long long m_u = p.out_edges_total, visited = 0, edges = 0;
-  unsigned prev_qn = 0, prev_qe = 0;
-  bool ovf = false, sig_ready = true; /* sigma(F_d) final at the start of phase d */
-  bool done = false;
+  const float alpha = want_sigma ? p.alpha * kSigmaAlpha : p.alpha;
+  bool ovf = false, done = false;
   /* Bound on the bits of the path counts of F_d: sigma(F_0) = 1, and a count
    * of F_{d+1} sums at most max-in-degree counts of F_d, so it has at most
    * deg_bits more bits.  Pushes into a level whose bound is at most 63 bits
@@ -618,7 +947,7 @@ __global__ void __launch_bounds__(kBlock, TBFS_MIN_BLOCKS) bfs_persistent_kernel
   for (;;) {
     const unsigned long long cur = __ldcg(&ctl->qctr[d % 3]);
     /* read with the counter, so that both loads are in flight together */
-    const bool ovf_seen = TBFS_RED_PUSH && want_sigma && __ldcg(&ctl->sigma_overflow) != 0;
+    const bool ovf_seen = want_sigma && __ldcg(&ctl->sigma_overflow) != 0;
     const unsigned qn = (unsigned)(cur >> 32);
     const unsigned qe = (unsigned)cur;
     if (qn == 0) {
@@ -631,18 +960,23 @@ __global__ void __launch_bounds__(kBlock, TBFS_MIN_BLOCKS) bfs_persistent_kernel
      * clear it for F_{d+2}, which phase d+1 fills */
     if (gtid == 0) ctl->qctr[(d + 2) % 3] = 0ull;
 
+    m_u -= qe; /* out-edges of the vertices not reached yet */
+    const bool no_queue = want_sigma && dir == DIR_BU; /* F_d has no queue yet */
     if (p.mode == TBFS_MODE_TOP_DOWN) {
       dir = DIR_TD;
     } else if (p.mode == TBFS_MODE_BOTTOM_UP) {
       dir = DIR_BU;
-    } else if (dir == DIR_TD) {
-      /* a bottom-up level also visits every vertex's bitmap word: without
-       * that term, the tail of a deep graph (few unexplored edges left)
-       * switched to bottom-up levels three times as costly as top-down ones */
-      if ((float)qe * p.alpha > (float)m_u + kBuWordCost * (float)nwords) dir = DIR_BU;
-      else m_u -= qe;
-    } else if (qn < prev_qn && (float)qn * p.beta <= (float)p.n) {
-      dir = DIR_TD;
+    } else if ((float)qe * alpha > (float)m_u + kBuWordCost * (float)nwords) {
+      /* a bottom-up level also visits every vertex's word: without that
+       * term, the tail of a deep graph (few unexplored edges left) switched
+       * to bottom-up levels three times as costly as top-down ones */
+      dir = DIR_BU;
+    } else if (dir == DIR_BU) {
+      /* leave when a bottom-up level costs more than the top-down one and
+       * the pass that collects its queue, unless the frontier is large */
+      if ((float)qn * p.beta <= (float)p.n &&
+          (!want_sigma || (float)qe * alpha + kLeaveCost < (float)m_u))
+        dir = DIR_TD;
     }
     if (gtid == 0 && p.trace && d < p.trace_cap - 1) {
       long long *rec = p.trace + 4 * (long long)d;
@@ -652,111 +986,189 @@ __global__ void __launch_bounds__(kBlock, TBFS_MIN_BLOCKS) bfs_persistent_kernel
       rec[3] = dir;
     }
 
-    /* queues of levels d-1, d, d+1 rotate through three buffers */
-    const int bc = d % 3, bn = (d + 1) % 3, bp = (d + 2) % 3;
-    const Queue Qc = {p.q[bc], p.e[bc], p.a[bc], qn, qe};
-    const Queue Qp = {p.q[bp], p.e[bp], p.a[bp], prev_qn, prev_qe};
-    const NextQueue nx = {p.q[bn], p.e[bn], p.a[bn], &ctl->qctr[bn]};
-    /* bitmaps: F_{d-1}, F_d read; F_{d+1} written; F_{d+2}'s cleared (its
-     * previous contents, F_{d-2}, were last read in phase d-1) */
-    const unsigned *bm_prev = p.fb[(d + 3) % 4];
-    const unsigned *bm_cur = p.fb[d % 4];
-    unsigned *bm_next = p.fb[(d + 1) % 4];
-    unsigned *bm_clear = p.fb[(d + 2) % 4];
-    for (unsigned i = gtid; i < nwords; i += nthreads) bm_clear[i] = 0u;
+    const int bc = d & 1, bn = bc ^ 1, b3 = (d + 1) % 3;
+    const NextQueue nx = {p.q[bn], p.e[bn], p.a[bn], &ctl->qctr[b3]};
+    /* depths only -- bitmaps: F_d read; F_{d+1} written; F_{d+2}'s cleared
+     * (its previous contents, F_{d-1}, were last read in phase d-1) */
+    const unsigned *bm_cur = p.fb[d % 3];
+    unsigned *bm_next = p.fb[b3];
+    if (!want_sigma) {
+      unsigned *bm_clear = p.fb[(d + 2) % 3];
+      for (unsigned i = gtid; i < nwords; i += nthreads) bm_clear[i] = 0u;
+    }
+    /* counts of level d and of level d+1 */
+    const unsigned long long *src = bc ? p.sigma_odd : p.sigma;
+    unsigned long long *dst = bc ? p.sigma : p.sigma_odd;
     /* work counter of phase d+2 (last used in phase d-2) */
     if (gtid == 0) ctl->work[(d + 2) & 3] = 0u;
-    bool next_ready = false;
 
-    /* this phase's work: up to two expansions, then bottom-up tiles */
-    ExpandTask A = {EX_NONE, 0, Qc, bm_prev, {1, 1, 0}, true};
-    ExpandTask B = {EX_NONE, 0, Qc, bm_prev, {1, 1, 0}, true};
+    /* this phase's work: an expansion, or hub segments and word tiles */
+    ExpandTask A = {{p.q[bc], p.e[bc], p.a[bc], qn, qe}, {1, 1, 0}, src, dst, false};
+    const unsigned max_ept =
+        p.max_ept > 0 && p.max_ept < kEPT ? (unsigned)p.max_ept : (unsigned)kEPT;
+    unsigned n_seg = 0, n_all = 0, n_static = nwarps, tiles = 0, per_item = 1;
+    const unsigned *filter = nullptr;
+    bool short_level = false, heavy = false;
+    Found fd = {0u, 0u};
     if (dir == DIR_TD) {
       ++td;
-      if (!want_sigma) {
-        A.kind = EX_DISC;
-      } else if (sig_ready) { /* parents final: counts ride on the push */
-        A.kind = EX_DISC_PUSH_NEW;
-        next_ready = true;
-      } else if (p.symmetric) { /* finish sigma(F_d) on the same list reads */
-        A.kind = EX_DISC_PULL;
-      } else { /* sigma(F_d) from F_{d-1}'s out-lists, discovery from F_d */
-        A = {EX_PUSH_AT, d, Qp, bm_cur, {1, 1, 0}, true};
-        B.kind = EX_DISC;
+      if (no_queue) {
+        collect_queue(p, d, p.q[bc], p.e[bc], p.a[bc],
+                      (threadIdx.x >> 5) * gridDim.x + blockIdx.x, nwarps);
+        if (!grid_barrier(ctl, p.timeout_ns, d)) break;
+      }
+      A.chk = want_sigma && !ovf_seen && !(p.deg_bits > 0 && sig_bits + p.deg_bits <= 63);
+      /* a small top-down level of a graph with short lists: items of
+       * kShortEntries queue entries each, no owner search (expand_chunk) and
+       * no edge-chunk plan */
+      short_level = SHORT && qn <= kShortEntries * nwarps;
+      if (!short_level) {
+        A.pl = plan_expand(qe, nwarps, max_ept);
+        n_all = A.pl.nch;
       }
     } else {
       ++bu;
-      if (want_sigma && !sig_ready) { /* sigma(F_d): pull unless push reads far less */
-        if (p.symmetric && (float)qe <= p.pull_ratio * (float)prev_qe)
-          A.kind = EX_PULL;
-        else
-          A = {EX_PUSH_AT, d, Qp, bm_cur, {1, 1, 0}, true};
+      if (gtid == 0) ctl->collect = 0ull;
+      n_seg = (n_hub + 31u) / 32u; /* 32 segments looked at per item */
+      heavy = want_sigma && p.tile && (float)m_u > kHeavyEntries &&
+              (float)m_u > kHeavyShare * (float)p.nnz;
+      if (heavy && s_filter && !no_queue && qn <= kFilterBits / 4u &&
+          (float)m_u > kFilterGain * (float)qn) {
+        filter = s_filter;
+        for (unsigned i = threadIdx.x; i < kFilterBits / 32u; i += blockDim.x) s_filter[i] = 0u;
+        __syncthreads();
+        for (unsigned i = threadIdx.x; i < qn; i += 8u * blockDim.x) {
+          int u[8]; /* eight in flight: every CTA reads the whole queue */
+#pragma unroll
+          for (unsigned j = 0; j < 8u; ++j)
+            u[j] = i + j * blockDim.x < qn ? __ldcg(p.q[bc] + i + j * blockDim.x) : -1;
+#pragma unroll
+          for (unsigned j = 0; j < 8u; ++j)
+            if (u[j] >= 0)
+              atomicOr(s_filter + (((unsigned)u[j] >> 5) & (kFilterBits / 32u - 1u)),
+                       1u << ((unsigned)u[j] & 31u));
+        }
+        __syncthreads();
       }
+      if (heavy) { /* items of equal cost */
+        tiles = (unsigned)(((long long)p.nnz + (long long)kTileVertex * p.n) / kTileCost) + 1u;
+        per_item = tiles / (4u * nwarps);
+        per_item = per_item < 1u ? 1u : (per_item > 8u ? 8u : per_item);
+      } else { /* words, at least one for every warp of a small graph */
+        tiles = nwords;
+        per_item = (nwords + nwarps - 1u) / nwarps;
+        const unsigned most = want_sigma ? (unsigned)kWords : (unsigned)kBuWords;
+        per_item = per_item > most ? most : per_item;
+      }
+      n_all = n_seg + (tiles + per_item - 1u) / per_item;
+      /* even work needs no counter */
+      if (want_sigma && !heavy) n_static = (n_all / nwarps + 1u) * nwarps;
     }
-    const unsigned max_ept =
-        p.max_ept > 0 && p.max_ept < kEPT ? (unsigned)p.max_ept : (unsigned)kEPT;
-    if (TBFS_RED_PUSH && want_sigma) {
-      const int nb_next = sig_bits + p.deg_bits; /* bound of F_{d+1} */
-      if (A.kind == EX_DISC_PUSH_NEW)
-        A.chk = !ovf_seen && !(p.deg_bits > 0 && nb_next <= 63);
-      if (A.kind == EX_PUSH_AT) A.chk = !ovf_seen && !(p.deg_bits > 0 && sig_bits <= 63);
-    }
-    /* a small top-down level of a graph with short lists: items of
-     * kShortEntries queue entries each, no owner search (expand_chunk) and
-     * no edge-chunk plan */
-    const bool short_level = SHORT && B.kind == EX_NONE &&
-                             (A.kind == EX_DISC || A.kind == EX_DISC_PUSH_NEW) &&
-                             qn <= kShortEntries * nwarps;
-    if (!short_level) {
-      if (A.kind != EX_NONE) A.pl = plan_expand(A.Q.qe, nwarps, max_ept);
-      if (B.kind != EX_NONE) B.pl = plan_expand(B.Q.qe, nwarps, max_ept);
-    }
-    const unsigned n_tiles = dir == DIR_BU ? (nwords + kBuWords - 1) / kBuWords : 0u;
-    const unsigned n_a = short_level ? 0u : A.pl.nch;
-    const unsigned n_ab = n_a + B.pl.nch, n_all = n_ab + n_tiles;
+    const Counts C = {src, filter, ovf_seen, d};
     unsigned *wctr = &ctl->work[d & 3];
     const int lane = threadIdx.x & 31;
-    /* work items: the first statically (one per warp), the rest from the
-     * level's counter past the static range, so that a small level costs
-     * no same-address atomics.  Static items go round-robin over the CTAs
-     * (item i to CTA i % grid), so that a small level's work spreads over
-     * as many SMs as it has items instead of filling the first CTAs' warps */
-    unsigned item = TBFS_SPREAD_ITEMS ? (threadIdx.x >> 5) * gridDim.x + blockIdx.x
-                                      : blockIdx.x * kWarps + (threadIdx.x >> 5);
+    /* work items: the first n_static statically (one per warp, or several),
+     * the rest from the level's counter past the static range, so that a
+     * small level costs no same-address atomics.  Static items go round-robin
+     * over the CTAs (item i to CTA i % grid), so that a small level's work
+     * spreads over as many SMs as it has items instead of filling the first
+     * CTAs' warps */
+    unsigned item = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
     if (short_level) {
       const unsigned first = item * kShortEntries;
-      if (first < qn) run_short_item(p, d, A, first, max_ept, nx, bm_next, win, ovf);
+      if (first < qn) run_short_item<SIG>(p, d, A, first, max_ept, nx, bm_next, win, ovf);
     }
     while (item < n_all) {
-      if (item < n_a) run_expand_item(p, d, A, item, nx, bm_next, win, ovf);
-      else if (item < n_ab) run_expand_item(p, d, B, item - n_a, nx, bm_next, win, ovf);
-      else bu_tile(p, d, nx, bm_cur, bm_next, item - n_ab);
-      if (n_all <= nwarps) break;
-      unsigned nxt = 0;
-      if (lane == 0) nxt = nwarps + atomicAdd(wctr, 1u);
-      item = __shfl_sync(FULL, nxt, 0);
+      /* the next item: static, or claimed now and looked at when this one is
+       * done */
+      unsigned nxt = item + nwarps;
+      const bool claim = nxt >= n_static;
+      if (claim && n_all > n_static && lane == 0) nxt = n_static + atomicAdd(wctr, 1u);
+      if (dir == DIR_TD) {
+        run_expand_item<SIG>(p, d, A, item, nx, bm_next, win, ovf);
+      } else if (item < n_seg) {
+        pull_segments(p, fd, C, dst, item, n_seg, n_hub, ovf);
+      } else {
+        const unsigned t = (item - n_seg) * per_item;
+        if constexpr (!SIG) {
+          bu_tile(p, d, nx, bm_cur, bm_next, t, per_item);
+        } else if (heavy) {
+          const int ve = __ldg(p.tile + (t + per_item < tiles ? t + per_item : tiles));
+          if (filter) pull_range<true>(p, fd, C, dst, __ldg(p.tile + t), ve, win, ovf);
+          else pull_range<false>(p, fd, C, dst, __ldg(p.tile + t), ve, win, ovf);
+        } else {
+          const int v = (int)(t * 32u), e = v + 32 * (int)per_item;
+          pull_range<false>(p, fd, C, dst, v, e < p.n ? e : p.n, win, ovf);
+        }
+      }
+      if (claim && n_all <= n_static) break;
+      item = claim ? __shfl_sync(FULL, nxt, 0) : nxt;
     }
-    prev_qn = qn;
-    prev_qe = qe;
+    if (dir == DIR_BU) {
+      const unsigned fn = __reduce_add_sync(FULL, fd.n), fe = __reduce_add_sync(FULL, fd.e);
+      if (lane == 0 && fn) atomicAdd(nx.ctr, ((unsigned long long)fn << 32) | fe);
+    }
     /* test hook: CTA 0 leaves without arriving; the others' waits expire */
     if (p.inject_barrier_skip > 0 && blockIdx.x == 0 && d == p.inject_barrier_skip - 1) return;
-    if (TBFS_RED_PUSH && want_sigma) { /* overflow recorded now: seen by every CTA after the barrier */
+    if (want_sigma) { /* overflow recorded now: seen by every CTA after the barrier */
       const bool any_ovf = __any_sync(FULL, ovf);
       if (any_ovf && (threadIdx.x & 31) == 0) atomicOr(&ctl->sigma_overflow, 1);
     }
     if (!grid_barrier(ctl, p.timeout_ns, d)) break;
-    sig_ready = next_ready;
     sig_bits = sig_bits + p.deg_bits < 64 ? sig_bits + p.deg_bits : 64;
     ++d;
   }
   if (__any_sync(FULL, ovf) && (threadIdx.x & 31) == 0) atomicOr(&ctl->sigma_overflow, 1);
-  /* results are final after the last barrier: scatter them into the
-   * caller's numbering (coalesced reads, stores need no round trip) */
+  /* results are final after the last barrier.  Renumbered graphs: gathered
+   * into the caller's numbering, kOut vertices per thread and round so that
+   * their dependent loads (id, depth, count of the depth's parity) overlap;
+   * coalesced stores.  Otherwise: counts of odd depths join the others, and
+   * kNoList becomes -1. */
+  constexpr int kOut = 4;
   if (done && p.perm) {
-    for (unsigned i = gtid; i < (unsigned)p.n; i += nthreads) {
-      const int o = __ldg(p.perm + i);
-      p.S_out[o] = p.S[i];
-      if (want_sigma) p.sigma_out[o] = p.sigma[i];
+    for (unsigned i0 = gtid; i0 < (unsigned)p.n; i0 += kOut * nthreads) {
+      int o[kOut], sv[kOut];
+      unsigned long long x[kOut];
+#pragma unroll
+      for (int j = 0; j < kOut; ++j) {
+        const unsigned i = i0 + j * nthreads;
+        o[j] = i < (unsigned)p.n ? __ldg(p.inv + i) : -1;
+      }
+#pragma unroll
+      for (int j = 0; j < kOut; ++j) sv[j] = o[j] >= 0 ? p.S[o[j]] : -1;
+      if (want_sigma) {
+#pragma unroll
+        for (int j = 0; j < kOut; ++j)
+          x[j] = sv[j] < 0 ? 0ull : (sv[j] & 1) ? p.sigma_odd[o[j]] : p.sigma[o[j]];
+      }
+#pragma unroll
+      for (int j = 0; j < kOut; ++j) {
+        const unsigned i = i0 + j * nthreads;
+        if (i < (unsigned)p.n) {
+          p.S_out[i] = sv[j] < 0 ? -1 : sv[j];
+          if (want_sigma) p.sigma_out[i] = x[j];
+        }
+      }
+    }
+  } else if (done && want_sigma) {
+    for (unsigned i0 = gtid; i0 < (unsigned)p.n; i0 += kOut * nthreads) {
+      bool odd[kOut];
+      unsigned long long x[kOut];
+#pragma unroll
+      for (int j = 0; j < kOut; ++j) {
+        const unsigned i = i0 + j * nthreads;
+        odd[j] = false;
+        if (i < (unsigned)p.n) {
+          const int sv = p.S[i];
+          odd[j] = sv > 0 && (sv & 1);
+          if (sv == kNoList) p.S[i] = -1;
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < kOut; ++j) x[j] = odd[j] ? p.sigma_odd[i0 + j * nthreads] : 0ull;
+#pragma unroll
+      for (int j = 0; j < kOut; ++j)
+        if (odd[j]) p.sigma[i0 + j * nthreads] = x[j];
     }
   }
   if (gtid == 0) {
@@ -778,60 +1190,68 @@ __global__ void __launch_bounds__(kBlock, TBFS_MIN_BLOCKS) bfs_persistent_kernel
 
 }  // namespace
 
+/* shared memory of a CTA of `block` threads */
+static size_t bfs_smem(int block, bool filter) {
+  return (size_t)(block / 32) * sizeof(ExpandWin) + (filter ? kFilterBits / 8 : 0);
+}
+
+/* the instance for graphs with (or without) short out-lists, with (or
+ * without) path counts */
+static const void *bfs_kernel(bool short_lists, bool sigma) {
+  if (sigma)
+    return short_lists ? reinterpret_cast<const void *>(bfs_persistent_kernel<true, true>)
+                       : reinterpret_cast<const void *>(bfs_persistent_kernel<false, true>);
+  return short_lists ? reinterpret_cast<const void *>(bfs_persistent_kernel<true, false>)
+                     : reinterpret_cast<const void *>(bfs_persistent_kernel<false, false>);
+}
+
 cudaError_t bfs_geometry(int device, LaunchGeom *out) {
-  int sms = 0, coop = 0, per = 0;
+  int sms = 0, coop = 0;
   cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   if (e != cudaSuccess) return e;
   e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
   if (e != cudaSuccess) return e;
   if (!coop) return cudaErrorNotSupported;
-  /* the kernel needs ~20 KB of shared memory per CTA: carve out just enough
-   * for TBFS_MIN_BLOCKS CTAs and leave the rest of the unified L1/shared
-   * array to L1, which caches the depth/path-count gathers */
   int smem_sm = 0;
   e = cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device);
   if (e != cudaSuccess) return e;
-  /* both instances (with and without the short-list levels) have the same
-   * shared memory and register bound; the launch takes the smaller fit */
-  per = 1 << 30;
-  for (const void *fn : {reinterpret_cast<const void *>(bfs_persistent_kernel<false>),
-                         reinterpret_cast<const void *>(bfs_persistent_kernel<true>)}) {
-    cudaFuncAttributes fa;
-    e = cudaFuncGetAttributes(&fa, fn);
-    if (e != cudaSuccess) return e;
-    const size_t need = (size_t)TBFS_MIN_BLOCKS * (fa.sharedSizeBytes + 1024);
-    int carve = (int)((100 * need + (size_t)smem_sm - 1) / (size_t)smem_sm);
-    carve = carve < 100 ? carve : 100;
-    e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, carve);
-    if (e != cudaSuccess) return e;
+  for (int k = 0; k < 4; ++k) { /* carve out what a CTA needs, the rest is L1 */
+    const void *fn = bfs_kernel((k & 1) != 0, (k & 2) != 0);
+    const size_t need = bfs_smem(kBlock, k == 2);
+    const int carve = (int)((100 * (need + 1024) + (size_t)smem_sm - 1) / (size_t)smem_sm);
+    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout,
+                               carve < 100 ? carve : 100);
     int fit = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, fn, kBlock, 0);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, fn, kBlock, need);
     if (e != cudaSuccess) return e;
-    per = fit < per ? fit : per;
+    if (fit < 1) return cudaErrorInvalidConfiguration;
   }
-  if (per < 1) return cudaErrorInvalidConfiguration;
   out->block = kBlock;
-  out->grid = sms * per;
+  out->grid = sms;
   out->sms = sms;
-  out->per_sm = per;
+  out->per_sm = kBlock / kBlockStep;
   return cudaSuccess;
 }
 
-cudaError_t bfs_launch(const BfsParams &p, const LaunchGeom &g, cudaStream_t s) {
-  /* fewer CTAs per SM than fit when the caller's options ask for it; by
-   * default 2 on short-list graphs, whose levels are many and small, so that
-   * fewer CTAs meet at each barrier (2048^2 grid 13.6 vs 15.6 ms per BFS,
-   * 8192^2 grid 68.4 vs 75.7, 200^3 grid 4.92 vs 5.03) */
-  const int want = p.ctas_per_sm > 0 ? p.ctas_per_sm
-                                     : (TBFS_SHORT_LEVELS && p.short_lists ? 2 : 0);
-  const int grid = want > 0 && want < g.per_sm ? g.sms * want : g.grid;
-  void *args[] = {const_cast<BfsParams *>(&p)};
-  /* graphs with short out-lists run the instance with entry-aligned small
-   * levels; the others run the one compiled without them */
-  const void *fn = TBFS_SHORT_LEVELS && p.short_lists
-                       ? reinterpret_cast<const void *>(bfs_persistent_kernel<true>)
-                       : reinterpret_cast<const void *>(bfs_persistent_kernel<false>);
-  return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(g.block), args, 0, s);
+cudaError_t bfs_launch(const BfsParams &p0, const LaunchGeom &g, cudaStream_t s) {
+  /* One CTA per SM, of 256 threads per unit of ctas_per_sm.  By default 2 on
+   * short-list graphs, whose levels are many and small; 4 for depths only and
+   * on large graphs regrouped by degree, whose heavy levels want every warp;
+   * else 3, which leaves more L1 and costs less at every barrier (ms per BFS
+   * with path counts at 3 / 4: RMAT-22 0.487 / 0.445, Erdos-Renyi of 2.5 M
+   * vertices 0.366 / 0.392, of 300 K 0.073 / 0.083, RMAT of 100 K 0.058 /
+   * 0.065). */
+  BfsParams p = p0;
+  const bool short_lists = p.short_lists != 0, sigma = p.sigma != nullptr;
+  const bool full = !sigma || (p.inv && p.nnz > kLargeEntries);
+  const int want = p.ctas_per_sm > 0 ? p.ctas_per_sm : short_lists ? 2 : full ? 4 : 3;
+  const int block = want < g.per_sm ? kBlockStep * want : g.block;
+  p.filter = !short_lists && sigma && p.tile && (double)p.nnz > kHeavyEntries;
+  void *args[] = {&p};
+  return cudaLaunchCooperativeKernel(bfs_kernel(short_lists, sigma), dim3(g.grid), dim3(block), args,
+                                     bfs_smem(block, p.filter), s);
 }
 
 }  // namespace tbfs

@@ -11,14 +11,14 @@
  * control block the traversal needs live in one file-scope device array,
  * g_noalloc_scratch, sized for graphs of up to TBFS_NOALLOC_MAX_VERTICES
  * vertices.  That array is part of the library's device code: once that code
- * is loaded on a GPU, the GPU holds the array (about 36 MB) until the process
+ * is loaded on a GPU, the GPU holds the array (about 33 MB) until the process
  * exits.
  *
  * Host code cannot use the array's name as a device address; on the first
  * call on each device (with that device current) the address is looked up
  * with cudaGetSymbolAddress and cached for the device's current context.
  * CUDA loads device code lazily, so when nothing else of the library ran on
- * that device yet, this first call is also the moment the 36 MB are
+ * that device yet, this first call is also the moment the 33 MB are
  * committed: make it as a warm-up before the host framework reserves the
  * device memory it manages, and before any stream capture.  If the memory
  * is not there, the call fails with TBFS_ERR_OUT_OF_MEMORY.  A new context
@@ -43,7 +43,8 @@ namespace {
 constexpr size_t kCtlBytes = 8192; /* control block + validation flag */
 constexpr size_t kQueueBytes = (size_t)TBFS_NOALLOC_MAX_VERTICES * sizeof(int);
 constexpr size_t kBitmapBytes = (size_t)TBFS_NOALLOC_MAX_VERTICES / 8;
-constexpr size_t kScratchBytes = kCtlBytes + 9 * kQueueBytes + 4 * kBitmapBytes;
+constexpr size_t kSigmaBytes = (size_t)TBFS_NOALLOC_MAX_VERTICES * sizeof(unsigned long long);
+constexpr size_t kScratchBytes = kCtlBytes + kSigmaBytes + 6 * kQueueBytes + 3 * kBitmapBytes;
 constexpr size_t kFlagOffset = kCtlBytes - 256;
 static_assert(sizeof(tbfs::BfsCtl) <= kFlagOffset, "control block must fit its slot");
 
@@ -109,7 +110,7 @@ tbfs_status setup_device(int dev, DeviceSetup **out) {
     cudaError_t e = cudaGetSymbolAddress(&ptr, g_noalloc_scratch);
     if (e == cudaErrorMemoryAllocation)
       return fail(TBFS_ERR_OUT_OF_MEMORY,
-                  "tbfs_bfs_noalloc: loading the library's device code (with its 36 MB scratch "
+                  "tbfs_bfs_noalloc: loading the library's device code (with its 33 MB scratch "
                   "array) on this device failed for lack of memory; make the first call before "
                   "device memory is reserved by the host framework");
     if (e != cudaSuccess) return cuda_fail(e, "cudaGetSymbolAddress(scratch)");
@@ -153,7 +154,7 @@ extern "C" tbfs_status tbfs_bfs_noalloc(const int32_t *d_col_ptr, const int32_t 
   unsigned char *base = ds->scratch;
   tbfs::BfsCtl *ctl = reinterpret_cast<tbfs::BfsCtl *>(base);
   int *flag = reinterpret_cast<int *>(base + kFlagOffset);
-  int *q = reinterpret_cast<int *>(base + kCtlBytes);
+  int *q = reinterpret_cast<int *>(base + kCtlBytes + kSigmaBytes);
 
   /* the array keeps the previous call's contents: clear control block + flag */
   if ((e = cudaMemsetAsync(base, 0, kCtlBytes, s)) != cudaSuccess) return cuda_fail(e, "clear");
@@ -181,13 +182,17 @@ extern "C" tbfs_status tbfs_bfs_noalloc(const int32_t *d_col_ptr, const int32_t 
   p.perm = nullptr;
   p.S_out = p.S;
   p.sigma_out = p.sigma;
-  for (int b = 0; b < 3; ++b) {
+  p.sigma_odd = reinterpret_cast<unsigned long long *>(base + kCtlBytes);
+  for (int b = 0; b < 2; ++b) {
     p.q[b] = q + (size_t)(0 + b) * TBFS_NOALLOC_MAX_VERTICES;
-    p.e[b] = q + (size_t)(3 + b) * TBFS_NOALLOC_MAX_VERTICES;
-    p.a[b] = q + (size_t)(6 + b) * TBFS_NOALLOC_MAX_VERTICES;
+    p.e[b] = q + (size_t)(2 + b) * TBFS_NOALLOC_MAX_VERTICES;
+    p.a[b] = q + (size_t)(4 + b) * TBFS_NOALLOC_MAX_VERTICES;
   }
-  for (int b = 0; b < 4; ++b)
-    p.fb[b] = reinterpret_cast<unsigned *>(base + kCtlBytes + 9 * kQueueBytes + b * kBitmapBytes);
+  for (int b = 0; b < 3; ++b)
+    p.fb[b] = reinterpret_cast<unsigned *>(base + kCtlBytes + kSigmaBytes + 6 * kQueueBytes +
+                                           b * kBitmapBytes);
+  p.nnz = nnz;
+  p.hub_len = ~0u; /* no segment list: a warp pulls a long list whole */
   p.trace = nullptr;
   p.trace_cap = 0;
   p.ctl = ctl;
@@ -199,7 +204,6 @@ extern "C" tbfs_status tbfs_bfs_noalloc(const int32_t *d_col_ptr, const int32_t 
   p.symmetric = symmetric ? 1 : 0;
   p.alpha = 15.0f;
   p.beta = 18.0f;
-  p.pull_ratio = 4.0f;
   p.inject_barrier_skip = 0;
   if ((e = tbfs::bfs_launch(p, ds->geom, s)) != cudaSuccess) return cuda_fail(e, "launch");
   tbfs::BfsCtl c;

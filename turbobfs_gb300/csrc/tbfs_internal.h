@@ -5,15 +5,16 @@
  *   cp[n+1], ic[nnz]   int32 CSC: in-lists (column v = sources of edges ->v)
  *   rp[n+1], jr[nnz]   int32 out-lists; aliases cp/ic when the graph is
  *                      symmetric, else the transpose built on the device
- * Per-traversal workspace (reused across calls on the same graph), three
- * rotating buffers so that the queues of levels d-1, d and d+1 coexist:
- *   q[3][n]            int32 frontier vertices
- *   e[3][n]            int32 out-edge offset of each queue entry (exclusive
+ * Per-traversal workspace (reused across calls on the same graph), two
+ * buffers so that the queues of levels d and d+1 coexist:
+ *   q[2][n]            int32 frontier vertices
+ *   e[2][n]            int32 out-edge offset of each queue entry (exclusive
  *                      prefix of out-degrees, in queue order)
- *   a[3][n]            int32 start of each queue entry's out-list (rp[v])
- *   fb[4][n/32]        frontier bitmaps (bit v of fb[d % 4]: v in F_d); four so
- *                      that F_{d-1} and F_d are read while F_{d+1} is written
- *                      and F_{d+2}'s is cleared in the same phase
+ *   a[2][n]            int32 start of each queue entry's out-list (rp[v])
+ *   fb[3][n/32]        frontier bitmaps (bit v of fb[d % 3]: v in F_d), kept by
+ *                      traversals without path counts; F_d is read while
+ *                      F_{d+1} is written and F_{d+2}'s is cleared
+ *   sigma_odd[n]       uint64 path counts of the vertices at odd depth
  *   ctl                control block: per-level counters, barrier words
  * Outputs: S[n] int32 (-1 unreached), sigma[n] uint64 bit patterns of the
  * int64 path counts.
@@ -58,7 +59,8 @@ struct __align__(128) BfsCtl {
   int timeout_level;   /* level + 2 of the barrier that gave up, else 0  */
   long long visited, edges;
   unsigned int work[4]; /* dynamic work counter of phase d in work[d % 4] */
-  unsigned int pad0[10];
+  unsigned long long collect; /* queue of a level found bottom-up: (count << 32) | edges */
+  unsigned int pad0[8];
   GridBarrier bar;
 };
 
@@ -66,21 +68,31 @@ struct BfsParams {
   const int *cp, *ic; /* in-lists  */
   const int *rp, *jr; /* out-lists */
   int *S;
-  unsigned long long *sigma; /* null: S only */
-  int *q[3], *e[3], *a[3];   /* queue buffers; level d uses buffer d % 3 */
-  unsigned *fb[4];           /* frontier bitmaps; F_d in fb[d % 4]         */
+  unsigned long long *sigma; /* null: S only; else counts of even depths until
+                                the end, of all depths then */
+  unsigned long long *sigma_odd; /* counts of odd depths (bfs_engine.cu) */
+  int *q[2], *e[2], *a[2];   /* queue buffers; level d uses buffer d % 2 */
+  unsigned *fb[3];           /* frontier bitmaps; F_d in fb[d % 3]         */
+  /* segments of the in-lists longer than hub_len, as (vertex, first entry)
+   * pairs, and their number (on the device; null: none, hub_len huge) */
+  const int *hub_seg, *hub_count;
+  unsigned hub_len;
+  /* first vertex of every piece of kTileCost in-list entries (a vertex costs
+   * kTileVertex more), tile_count(n, nnz) + 1 of them, or null */
+  const int *tile;
+  long long nnz;
+  int filter; /* the launch has shared memory for a frontier filter */
   BfsCtl *ctl;
   long long out_edges_total;
   long long timeout_ns;
   int n, root, mode, symmetric;
   float alpha, beta;
-  float pull_ratio; /* see tbfs_options.pull_ratio */
   int inject_barrier_skip; /* test hook, 0 = off */
   int trace_cap;           /* records in trace */
   long long *trace;        /* device buffer of trace_cap x 4 int64, or null */
   /* graph stored in its own numbering: inv[caller id] = internal id,
    * perm[internal id] = caller id; S and sigma above are then internal work
-   * arrays, scattered into S_out / sigma_out (caller order) at the end.
+   * arrays, gathered into S_out / sigma_out (caller order) at the end.
    * Null: identity. */
   const int *inv;
   const int *perm;
@@ -100,6 +112,11 @@ struct BfsParams {
 
 /* longest out-list for which a lane walks a whole list alone */
 constexpr int kShortList = 16;
+/* work of a bottom-up level is cut by in-list entries plus this per vertex */
+constexpr int kTileCost = 512;
+constexpr int kTileVertex = 4;
+/* in-lists longer than this are pulled in segments of this many entries */
+constexpr int kHubLen = 1024;
 
 /* Control block of a COOC traversal (cooc_engine.cu); zeroed before every
  * launch. */
@@ -143,6 +160,17 @@ cudaError_t cooc_check(const int *I, const int *J, long long nnz, int n, int *d_
 /* *out = the longest list of the n lists delimited by ptr[0..n] (ptr on the
  * device), synchronously on the current device */
 cudaError_t longest_list(const int *ptr, int n, int *out);
+/* *count = segments of kHubLen entries of the lists longer than that, and
+ * seg[0 .. 2 * count) = their (list, first entry) pairs, in no order; seg holds
+ * hub_segments_cap(nnz) ints.  Queued on s. */
+inline size_t hub_segments_cap(int64_t nnz) { return 4 * ((size_t)nnz / kHubLen + 1); }
+/* pieces of equal cost of the lists delimited by ptr[0..n] (BfsParams::tile):
+ * tile[0 .. tile_count] */
+inline long long tile_count(int n, int64_t nnz) {
+  return (nnz + (long long)kTileVertex * n) / kTileCost + 1;
+}
+cudaError_t fill_tiles(const int *ptr, int n, int64_t nnz, int *tile, cudaStream_t s);
+cudaError_t hub_segments(const int *ptr, int n, int *count, int *seg, cudaStream_t s);
 
 /* ---- frontier-matrix batch (batch_engine.cu) ----
  * Up to 256 roots on one graph advance together: bit r of a vertex's row
@@ -349,14 +377,17 @@ struct tbfs_graph {
   bool separate_out = false;
   long long out_edges_total = 0;
   /* workspace */
-  int *queues = nullptr; /* one allocation: q[3], e[3], a[3], n ints each */
-  char *hot = nullptr;   /* one allocation: sigma_work, S_work, bitmaps */
+  int *queues = nullptr; /* one allocation: q[2], e[2], a[2], n ints each */
+  char *hot = nullptr;   /* one allocation: sigma_odd, sigma_work, S_work, bitmaps */
+  int *tile = nullptr;   /* BfsParams::tile */
+  int *hubs = nullptr;   /* segment count, then the hub segments (BfsParams::hub_seg) */
   int deg_bits = 0;      /* bits of the largest in-degree */
   bool short_lists = false; /* no out-list longer than kShortList */
   /* the caller's TBFS_GRAPH_SYMMETRIC (flags may also carry it when the
    * lists were found to equal their transpose on upload) */
   bool declared_symmetric = false;
-  unsigned *bitmaps = nullptr; /* four frontier bitmaps, (n+31)/32 words each */
+  unsigned *bitmaps = nullptr; /* three frontier bitmaps, (n+31)/32 words each */
+  unsigned long long *sigma_odd = nullptr;
   /* degree-grouped numbering: inv[caller id] = internal id (null: identity);
    * the traversal works on internal S/sigma and un-permutes at the end */
   int *inv = nullptr;

@@ -19,8 +19,8 @@
  * accumulated distributions are the reference's to the bit.
  *
  * Autotuner: the single-source engine's shape (list entries per lane and
- * round, CTAs per SM), then its direction switch (alpha, beta) and path-count
- * schedule (pull_ratio) are chosen by timing traversals from sample roots
+ * round, threads per SM), then its direction switch (alpha, beta) are chosen
+ * by timing traversals from sample roots
  * (CUDA events) over a small grid of candidates; the frontier-matrix batch's
  * push/pull threshold likewise by timing batch launches.  The winner is
  * cached under a key made of the profile's shape (log2 of n, nnz and the
@@ -65,6 +65,36 @@ __global__ void degree_profile_kernel(const int *cp, int n, unsigned long long *
   __syncthreads();
   if (threadIdx.x < kBuckets && h[threadIdx.x]) atomicAdd(hist + threadIdx.x, (unsigned long long)h[threadIdx.x]);
   if (threadIdx.x == 0) atomicMax(maxdeg, mx);
+}
+
+/* tile[i] = first vertex v with ptr[v] + kTileVertex * v >= i * kTileCost, for
+ * i <= tiles (n where there is none) */
+__global__ void tile_kernel(const int *ptr, int n, int tiles, int *tile) {
+  for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v <= n;
+       v += (long long)gridDim.x * blockDim.x) {
+    const long long at = ptr[v] + (long long)kTileVertex * v;
+    const long long before = v > 0 ? ptr[v - 1] + (long long)kTileVertex * (v - 1) : -1;
+    long long i = before < 0 ? 0 : before / kTileCost + 1;
+    for (; i <= tiles && i * kTileCost <= at; ++i) tile[i] = (int)v;
+    if (v == n)
+      for (; i <= tiles; ++i) tile[i] = n;
+  }
+}
+
+/* (list, first entry) of every kHubLen-entry segment of the lists longer
+ * than that */
+__global__ void hub_segments_kernel(const int *ptr, int n, int *count, int *seg) {
+  for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n;
+       v += (long long)gridDim.x * blockDim.x) {
+    const int b = ptr[v], len = ptr[v + 1] - b;
+    if (len <= kHubLen) continue;
+    const int k = (len + kHubLen - 1) / kHubLen;
+    const int at = atomicAdd(count, k);
+    for (int j = 0; j < k; ++j) {
+      seg[2 * (at + j)] = (int)v;
+      seg[2 * (at + j) + 1] = b + j * kHubLen;
+    }
+  }
 }
 
 /* degree of internal vertex v: in (cp), out (rp), or the undirected degree
@@ -194,6 +224,21 @@ cudaError_t longest_list(const int *ptr, int n, int *out) {
   if (e == cudaSuccess) e = cudaMemcpy(out, dm, sizeof(int), cudaMemcpyDeviceToHost);
   if (dh) dev_free(dh);
   return e;
+}
+
+cudaError_t fill_tiles(const int *ptr, int n, int64_t nnz, int *tile, cudaStream_t s) {
+  const int tiles = (int)tile_count(n, nnz);
+  const int blocks = (int)std::min<long long>(((long long)n + 255) / 256, 4096);
+  tile_kernel<<<blocks, 256, 0, s>>>(ptr, n, tiles, tile);
+  return cudaGetLastError();
+}
+
+cudaError_t hub_segments(const int *ptr, int n, int *count, int *seg, cudaStream_t s) {
+  cudaError_t e = cudaMemsetAsync(count, 0, sizeof(int), s);
+  if (e != cudaSuccess) return e;
+  const int blocks = (int)std::min<long long>(((long long)n + 255) / 256, 4096);
+  hub_segments_kernel<<<blocks, 256, 0, s>>>(ptr, n, count, seg);
+  return cudaGetLastError();
 }
 
 }  // namespace tbfs
@@ -382,7 +427,7 @@ extern "C" tbfs_status tbfs_autotune(tbfs_graph *g, const int32_t *roots, int32_
   /* stage 1, the engine's shape at the default direction parameters: list
    * entries per lane and round, CTAs per SM */
   const int epts[] = {2, 4, 0};
-  const int ctass[] = {1, 2, 4}; /* 4 = every CTA that fits (0 means 2 on short-list graphs) */
+  const int ctass[] = {1, 2, 4}; /* 4 = every thread that fits (0: 2 to 4 by the graph) */
   const tbfs::Tuned s0 = best;
   for (int e : epts)
     for (int c : ctass) {
@@ -391,22 +436,18 @@ extern "C" tbfs_status tbfs_autotune(tbfs_graph *g, const int32_t *roots, int32_
       t.ctas = c;
       if (t.ept != s0.ept || t.ctas != s0.ctas) consider(t);
     }
-  /* stage 2, every combination of a grid of the direction switch and the
-   * path-count schedule at that shape (a coordinate search over wider lists
-   * stalled in a local optimum on RMAT) */
+  /* stage 2, every combination of a grid of the direction switch at that
+   * shape */
   const float alphas[] = {4.0f, 6.0f, 9.0f, 12.0f, 15.0f, 24.0f, 60.0f};
   const float betas[] = {1.0f, 2.0f, 4.0f, 18.0f};
-  const float ratios[] = {0.5f, 1.0f, 2.0f, 4.0f};
   const tbfs::Tuned s1 = best;
   for (float xa : alphas)
-    for (float xb : betas)
-      for (float xp : ratios) {
-        tbfs::Tuned t = s1;
-        t.a = xa;
-        t.b = xb;
-        t.pr = xp;
-        if (xa != s1.a || xb != s1.b || xp != s1.pr) consider(t);
-      }
+    for (float xb : betas) {
+      tbfs::Tuned t = s1;
+      t.a = xa;
+      t.b = xb;
+      if (xa != s1.a || xb != s1.b) consider(t);
+    }
   tbfs::dev_free(S);
   tbfs::dev_free(sg);
   if (st != TBFS_OK) return st;
