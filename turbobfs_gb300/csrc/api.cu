@@ -277,7 +277,7 @@ static tbfs_status finish_lists(tbfs_graph *g, int *d_flag) {
   g->separate_out = true;
   cudaError_t e = tbfs::dev_alloc(&g->rp, (n + 1) * sizeof(int));
   if (e == cudaSuccess) e = tbfs::dev_alloc(&g->jr, (nnz ? nnz : 1) * sizeof(int));
-  if (e == cudaSuccess) e = tbfs::expand_columns(g->cp, g->n, col, 0);
+  if (e == cudaSuccess) e = tbfs::expand_columns(g->cp, g->n, g->nnz, col, 0);
   if (e == cudaSuccess)
     e = tbfs::counting_sort_lists(g->ic, col, g->nnz, g->n, g->rp, g->jr, d_flag, 0);
   tbfs::dev_free(col);
@@ -599,7 +599,7 @@ extern "C" tbfs_status tbfs_graph_get_cooc(const tbfs_graph *g, int32_t *row, in
   CUDA_TRY(cudaSetDevice(g->device));
   int *dcol = nullptr;
   CUDA_TRY(tbfs::dev_alloc(&dcol, (size_t)g->nnz * sizeof(int)));
-  cudaError_t e = tbfs::expand_columns(g->cp, g->n, dcol, 0);
+  cudaError_t e = tbfs::expand_columns(g->cp, g->n, g->nnz, dcol, 0);
   if (e == cudaSuccess)
     e = cudaMemcpy(col, dcol, (size_t)g->nnz * sizeof(int), cudaMemcpyDeviceToHost);
   if (e == cudaSuccess)

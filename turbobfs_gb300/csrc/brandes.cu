@@ -495,7 +495,7 @@ extern "C" tbfs_status tbfs_brandes(tbfs_graph *g, const int32_t *roots, int32_t
     x.part = x.q + n;
   }
   BTRY(tbfs::dev_alloc(&w.fill, (n + 1) * sizeof(int)), "alloc");
-  BTRY(tbfs::dev_alloc(&w.partial, (size_t)tbfs::scan_partials((long long)n + 2) * sizeof(int)),
+  BTRY(tbfs::dev_alloc(&w.partial, (size_t)tbfs::scan_partials_most((long long)n + 2) * sizeof(int)),
        "alloc");
   BTRY(tbfs::dev_alloc(&w.dl, (size_t)K * n * sizeof(double)), "alloc");
   BTRY(tbfs::dev_alloc(&w.bc, n * sizeof(double)), "alloc");

@@ -320,10 +320,16 @@ cudaError_t validate_csc(const int *cp, const int *ic, int n, long long nnz,
 cudaError_t counting_sort_lists(const int *keys, const int *vals, long long nnz,
                                 int n, int *ptr_out, int *idx_out, int *d_flag,
                                 cudaStream_t s);
-/* stable LSD radix sort of len (key, val) pairs by the low `bits` bits of
- * the key; ktmp / vtmp are len-element scratch; synchronises s */
-cudaError_t stable_sort_pairs(unsigned *keys, unsigned *vals, long long len, int bits,
-                              unsigned *ktmp, unsigned *vtmp, cudaStream_t s);
+/* stable LSD radix sort of len (key, val) pairs by the low `bits` bits of the
+ * key; *ktmp / *vtmp are len-element scratch.  On return *keys / *vals hold
+ * the sorted pairs and *ktmp / *vtmp the other buffers; waits for the device */
+cudaError_t stable_sort_pairs(unsigned **keys, unsigned **vals, long long len, int bits,
+                              unsigned **ktmp, unsigned **vtmp, cudaStream_t s);
+/* Where ptr[c] < 0, c in [0, n]: the start ptr[] already holds of the first
+ * column of sorted keys[0..len) from c on, or total when no key in [c, n) is
+ * left. */
+cudaError_t fill_starts(const unsigned *keys, long long len, int n, int total, int *ptr,
+                        cudaStream_t s);
 /* bits needed for keys up to max_key */
 int key_bits(unsigned max_key);
 
@@ -344,16 +350,19 @@ cudaError_t mm_parse_device(const char *text, long long len, long long nz, long 
 /* exclusive prefix sum of len ints (in place allowed); synchronises s */
 cudaError_t exclusive_scan(const int *in, long long len, int *out, cudaStream_t s);
 /* the same queued on s without synchronising, with the caller's scratch of
- * scan_partials(len) ints */
+ * scan_partials(len) ints; scan_partials_most(len) serve every scan of up to
+ * len ints */
 long long scan_partials(long long len);
+long long scan_partials_most(long long len);
 cudaError_t exclusive_scan_ws(const int *in, long long len, int *out, int *partial,
                               cudaStream_t s);
-cudaError_t expand_columns(const int *cp, int n, int *col_of_entry, cudaStream_t s);
+cudaError_t expand_columns(const int *cp, int n, long long nnz, int *col_of_entry, cudaStream_t s);
 /* Whether the CSC (validated) equals its transpose as a multiset of entries:
- * the sums over all entries u -> v of h(u, v) - h(v, u) vanish for two
- * keyed 64-bit hashes (keys chosen by the caller at random).  A graph that
- * is its own transpose always passes; any other passes only when both
- * independent sums cancel by chance (about 2^-128 for random keys). */
+ * the sums over all entries u -> v of +h({u, v}) where u < v and -h({u, v})
+ * where u > v vanish for two keyed 64-bit hashes (keys chosen by the caller
+ * at random).  A graph that is its own transpose always passes; any other
+ * passes only when both independent sums cancel by chance (about 2^-128 for
+ * random keys). */
 cudaError_t symmetric_check(const int *cp, const int *ic, int n, long long nnz,
                             unsigned long long key1, unsigned long long key2, bool *symmetric,
                             cudaStream_t s);
