@@ -713,19 +713,6 @@ static tbfs_status enqueue_bfs(tbfs_graph *g, const BfsParams &p, cudaStream_t s
   return TBFS_OK;
 }
 
-/* forward traversal with S / sigma left in the graph's internal numbering
- * (device arrays of n), for consumers inside the library */
-tbfs_status tbfs::forward_internal(tbfs_graph *g, int32_t root, const tbfs_options &o, int *S,
-                                   unsigned long long *sigma, cudaStream_t s, BfsCtl *ctl_host) {
-  BfsParams p = make_params(g, root, o, S, sigma);
-  p.S = S;
-  p.sigma = o.want_sigma ? sigma : nullptr;
-  p.S_out = S;
-  p.sigma_out = p.sigma;
-  p.perm = nullptr; /* no scatter into the caller's order; inv still maps the root */
-  return enqueue_bfs(g, p, s, g->ev0, g->ev1, ctl_host);
-}
-
 static tbfs_status stats_from(const BfsCtl &c, cudaEvent_t ev0, cudaEvent_t ev1,
                               tbfs_stats *st) {
   float ms = 0.0f;
@@ -843,6 +830,31 @@ static tbfs_status many_reserve(tbfs_graph *g, int32_t k) {
     g->many_sync.push_back(x);
   }
   g->many_cap = k;
+  return TBFS_OK;
+}
+
+/* forward traversals with S / sigma left in the graph's internal numbering
+ * (device arrays of n), for consumers inside the library: queued on s one
+ * after another, *ctl_host[j] holding root j's control block once s is waited
+ * for */
+tbfs_status tbfs::forward_internal(tbfs_graph *g, const ForwardRoot *roots, int32_t k,
+                                   const tbfs_options &o, cudaStream_t s, BfsCtl **ctl_host) {
+  tbfs_status st = many_reserve(g, k);
+  if (st != TBFS_OK) return st;
+  CUDA_TRY(cudaMemsetAsync(g->many_ctl, 0, (size_t)k * sizeof(BfsCtl), s));
+  for (int32_t j = 0; j < k; ++j) {
+    BfsParams p = make_params(g, roots[j].root, o, roots[j].S, roots[j].sigma);
+    p.S = roots[j].S;
+    p.sigma = o.want_sigma ? roots[j].sigma : nullptr;
+    p.S_out = p.S;
+    p.sigma_out = p.sigma;
+    p.perm = nullptr; /* not into the caller's order; inv still maps the root */
+    p.ctl = g->many_ctl + j;
+    CUDA_TRY(tbfs::bfs_launch(p, g->geom, s));
+  }
+  CUDA_TRY(cudaMemcpyAsync(g->many_ctl_host, g->many_ctl, (size_t)k * sizeof(BfsCtl),
+                           cudaMemcpyDeviceToHost, s));
+  *ctl_host = g->many_ctl_host;
   return TBFS_OK;
 }
 

@@ -15,7 +15,8 @@
  * cooperative launch for up to kMaxSweepRoots roots at once: step D works on
  * level D of every root whose traversal reached that deep, so the roots share
  * the grid barriers and fill the GPU where one root's level would not.
- * Vertices are grouped by depth with a block-aggregated counting sort.
+ * Vertices are grouped by depth and, within it, by the class of their
+ * out-list, with one block-aggregated counting sort for all roots of a launch.
  * Every delta is a pull over the vertex's own out-list in a fixed order, so
  * the result does not depend on scheduling:
  *   out-degree < 32: one lane sums the terms in list order;
@@ -35,6 +36,7 @@
 #include <stdint.h>
 #include <string.h>
 
+#include <algorithm>
 #include <vector>
 
 #include "device_common.cuh"
@@ -48,7 +50,7 @@ using dev::FULL;
 using dev::grid_barrier;
 
 constexpr int kBlock = 256;
-constexpr int kSmemLevels = 8192; /* levels counted in shared memory per block */
+constexpr int kSmemKeys = 11264;  /* depth-and-class keys counted in shared memory per block */
 constexpr int kTile = 4096;       /* vertices per block of the counting sort   */
 constexpr int kWarpDegree = 32;   /* out-degree from which a warp sums a vertex */
 constexpr int kSeg = 2048;        /* entries per segment of a hub's list        */
@@ -62,29 +64,34 @@ struct __align__(128) SweepCtl {
 
 constexpr int kMaxSweepRoots = 32; /* roots per sweep launch (one lane each in the plan) */
 
+/* Out-list classes of a level, in list order; the lists of a lane each in four
+ * classes by length, so that the lanes of a chunk have about as much to add
+ * (one class where the keys of six would not fit shared memory). */
+enum { C_HUB = 0, C_WARP = 1, C_LANE = 2, kClasses = 6, kClassesFew = 3 };
+
 /* one root's arrays (internal numbering) */
 struct RootSweep {
-  const int *S;                      /* depths of the forward traversal      */
-  const unsigned long long *sig;     /* path counts                          */
-  const int *list;                   /* vertices grouped by depth ...        */
-  const int *off;                    /* ... level d at list[off[d], off[d+1]) */
-  int levels;
-  int root;                          /* internal id of the root               */
-  double *q;                         /* (1 + delta[v]) / sigma[v]             */
+  int *S;                            /* depths of the forward traversal      */
+  unsigned long long *sig;           /* path counts                          */
+  int *list;                         /* vertices grouped by depth and class  */
+  int *off;                          /* class c of level d starts at list[off[classes d + c]] */
+  int *fill;                         /* next free position of each           */
+  int levels, classes;
+  int root;                          /* the root (caller numbering in the host's
+                                        copy, internal in the kernels')       */
+  double *q[2];                      /* (1 + delta[v]) / sigma[v] in q[depth % 2],
+                                        zero where it is not computed yet     */
   double *dl;                        /* delta[v] (0 at the root), zero on entry */
-  /* hubs (out-degree > kSeg) by list position i: segoff[i] (exclusive prefix
-   * of their segment counts over positions), hoff[i] (of the hub flags);
-   * hubpos[h] = position of hub h, seg_hub[s] = hub of segment s,
-   * part[s] = sum of segment s */
-  const int *segoff, *hoff, *hubpos, *seg_hub;
+  /* segments of kSeg entries of the hubs (out-degree > kSeg): those of level d
+   * are seg[d] .. seg[d + 1], seg_pos[s] = list position of segment s's hub,
+   * hseg[i] = first segment of the hub at position i, part[s] = its sum */
+  int *seg, *seg_fill, *seg_pos, *hseg;
   double *part;
-  /* vertices with 32 <= out-degree <= kSeg (a warp each): moff[i] exclusive
-   * prefix of their flags over positions, medpos[m] = position of the m-th */
-  const int *moff, *medpos;
 };
 
 struct SweepParams {
   const int *rp, *jr; /* out-lists (internal numbering) */
+  const int *inv;     /* caller id -> internal id, or null */
   const RootSweep *rs;
   int k;              /* roots of the launch            */
   int dmax;           /* largest number of levels       */
@@ -92,37 +99,46 @@ struct SweepParams {
   long long timeout_ns;
 };
 
-/* v is final with the sum acc of its children's q: its delta, q[v] */
-__device__ __forceinline__ void finish(const RootSweep &R, int v, double acc) {
+/* v, of depth d, is final with the sum acc of its children's q: its delta and q */
+__device__ __forceinline__ void finish(const RootSweep &R, int d, int v, double acc) {
   const double sv = (double)__ldg(R.sig + v);
   const double dv = __dmul_rn(sv, acc);
-  R.q[v] = __ddiv_rn(__dadd_rn(1.0, dv), sv);
+  R.q[d & 1][v] = __ddiv_rn(__dadd_rn(1.0, dv), sv);
   if (v != R.root) R.dl[v] = dv;
 }
 
-/* acc += q[w] of the entries k0, k0 + step, ... < e with S[w] = d + 1, in
- * that order; four entries' loads are issued before they are added */
+/* The sum of q[w] over the entries k0, k0 + step, ... < e with S[w] = d + 1, in
+ * that order.  No depth is looked at: an out-neighbour w of a vertex of depth d
+ * has S[w] <= d + 1, and in the array of d + 1's parity only depths d + 1,
+ * d + 3, ... are computed, the others 0.0, which leaves the sum as it is, to
+ * the bit: one gather per entry where the depth and then a child's q took
+ * two, the second waiting for the first.  Eight entries' loads are issued
+ * before they are added. */
 __device__ __forceinline__ double sum_entries(const SweepParams &p, const RootSweep &R, int d,
                                               int k0, int e, int step) {
+  const double *q = R.q[(d + 1) & 1];
   double acc = 0.0;
   int k = k0;
-  for (; k + 3 * step < e; k += 4 * step) {
+  for (; k + 7 * step < e; k += 8 * step) {
+    int w[8];
+    double t[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) w[j] = __ldg(p.jr + k + j * step);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) t[j] = q[w[j]];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc = __dadd_rn(acc, t[j]);
+  }
+  for (; k < e; k += 4 * step) {
     int w[4];
-    bool c[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) w[j] = __ldg(p.jr + k + j * step);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) c[j] = __ldg(R.S + w[j]) == d + 1;
     double t[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) t[j] = c[j] ? __ldcg(R.q + w[j]) : 0.0;
+    for (int j = 0; j < 4; ++j) w[j] = k + j * step < e ? __ldg(p.jr + k + j * step) : -1;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) t[j] = w[j] >= 0 ? q[w[j]] : 0.0;
 #pragma unroll
     for (int j = 0; j < 4; ++j)
-      if (c[j]) acc = __dadd_rn(acc, t[j]);
-  }
-  for (; k < e; k += step) {
-    const int w = __ldg(p.jr + k);
-    if (__ldg(R.S + w) == d + 1) acc = __dadd_rn(acc, __ldcg(R.q + w));
+      if (w[j] >= 0) acc = __dadd_rn(acc, t[j]);
   }
   return acc;
 }
@@ -138,55 +154,93 @@ __device__ __forceinline__ double warp_sum(const SweepParams &p, const RootSweep
   return __shfl_sync(FULL, acc, 0);
 }
 
-/* Items of step D for root R: hub segments, lists a warp sums, chunks of 32
- * positions of short lists -- or, at the root's deepest level, chunks of 32
- * positions whose q = 1 / sigma (no children).  cnt[0..3]: segments, warp
- * lists, chunks, hubs to combine afterwards. */
+/* The butterfly of eight lists at once: a[i] is this lane's part of list i's
+ * sum, and lanes 4 i .. 4 i + 3 return list i's.  Where two lists are left in a
+ * register pair, a lane keeps one and hands the other to the lane it would
+ * have been added from: the adds are those of warp_sum, one for two lists (9
+ * instead of 40).  FP64 runs at two lanes per clock and SM here, so an add of
+ * a whole warp costs 16 clocks, and the division of one list by one lane as
+ * much as that of eight by eight. */
+__device__ __forceinline__ double warp_sum8(double (&a)[8]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int h = 4, o = 16; h > 0; h >>= 1, o >>= 1) { /* lists left per lane: 2h -> h */
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int i = 0; i < h; ++i) {
+      const double keep = up ? a[i + h] : a[i], give = up ? a[i] : a[i + h];
+      a[i] = __dadd_rn(keep, __shfl_xor_sync(FULL, give, o));
+    }
+  }
+  a[0] = __dadd_rn(a[0], __shfl_xor_sync(FULL, a[0], 2));
+  return __dadd_rn(a[0], __shfl_xor_sync(FULL, a[0], 1));
+}
+
+/* Items of step D for root R: hub segments, groups of `per` lists a warp sums,
+ * chunks of 32 short lists -- or, at the root's deepest level, chunks of 32 positions whose
+ * q = 1 / sigma (no children).  cnt[0..3]: segments, warp lists (not yet in
+ * groups), chunks, hubs to combine afterwards. */
 __device__ __forceinline__ void step_counts(const RootSweep &R, int D, unsigned (&cnt)[4]) {
   cnt[0] = cnt[1] = cnt[2] = cnt[3] = 0u;
   if (D >= R.levels) return;
-  const int lo = __ldg(R.off + D), hi = __ldg(R.off + D + 1);
-  cnt[2] = (unsigned)(hi - lo + 31) / 32u;
-  if (D == R.levels - 1) return;
-  cnt[0] = (unsigned)(__ldg(R.segoff + hi) - __ldg(R.segoff + lo));
-  cnt[1] = (unsigned)(__ldg(R.moff + hi) - __ldg(R.moff + lo));
-  cnt[3] = (unsigned)(__ldg(R.hoff + hi) - __ldg(R.hoff + lo));
+  const int *o = R.off + R.classes * D;
+  const int lo = __ldg(o), hi = __ldg(o + R.classes);
+  if (D == R.levels - 1) {
+    cnt[2] = (unsigned)(hi - lo + 31) / 32u;
+    return;
+  }
+  const int w = __ldg(o + C_WARP), l = __ldg(o + C_LANE);
+  cnt[0] = (unsigned)(__ldg(R.seg + D + 1) - __ldg(R.seg + D));
+  cnt[1] = (unsigned)(l - w);
+  cnt[2] = (unsigned)(hi - l + 31) / 32u;
+  cnt[3] = (unsigned)(w - lo);
 }
 
-/* phase A item `it` (< ns + nm + nch) of root R at step D */
+/* phase A item `it` of root R at step D */
 __device__ __forceinline__ void sweep_item(const SweepParams &p, const RootSweep &R, int D,
-                                           unsigned it) {
+                                           unsigned it, unsigned per) {
   const int lane = threadIdx.x & 31;
-  const int lo = __ldg(R.off + D), hi = __ldg(R.off + D + 1);
+  const int *o = R.off + R.classes * D;
+  const int hi = __ldg(o + R.classes);
   if (D == R.levels - 1) { /* the root's deepest level: no children */
-    const int i = lo + (int)it * 32 + lane;
+    const int i = __ldg(o) + (int)it * 32 + lane;
     if (i < hi) {
       const int v = __ldg(R.list + i);
-      R.q[v] = __ddiv_rn(1.0, (double)__ldg(R.sig + v));
+      R.q[D & 1][v] = __ddiv_rn(1.0, (double)__ldg(R.sig + v));
     }
     return;
   }
-  const int s_lo = __ldg(R.segoff + lo), m_lo = __ldg(R.moff + lo);
-  const unsigned ns = (unsigned)(__ldg(R.segoff + hi) - s_lo);
-  const unsigned nm = (unsigned)(__ldg(R.moff + hi) - m_lo);
+  const int s_lo = __ldg(R.seg + D), w = __ldg(o + C_WARP), l = __ldg(o + C_LANE);
+  const unsigned ns = (unsigned)(__ldg(R.seg + D + 1) - s_lo), nm = (unsigned)(l - w);
+  const unsigned ng = (nm + per - 1u) / per;
   if (it < ns) { /* segment sg of a hub */
     const int sg = s_lo + (int)it;
-    const int i = __ldg(R.hubpos + __ldg(R.seg_hub + sg));
+    const int i = __ldg(R.seg_pos + sg);
     const int v = __ldg(R.list + i);
-    const int b = __ldg(p.rp + v) + (sg - __ldg(R.segoff + i)) * kSeg;
+    const int b = __ldg(p.rp + v) + (sg - __ldg(R.hseg + i)) * kSeg;
     const int e = min(b + kSeg, __ldg(p.rp + v + 1));
     const double acc = warp_sum(p, R, D, b, e);
     if (lane == 0) R.part[sg] = acc;
-  } else if (it < ns + nm) { /* a one-segment list, the whole warp */
-    const int v = __ldg(R.list + __ldg(R.medpos + m_lo + (int)(it - ns)));
-    const double acc = warp_sum(p, R, D, __ldg(p.rp + v), __ldg(p.rp + v + 1));
-    if (lane == 0) finish(R, v, acc);
+  } else if (it < ns + ng) { /* one-segment lists, the whole warp on each */
+    const int i0 = w + (int)((it - ns) * per), i1 = min(i0 + (int)per, l);
+    double a[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      a[j] = 0.0;
+      if (i0 + j < i1) {
+        const int v = __ldg(R.list + i0 + j);
+        a[j] = sum_entries(p, R, D, __ldg(p.rp + v) + lane, __ldg(p.rp + v + 1), 32);
+      }
+    }
+    __syncwarp();
+    const double acc = warp_sum8(a);
+    const int i = i0 + (((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1));
+    if ((lane & 3) == 0 && i < i1) finish(R, D, __ldg(R.list + i), acc);
   } else { /* short lists, one lane each */
-    const int i = lo + (int)(it - ns - nm) * 32 + lane;
+    const int i = l + (int)(it - ns - ng) * 32 + lane;
     if (i < hi) {
       const int v = __ldg(R.list + i);
-      const int b = __ldg(p.rp + v), e = __ldg(p.rp + v + 1);
-      if (e - b < kWarpDegree) finish(R, v, sum_entries(p, R, D, b, e, 1));
+      finish(R, D, v, sum_entries(p, R, D, __ldg(p.rp + v), __ldg(p.rp + v + 1), 1));
     }
   }
 }
@@ -205,12 +259,16 @@ __device__ __forceinline__ int root_of(const unsigned *pre, int k, unsigned x) {
 __global__ void __launch_bounds__(kBlock) sweep_kernel(const SweepParams p) {
   __shared__ unsigned s_pa[kMaxSweepRoots + 1], s_pb[kMaxSweepRoots + 1];
   __shared__ RootSweep s_rs[kMaxSweepRoots];
+  __shared__ unsigned s_per;
   const int lane = threadIdx.x & 31;
   const unsigned gwarp = (blockIdx.x * kBlock + threadIdx.x) >> 5;
   const unsigned nwarps = (gridDim.x * kBlock) >> 5;
   const unsigned gthread = blockIdx.x * kBlock + threadIdx.x;
   const unsigned nthreads = gridDim.x * kBlock;
-  for (int r = threadIdx.x; r < p.k; r += kBlock) s_rs[r] = p.rs[r];
+  for (int r = threadIdx.x; r < p.k; r += kBlock) {
+    s_rs[r] = p.rs[r];
+    if (p.inv) s_rs[r].root = __ldg(p.inv + s_rs[r].root);
+  }
   __syncthreads();
   for (int D = p.dmax - 1; D >= 0; --D) {
     /* the step's plan, identical in every CTA: per root, its phase-A items
@@ -218,7 +276,11 @@ __global__ void __launch_bounds__(kBlock) sweep_kernel(const SweepParams p) {
     if (threadIdx.x < 32) { /* lane r: root r's counts, then prefixes over the lanes */
       unsigned c[4] = {0u, 0u, 0u, 0u};
       if (lane < p.k) step_counts(s_rs[lane], D, c);
-      const unsigned a = c[0] + c[1] + c[2], b = c[3];
+      /* lists per warp item: as many as leave two items for every warp */
+      unsigned all = __reduce_add_sync(FULL, c[1]) / (2u * nwarps);
+      const unsigned per = all < 1u ? 1u : all > 8u ? 8u : all;
+      if (lane == 0) s_per = per;
+      const unsigned a = c[0] + (c[1] + per - 1u) / per + c[2], b = c[3];
       unsigned ia = a, ib = b;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -240,12 +302,12 @@ __global__ void __launch_bounds__(kBlock) sweep_kernel(const SweepParams p) {
     /* work counter of step D-2 (last used at step D+2) */
     if (gthread == 0) p.ctl->work[(D + 2) & 3] = 0u;
     __syncthreads();
-    const unsigned items = s_pa[p.k], hubs = s_pb[p.k];
+    const unsigned items = s_pa[p.k], hubs = s_pb[p.k], per = s_per;
     /* items: static first, then claimed; each root's long items come first */
     unsigned it = gwarp;
     while (it < items) {
       const int r = root_of(s_pa, p.k, it);
-      sweep_item(p, s_rs[r], D, it - s_pa[r]);
+      sweep_item(p, s_rs[r], D, it - s_pa[r], per);
       if (items <= nwarps) break;
       unsigned nxt = 0;
       if (lane == 0) nxt = nwarps + atomicAdd(&p.ctl->work[D & 3], 1u);
@@ -256,13 +318,13 @@ __global__ void __launch_bounds__(kBlock) sweep_kernel(const SweepParams p) {
       for (unsigned t = gthread; t < hubs; t += nthreads) {
         const int r = root_of(s_pb, p.k, t);
         const RootSweep &R = s_rs[r];
-        const int lo = __ldg(R.off + D);
-        const int i = __ldg(R.hubpos + __ldg(R.hoff + lo) + (int)(t - s_pb[r]));
+        const int i = __ldg(R.off + R.classes * D) + (int)(t - s_pb[r]);
         const int v = __ldg(R.list + i);
-        const int s0 = __ldg(R.segoff + i), s1 = __ldg(R.segoff + i + 1);
+        const int s0 = __ldg(R.hseg + i);
+        const int s1 = s0 + (__ldg(p.rp + v + 1) - __ldg(p.rp + v) + kSeg - 1) / kSeg;
         double acc = __ldcg(R.part + s0);
         for (int sg = s0 + 1; sg < s1; ++sg) acc = __dadd_rn(acc, __ldcg(R.part + sg));
-        finish(R, v, acc);
+        finish(R, D, v, acc);
       }
     }
     if (!grid_barrier(p.ctl, p.timeout_ns, D)) return;
@@ -280,104 +342,126 @@ __global__ void bc_add_kernel(double *bc, const double *dl, int k, int n) {
   }
 }
 
-/* segs[i] = segments of the vertex at list position i (0 unless a hub),
- * flag[i] = it is a hub, mflag[i] = a warp sums its list; for i < *cnt (the
- * reached vertices), 0 up to len */
-__global__ void hub_count_kernel(const int *list, const int *rp, const int *cnt, int len,
-                                 int *segs, int *flag, int *mflag) {
-  const int c = *cnt;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < len; i += gridDim.x * blockDim.x) {
-    int h = 0, sg = 0, m = 0;
-    if (i < c) {
-      const int v = list[i];
-      const int deg = rp[v + 1] - rp[v];
-      h = deg > kSeg ? 1 : 0;
-      sg = h ? (deg + kSeg - 1) / kSeg : 0;
-      m = deg >= kWarpDegree && deg <= kSeg ? 1 : 0;
-    }
-    segs[i] = sg;
-    flag[i] = h;
-    mflag[i] = m;
+/* ---- vertices grouped by depth and class (counting sort, block-aggregated),
+ * for all roots of a launch at once: blockIdx.y is the root.  Sixteen launches
+ * and a wait per root (a sort by depth, then flags, prefixes and position maps
+ * of the classes) took 105 us of an RMAT-18 root; three launches for sixteen
+ * roots take 80 us in all. ---- */
+
+/* key of v (classes * depth + class), or -1 if the root does not reach it; segs = its
+ * segments if it is a hub */
+__device__ __forceinline__ int sort_key(const RootSweep &R, const int *rp, int v, int &segs) {
+  const int d = __ldg(R.S + v);
+  segs = 0;
+  if (d < 0) return -1;
+  const int deg = __ldg(rp + v + 1) - __ldg(rp + v);
+  if (deg > kSeg) {
+    segs = (deg + kSeg - 1) / kSeg;
+    return R.classes * d + C_HUB;
   }
-}
-
-/* medpos[moff[i]] = i for the positions a warp sums */
-__global__ void med_fill_kernel(const int *moff, const int *cnt, int *medpos) {
-  const int c = *cnt;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < c; i += gridDim.x * blockDim.x)
-    if (moff[i + 1] != moff[i]) medpos[moff[i]] = i;
-}
-
-/* hubpos[hoff[i]] = i and seg_hub[s] = hoff[i] for the hubs' segments */
-__global__ void hub_fill_kernel(const int *segoff, const int *hoff, const int *cnt,
-                                int *hubpos, int *seg_hub) {
-  const int c = *cnt;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < c; i += gridDim.x * blockDim.x) {
-    const int h = hoff[i];
-    if (hoff[i + 1] == h) continue;
-    hubpos[h] = i;
-    for (int sg = segoff[i]; sg < segoff[i + 1]; ++sg) seg_hub[sg] = h;
+  int c = C_WARP;
+  if (deg < kWarpDegree) {
+    c = C_LANE;
+    if (R.classes == kClasses) c += deg >= 16 ? 0 : deg >= 8 ? 1 : deg >= 4 ? 2 : 3;
   }
+  return R.classes * d + c;
 }
 
-/* ---- vertices grouped by depth (counting sort, block-aggregated) ---- */
-
-/* counts[d] = vertices at depth d */
-__global__ void level_count_kernel(const int *S, int n, int levels, int *counts) {
-  __shared__ int h[kSmemLevels];
-  const bool local = levels <= kSmemLevels;
+/* off[key] = vertices of that key, seg[d] = segments of level d (zero before) */
+__global__ void level_count_kernel(const RootSweep *rs, const int *rp, int n) {
+  __shared__ int h[kSmemKeys];
+  const RootSweep R = rs[blockIdx.y];
+  const int keys = R.classes * R.levels;
+  const bool local = keys <= kSmemKeys;
   if (local)
-    for (int d = threadIdx.x; d < levels; d += blockDim.x) h[d] = 0;
+    for (int k = threadIdx.x; k < keys; k += blockDim.x) h[k] = 0;
   __syncthreads();
   const long long base = (long long)blockIdx.x * kTile;
   for (int j = threadIdx.x; j < kTile; j += blockDim.x) {
     const long long v = base + j;
     if (v >= n) break;
-    const int d = S[v];
-    if (d < 0) continue;
-    if (local)
-      atomicAdd(&h[d], 1);
-    else
-      atomicAdd(&counts[d], 1);
+    int segs;
+    const int k = sort_key(R, rp, (int)v, segs);
+    if (k < 0) continue;
+    atomicAdd(local ? &h[k] : &R.off[k], 1);
+    if (segs) atomicAdd(&R.seg[k / R.classes], segs);
   }
   __syncthreads();
   if (local)
-    for (int d = threadIdx.x; d < levels; d += blockDim.x)
-      if (h[d]) atomicAdd(&counts[d], h[d]);
+    for (int k = threadIdx.x; k < keys; k += blockDim.x)
+      if (h[k]) atomicAdd(&R.off[k], h[k]);
 }
 
-/* list[...] = vertices by depth; fill[d] starts at the exclusive prefix */
-__global__ void level_fill_kernel(const int *S, int n, int levels, int *fill, int *list) {
-  __shared__ int h[kSmemLevels];
-  const bool local = levels <= kSmemLevels;
+/* a[0..len] -> exclusive prefix, copied to b, by one block */
+__device__ void block_prefix(int *a, int *b, int len, int *s_warp) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int carry = 0;
+  for (int i0 = 0; i0 <= len; i0 += blockDim.x) {
+    const int i = i0 + threadIdx.x;
+    const int x = i < len ? a[i] : 0;
+    int inc = x;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(FULL, inc, o);
+      if (lane >= o) inc += t;
+    }
+    if (lane == 31) s_warp[w] = inc;
+    __syncthreads();
+    int before = carry, all = 0;
+    for (int ww = 0; ww < (int)(blockDim.x >> 5); ++ww) {
+      const int t = s_warp[ww];
+      before += ww < w ? t : 0;
+      all += t;
+    }
+    if (i <= len) a[i] = b[i] = before + inc - x;
+    carry += all;
+    __syncthreads();
+  }
+}
+
+__global__ void level_prefix_kernel(const RootSweep *rs) {
+  __shared__ int s_warp[32];
+  const RootSweep R = rs[blockIdx.y];
+  if (blockIdx.x == 0) block_prefix(R.off, R.fill, R.classes * R.levels, s_warp);
+  else block_prefix(R.seg, R.seg_fill, R.levels, s_warp);
+}
+
+/* list[...] = vertices by key, and the hubs' segments */
+__global__ void level_fill_kernel(const RootSweep *rs, const int *rp, int n) {
+  __shared__ int h[kSmemKeys];
+  const RootSweep R = rs[blockIdx.y];
+  const int keys = R.classes * R.levels;
+  const bool local = keys <= kSmemKeys;
   if (local)
-    for (int d = threadIdx.x; d < levels; d += blockDim.x) h[d] = 0;
+    for (int k = threadIdx.x; k < keys; k += blockDim.x) h[k] = 0;
   __syncthreads();
   const long long base = (long long)blockIdx.x * kTile;
   if (local) {
     for (int j = threadIdx.x; j < kTile; j += blockDim.x) {
       const long long v = base + j;
       if (v >= n) break;
-      const int d = S[v];
-      if (d >= 0) atomicAdd(&h[d], 1);
+      int segs;
+      const int k = sort_key(R, rp, (int)v, segs);
+      if (k >= 0) atomicAdd(&h[k], 1);
     }
     __syncthreads();
-    /* reserve this block's range of every level, then hand out positions */
-    for (int d = threadIdx.x; d < levels; d += blockDim.x)
-      if (h[d]) h[d] = atomicAdd(&fill[d], h[d]);
+    /* reserve this block's range of every key, then hand out positions */
+    for (int k = threadIdx.x; k < keys; k += blockDim.x)
+      if (h[k]) h[k] = atomicAdd(&R.fill[k], h[k]);
     __syncthreads();
-    for (int j = threadIdx.x; j < kTile; j += blockDim.x) {
-      const long long v = base + j;
-      if (v >= n) break;
-      const int d = S[v];
-      if (d >= 0) list[atomicAdd(&h[d], 1)] = (int)v;
-    }
-  } else {
-    for (int j = threadIdx.x; j < kTile; j += blockDim.x) {
-      const long long v = base + j;
-      if (v >= n) break;
-      const int d = S[v];
-      if (d >= 0) list[atomicAdd(&fill[d], 1)] = (int)v;
+  }
+  for (int j = threadIdx.x; j < kTile; j += blockDim.x) {
+    const long long v = base + j;
+    if (v >= n) break;
+    int segs;
+    const int k = sort_key(R, rp, (int)v, segs);
+    if (k < 0) continue;
+    const int i = atomicAdd(local ? &h[k] : &R.fill[k], 1);
+    R.list[i] = (int)v;
+    if (segs) {
+      const int s0 = atomicAdd(&R.seg_fill[k / R.classes], segs);
+      R.hseg[i] = s0;
+      for (int t = 0; t < segs; ++t) R.seg_pos[s0 + t] = i;
     }
   }
 }
@@ -408,40 +492,16 @@ tbfs_status bfail(cudaError_t e, const char *what) {
     if (e_ != cudaSuccess) return bfail(e_, what);  \
   } while (0)
 
-/* the arrays of one root of a sweep launch (views into Scratch's pools) */
-struct Slot {
-  int *S = nullptr, *list = nullptr, *off = nullptr;
-  int *segoff = nullptr, *hoff = nullptr, *hubpos = nullptr, *seg_hub = nullptr;
-  int *moff = nullptr, *medpos = nullptr;
-  unsigned long long *sig = nullptr;
-  double *q = nullptr, *part = nullptr;
-};
-
-/* one allocation per kind of array for all slots: a call costs a dozen
- * cudaMalloc calls, not a dozen per root */
+/* the call's device memory, one block */
 struct Scratch {
-  std::vector<Slot> slots;
-  int *ints = nullptr;                /* S, list, off, segoff, hoff, hubpos, moff, medpos, seg_hub */
-  unsigned long long *sigs = nullptr;
-  double *dbls = nullptr;             /* q, part */
-  int *fill = nullptr, *partial = nullptr;
-  double *dl = nullptr; /* K x n: each root's delta */
-  double *bc = nullptr, *out = nullptr;
-  RootSweep *rs = nullptr;
-  SweepCtl *ctl = nullptr;
-  tbfs::BfsCtl *fctl_host = nullptr;
-  ~Scratch() {
-    tbfs::dev_free(ints);
-    tbfs::dev_free(sigs);
-    tbfs::dev_free(dbls);
-    tbfs::dev_free(fill);
-    tbfs::dev_free(partial);
-    tbfs::dev_free(dl);
-    tbfs::dev_free(bc);
-    tbfs::dev_free(out);
-    tbfs::dev_free(rs);
-    tbfs::dev_free(ctl);
-    if (fctl_host) cudaFreeHost(fctl_host);
+  char *base = nullptr;
+  size_t used = 0;
+  ~Scratch() { tbfs::dev_free(base); }
+  template <class T>
+  T *take(size_t count) {
+    T *p = reinterpret_cast<T *>(base + used);
+    used += (count * sizeof(T) + 255) / 256 * 256;
+    return p;
   }
 };
 
@@ -465,44 +525,47 @@ extern "C" tbfs_status tbfs_brandes(tbfs_graph *g, const int32_t *roots, int32_t
   cudaStream_t s = (cudaStream_t)o.stream;
   const size_t n = (size_t)g->n;
   /* roots per sweep launch: up to kMaxSweepRoots, fewer on large graphs
-   * (each root holds about 60 n bytes while its launch runs) */
+   * (each root holds about 80 n bytes while its launch runs) */
   int K = k < tbfs::kMaxSweepRoots ? (k > 0 ? k : 1) : tbfs::kMaxSweepRoots;
-  while (K > 1 && (double)K * 64.0 * (double)n > 16e9) K /= 2;
-  Scratch w;
-  w.slots.resize((size_t)K);
+  while (K > 1 && (double)K * 80.0 * (double)n > 16e9) K /= 2;
   /* segments: each hub has deg > kSeg, so sum of ceil(deg / kSeg) < 2 nnz / kSeg + 1 */
   const size_t seg_cap = (size_t)(2 * g->nnz / tbfs::kSeg + 1);
-  const size_t nI = n + 2; /* every int array of a slot: n + 2 entries */
-  const size_t ints_per_slot = 8 * nI + seg_cap;
-  const size_t dbls_per_slot = n + seg_cap;
-  BTRY(tbfs::dev_alloc(&w.ints, (size_t)K * ints_per_slot * sizeof(int)), "alloc");
-  BTRY(tbfs::dev_alloc(&w.sigs, (size_t)K * n * sizeof(unsigned long long)), "alloc");
-  BTRY(tbfs::dev_alloc(&w.dbls, (size_t)K * dbls_per_slot * sizeof(double)), "alloc");
-  for (int j = 0; j < K; ++j) {
-    Slot &x = w.slots[(size_t)j];
-    int *b = w.ints + (size_t)j * ints_per_slot;
-    x.S = b;
-    x.list = b + nI;
-    x.off = b + 2 * nI;
-    x.segoff = b + 3 * nI;
-    x.hoff = b + 4 * nI;
-    x.hubpos = b + 5 * nI;
-    x.moff = b + 6 * nI;
-    x.medpos = b + 7 * nI;
-    x.seg_hub = b + 8 * nI;
-    x.sig = w.sigs + (size_t)j * n;
-    x.q = w.dbls + (size_t)j * dbls_per_slot;
-    x.part = x.q + n;
+  /* keys of at most n levels: six classes up to kSmemKeys keys, else three */
+  const size_t key_cap = std::max((size_t)tbfs::kSmemKeys, tbfs::kClassesFew * (n + 1)) + 1;
+  std::vector<RootSweep> rs((size_t)K);
+  Scratch w;
+  double *dl = nullptr, *qs = nullptr, *sum = nullptr;
+  int *offs = nullptr, *segs = nullptr;
+  RootSweep *rs_dev = nullptr;
+  SweepCtl *ctl = nullptr;
+  for (int pass = 0; pass < 2; ++pass) { /* sizes first, then the views */
+    w.used = 0;
+    dl = w.take<double>((size_t)K * n);
+    qs = w.take<double>((size_t)K * 2 * n);
+    sum = w.take<double>(n);
+    rs_dev = w.take<RootSweep>((size_t)K);
+    ctl = w.take<SweepCtl>(1);
+    offs = w.take<int>((size_t)K * key_cap);
+    segs = w.take<int>((size_t)K * (n + 2));
+    for (int j = 0; j < K; ++j) {
+      RootSweep &R = rs[(size_t)j];
+      R.S = w.take<int>(n);
+      R.sig = w.take<unsigned long long>(n);
+      R.list = w.take<int>(n);
+      R.off = offs + (size_t)j * key_cap;
+      R.fill = w.take<int>(key_cap);
+      R.q[0] = qs + (size_t)j * 2 * n;
+      R.q[1] = R.q[0] + n;
+      R.dl = dl + (size_t)j * n;
+      R.seg = segs + (size_t)j * (n + 2);
+      R.seg_fill = w.take<int>(n + 2);
+      R.seg_pos = w.take<int>(seg_cap);
+      R.hseg = w.take<int>(n);
+      R.part = w.take<double>(seg_cap);
+    }
+    if (pass == 0) BTRY(tbfs::dev_alloc(&w.base, w.used), "alloc");
   }
-  BTRY(tbfs::dev_alloc(&w.fill, (n + 1) * sizeof(int)), "alloc");
-  BTRY(tbfs::dev_alloc(&w.partial, (size_t)tbfs::scan_partials_most((long long)n + 2) * sizeof(int)),
-       "alloc");
-  BTRY(tbfs::dev_alloc(&w.dl, (size_t)K * n * sizeof(double)), "alloc");
-  BTRY(tbfs::dev_alloc(&w.bc, n * sizeof(double)), "alloc");
-  BTRY(tbfs::dev_alloc(&w.rs, (size_t)K * sizeof(RootSweep)), "alloc");
-  BTRY(tbfs::dev_alloc(&w.ctl, sizeof(SweepCtl)), "alloc");
-  BTRY(cudaMallocHost(&w.fctl_host, sizeof(tbfs::BfsCtl)), "alloc");
-  BTRY(cudaMemsetAsync(w.bc, 0, n * sizeof(double), s), "clear");
+  BTRY(cudaMemsetAsync(sum, 0, n * sizeof(double), s), "clear");
   /* grid of the sweep: all SMs, as occupancy allows (cooperative) */
   int sms = 0, per = 0;
   BTRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, g->device), "attribute");
@@ -522,92 +585,68 @@ extern "C" tbfs_status tbfs_brandes(tbfs_graph *g, const int32_t *roots, int32_t
   fo.outputs_on_device = 1;
   fo.level_trace = nullptr;
   fo.level_trace_cap = 0;
-  std::vector<RootSweep> rs((size_t)K);
   for (int32_t r0 = 0; r0 < k; r0 += K) {
     const int kk = k - r0 < K ? k - r0 : K;
     int dmax = 0;
-    BTRY(cudaMemsetAsync(w.dl, 0, (size_t)kk * n * sizeof(double), s), "clear");
-    for (int j = 0; j < kk; ++j) {
-      Slot &x = w.slots[(size_t)j];
-      tbfs_status st = tbfs::forward_internal(g, roots[r0 + j], fo, x.S, x.sig, s, w.fctl_host);
+    size_t key_max = 0;
+    BTRY(cudaMemsetAsync(dl, 0, (size_t)kk * n * sizeof(double), s), "clear");
+    BTRY(cudaMemsetAsync(qs, 0, (size_t)kk * 2 * n * sizeof(double), s), "clear");
+    /* the forward traversals, one after another without a wait between them */
+    tbfs::BfsCtl *fc = nullptr;
+    {
+      std::vector<tbfs::ForwardRoot> fr((size_t)kk);
+      for (int j = 0; j < kk; ++j)
+        fr[(size_t)j] = {roots[r0 + j], rs[(size_t)j].S, rs[(size_t)j].sig};
+      tbfs_status st = tbfs::forward_internal(g, fr.data(), kk, fo, s, &fc);
       if (st != TBFS_OK) return st;
-      BTRY(cudaStreamSynchronize(s), "forward traversal");
-      const tbfs::BfsCtl &fc = *w.fctl_host;
-      if (fc.status != 0) {
+    }
+    BTRY(cudaStreamSynchronize(s), "forward traversal");
+    for (int j = 0; j < kk; ++j) {
+      if (fc[j].status != 0) {
         tbfs_set_error("tbfs_brandes: forward traversal: grid barrier wait exceeded its budget");
         return TBFS_ERR_TIMEOUT;
       }
-      if (fc.sigma_overflow) ++ovf_roots;
-      const int levels = fc.levels;
-      dmax = levels > dmax ? levels : dmax;
-      /* vertices by depth */
-      BTRY(cudaMemsetAsync(x.off, 0, ((size_t)levels + 1) * sizeof(int), s), "clear");
-      tbfs::level_count_kernel<<<tiles, tbfs::kBlock, 0, s>>>(x.S, g->n, levels, x.off);
-      BTRY(cudaGetLastError(), "level count");
-      BTRY(tbfs::exclusive_scan_ws(x.off, (long long)levels + 1, x.off, w.partial, s),
-           "level prefix");
-      BTRY(cudaMemcpyAsync(w.fill, x.off, (size_t)levels * sizeof(int), cudaMemcpyDeviceToDevice,
-                           s),
-           "fill pointers");
-      tbfs::level_fill_kernel<<<tiles, tbfs::kBlock, 0, s>>>(x.S, g->n, levels, w.fill, x.list);
-      BTRY(cudaGetLastError(), "level fill");
-      /* hubs and warp lists: flags by list position (positions < off[levels],
-       * the reached vertices), their prefixes, the position maps */
-      tbfs::hub_count_kernel<<<cgrid, 256, 0, s>>>(x.list, g->rp, x.off + levels, g->n + 1,
-                                                   x.segoff, x.hoff, x.moff);
-      BTRY(cudaGetLastError(), "hub count");
-      BTRY(tbfs::exclusive_scan_ws(x.segoff, (long long)n + 1, x.segoff, w.partial, s),
-           "segment prefix");
-      BTRY(tbfs::exclusive_scan_ws(x.hoff, (long long)n + 1, x.hoff, w.partial, s), "hub prefix");
-      BTRY(tbfs::exclusive_scan_ws(x.moff, (long long)n + 1, x.moff, w.partial, s),
-           "warp prefix");
-      tbfs::med_fill_kernel<<<cgrid, 256, 0, s>>>(x.moff, x.off + levels, x.medpos);
-      BTRY(cudaGetLastError(), "warp positions");
-      tbfs::hub_fill_kernel<<<cgrid, 256, 0, s>>>(x.segoff, x.hoff, x.off + levels, x.hubpos,
-                                                  x.seg_hub);
-      BTRY(cudaGetLastError(), "hub fill");
-      RootSweep &R = rs[(size_t)j];
-      R.S = x.S;
-      R.sig = x.sig;
-      R.list = x.list;
-      R.off = x.off;
-      R.levels = levels;
-      R.root = g->inv ? -1 : roots[r0 + j]; /* internal id, filled below when renumbered */
-      R.q = x.q;
-      R.dl = w.dl + (size_t)j * n;
-      R.segoff = x.segoff;
-      R.hoff = x.hoff;
-      R.hubpos = x.hubpos;
-      R.seg_hub = x.seg_hub;
-      R.part = x.part;
-      R.moff = x.moff;
-      R.medpos = x.medpos;
-      if (g->inv)
-        BTRY(cudaMemcpyAsync(&R.root, g->inv + roots[r0 + j], sizeof(int), cudaMemcpyDeviceToHost,
-                             s),
-             "root id");
+      if (fc[j].sigma_overflow) ++ovf_roots;
+      rs[(size_t)j].levels = fc[j].levels;
+      rs[(size_t)j].classes =
+          tbfs::kClasses * fc[j].levels <= tbfs::kSmemKeys ? tbfs::kClasses : tbfs::kClassesFew;
+      key_max = std::max(key_max, (size_t)(rs[(size_t)j].classes * (long long)fc[j].levels));
+      rs[(size_t)j].root = roots[r0 + j];
+      dmax = fc[j].levels > dmax ? fc[j].levels : dmax;
     }
-    BTRY(cudaStreamSynchronize(s), "sweep setup");
-    BTRY(cudaMemcpyAsync(w.rs, rs.data(), (size_t)kk * sizeof(RootSweep), cudaMemcpyHostToDevice,
+    BTRY(cudaMemcpyAsync(rs_dev, rs.data(), (size_t)kk * sizeof(RootSweep), cudaMemcpyHostToDevice,
                          s),
          "sweep descriptors");
-    BTRY(cudaMemsetAsync(w.ctl, 0, sizeof(SweepCtl), s), "clear");
+    /* vertices by depth and class */
+    BTRY(cudaMemset2DAsync(offs, key_cap * sizeof(int), 0,
+                           (key_max + 1) * sizeof(int), (size_t)kk, s),
+         "clear");
+    BTRY(cudaMemset2DAsync(segs, (n + 2) * sizeof(int), 0, ((size_t)dmax + 1) * sizeof(int),
+                           (size_t)kk, s),
+         "clear");
+    const dim3 by_root(tiles, (unsigned)kk);
+    tbfs::level_count_kernel<<<by_root, tbfs::kBlock, 0, s>>>(rs_dev, g->rp, g->n);
+    tbfs::level_prefix_kernel<<<dim3(2, (unsigned)kk), 1024, 0, s>>>(rs_dev);
+    tbfs::level_fill_kernel<<<by_root, tbfs::kBlock, 0, s>>>(rs_dev, g->rp, g->n);
+    BTRY(cudaGetLastError(), "vertices by depth");
+    BTRY(cudaMemsetAsync(ctl, 0, sizeof(SweepCtl), s), "clear");
     SweepParams p;
     p.rp = g->rp;
     p.jr = g->jr;
-    p.rs = w.rs;
+    p.inv = g->inv;
+    p.rs = rs_dev;
     p.k = kk;
     p.dmax = dmax;
-    p.ctl = w.ctl;
+    p.ctl = ctl;
     p.timeout_ns = timeout;
     void *args[] = {&p};
     BTRY(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(tbfs::sweep_kernel), dim3(grid),
                                      dim3(tbfs::kBlock), args, 0, s),
          "dependency sweep");
-    tbfs::bc_add_kernel<<<cgrid, 256, 0, s>>>(w.bc, w.dl, kk, g->n);
+    tbfs::bc_add_kernel<<<cgrid, 256, 0, s>>>(sum, dl, kk, g->n);
     BTRY(cudaGetLastError(), "bc sums");
     SweepCtl sc;
-    BTRY(cudaMemcpyAsync(&sc, w.ctl, sizeof(sc), cudaMemcpyDeviceToHost, s), "read sweep status");
+    BTRY(cudaMemcpyAsync(&sc, ctl, sizeof(sc), cudaMemcpyDeviceToHost, s), "read sweep status");
     BTRY(cudaStreamSynchronize(s), "dependency sweep");
     if (sc.status != 0) {
       tbfs_set_error("tbfs_brandes: sweep: grid barrier wait exceeded its budget");
@@ -616,14 +655,11 @@ extern "C" tbfs_status tbfs_brandes(tbfs_graph *g, const int32_t *roots, int32_t
   }
   /* results in the caller's numbering */
   double *dst = bc;
-  if (!o.outputs_on_device) {
-    BTRY(tbfs::dev_alloc(&w.out, n * sizeof(double)), "alloc");
-    dst = w.out;
-  }
-  tbfs::gather_double_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(w.bc, g->inv, g->n, dst);
+  if (!o.outputs_on_device) dst = dl; /* free again */
+  tbfs::gather_double_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(sum, g->inv, g->n, dst);
   BTRY(cudaGetLastError(), "gather");
   if (!o.outputs_on_device)
-    BTRY(cudaMemcpyAsync(bc, w.out, n * sizeof(double), cudaMemcpyDeviceToHost, s), "copy bc");
+    BTRY(cudaMemcpyAsync(bc, dst, n * sizeof(double), cudaMemcpyDeviceToHost, s), "copy bc");
   BTRY(cudaStreamSynchronize(s), "results");
   if (overflow) *overflow = ovf_roots;
   return TBFS_OK;

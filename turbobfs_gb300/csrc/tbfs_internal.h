@@ -431,9 +431,14 @@ struct tbfs_graph {
 };
 
 namespace tbfs {
-/* one traversal with results in the internal numbering (api.cu) */
-tbfs_status forward_internal(tbfs_graph *g, int32_t root, const tbfs_options &o, int *S,
-                             unsigned long long *sigma, cudaStream_t s, BfsCtl *ctl_host);
+/* traversals with results in the internal numbering (api.cu) */
+struct ForwardRoot {
+  int32_t root; /* caller numbering */
+  int *S;       /* n device values each */
+  unsigned long long *sigma;
+};
+tbfs_status forward_internal(tbfs_graph *g, const ForwardRoot *roots, int32_t k,
+                             const tbfs_options &o, cudaStream_t s, BfsCtl **ctl_host);
 }  // namespace tbfs
 
 extern "C" void tbfs_set_error(const char *fmt, ...);
