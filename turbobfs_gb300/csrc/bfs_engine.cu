@@ -48,7 +48,8 @@
  * instances bfs_persistent_kernel<true, .> cut small top-down levels into
  * items of kShortEntries whole queue entries instead, which need no owner
  * search (the chain of dependent L2 round trips is what a small level
- * costs); other graphs run the instance compiled without that path.
+ * costs), and run narrow levels without the global queue (narrow_levels);
+ * other graphs run the instance compiled without these.
  *
  * Direction rule (device side; after Beamer, Asanovic, Patterson,
  * "Direction-optimizing breadth-first search", SC 2012): a level runs
@@ -88,6 +89,9 @@ using dev::global_ns;
 using dev::grid_barrier;
 using dev::warp_find_owner;
 constexpr int kBlock = 1024;       /* threads of a full CTA, one CTA per SM */
+/* ... on short-list graphs: levels that are latency alone want registers (a
+ * barrier's acquire drops L1, so a spilled value costs a round trip to L2) */
+constexpr int kShortBlock = 512;
 constexpr long long kLargeEntries = 48 << 20;
 constexpr int kBlockStep = 256;    /* threads per unit of ctas_per_sm */
 constexpr int kFilterBits = 1 << 18; /* frontier filter in shared memory (32 KB) */
@@ -872,8 +876,312 @@ __device__ __forceinline__ void bu_tile(const BfsParams &p, int d, const NextQue
   }
 }
 
+/* ---- narrow levels of short-list graphs ----
+ * A deep graph has thousands of levels of a few thousand vertices, and such a
+ * level costs the chain of its dependent round trips to L2, not its work:
+ * counter, queue entries, list entries, claim, reservation in the next queue,
+ * barrier.  In a narrow level every CTA keeps the vertices it finds in its own
+ * shared memory and expands them itself in the next one.  Nothing of the
+ * queue goes through L2 then; the lists of the kept vertices, and where their
+ * targets' lists are, are read while the barrier is waited for; and what all
+ * CTAs have to know, the size of the level, comes back with the barrier.
+ * Left between two barriers: one claim.
+ *   Frontiers drift into few CTAs (the faster one claims first), so every
+ * kShareEvery levels, and when a CTA has more than kRound, all finds of a
+ * level go to the global queue, which the next one shares out evenly.  (With
+ * only the finds beyond kRound sent there, such a vertex was expanded three
+ * round trips after the kept ones and lost its targets to them: who had much
+ * got more, and 84 % of a grid's levels used the queue.)
+ *   Grid of 2048 x 2048 with path counts, us per level: 6.5 with every level
+ * through the global queue, 3.1 so (depths only: 2.5).  What is left is the
+ * claim, the fence and the barrier's two trips, ~700 clocks each, and DRAM
+ * misses (0.2 us: a grid of 512 x 512, which fits L2, takes 2.9).  With 256
+ * threads 4.0; sharing every 12 or 96 levels instead of 32: +2 %, +0 %. */
+constexpr unsigned kKeep = 256, kRound = 64;
+constexpr int kShareEvery = 32;
+/* mean vertices per CTA up to which a level is narrow, and starts to be */
+constexpr unsigned kNarrow = 64, kNarrowEnter = 32;
+/* A barrier's 64-bit sum: arrivals, the level's vertices, their out-edges,
+ * CTAs with more than kRound of them. */
+constexpr int kSumCount = 9, kSumEdges = 29, kSumSpill = 55;
+constexpr unsigned kSumGrid = 240; /* CTAs up to which no field can overflow: */
+static_assert((unsigned long long)kNarrow * kSumGrid * kShortList < 1ull << (kSumEdges - kSumCount),
+              "vertices found by a narrow level");
+static_assert((unsigned long long)kNarrow * kSumGrid * kShortList * kShortList <
+                  1ull << (kSumSpill - kSumEdges),
+              "their out-edges");
+static_assert(kSumGrid < 1u << (kSumCount - 1), "arrivals");
+
+struct NarrowState {
+  int v[2][kKeep], a[2][kKeep], deg[2][kKeep]; /* kept vertices of level d in [d & 1] */
+  unsigned found[3], edges[3];   /* found for level d in [d % 3], their out-edges */
+  unsigned long long last[2];    /* the barrier words after their last use        */
+  unsigned long long sum;
+  int ok;
+};
+
+/* One entry (v; list a, deg entries; deg = 0: none) per 2^sub lanes; su, ad,
+ * dg: depth, list start and list length of the lane's first target u.  su may
+ * have been read while other CTAs were in level d - 1 or d already: a target
+ * with su in [0, d] is no child.  Called by all 32 lanes. */
+template <bool SIG>
+__device__ __forceinline__ void narrow_expand(const BfsParams &p, NarrowState &ns, int d, int sub,
+                                              int v, int a, int deg, int u, int su, int ad, int dg,
+                                              bool chk, unsigned cap,
+                                              const NextQueue &nx,
+                                              const unsigned long long *src,
+                                              unsigned long long *dst, bool &ovf) {
+  const int lane = threadIdx.x & 31, b = (d + 1) & 1;
+  const unsigned lt = (1u << lane) - 1u;
+  const unsigned long long x = SIG && deg > 0 ? __ldcg(src + v) : 0ull;
+  for (int j = lane & ((1 << sub) - 1);;) {
+    int old = -2;
+    if (j < deg && (su < 0 || su == d + 1)) old = atomicCAS(p.S + u, -1, d + 1);
+    const bool won = old == -1;
+    if (SIG && (won || old == d + 1)) {
+      if (chk) add_chk(atomicAdd(dst + u, x), x, ovf);
+      else atomicAdd(dst + u, x);
+    }
+    const unsigned m = __ballot_sync(FULL, won);
+    if (m) {
+      const unsigned es = __reduce_add_sync(FULL, won ? (unsigned)dg : 0u);
+      unsigned pos = 0;
+      if (lane == 0) {
+        pos = atomicAdd(&ns.found[(d + 1) % 3], (unsigned)__popc(m));
+        atomicAdd(&ns.edges[(d + 1) % 3], es);
+      }
+      pos = __shfl_sync(FULL, pos, 0);
+      const bool over = pos + (unsigned)__popc(m) > cap;
+      pos += (unsigned)__popc(m & lt);
+      if (won && pos < cap) {
+        ns.v[b][pos] = u;
+        ns.a[b][pos] = ad;
+        ns.deg[b][pos] = dg;
+      }
+      if (over) {
+        const int vv[1] = {u}, gg[1] = {dg}, aa[1] = {ad};
+        warp_append<1>(won && pos >= cap ? 1u : 0u, vv, gg, aa, nx.q, nx.e, nx.a, nx.ctr);
+      }
+    }
+    j += 1 << sub;
+    if (!__any_sync(FULL, j < deg)) break;
+    if (j < deg) {
+      u = __ldg(p.jr + a + j);
+      su = -1;
+      ad = __ldg(p.rp + u);
+      dg = __ldg(p.rp + u + 1) - ad;
+    }
+  }
+}
+
+/* lanes (as a power of two) of an entry, when `n` entries are for `warps` */
+__device__ __forceinline__ int narrow_sub(unsigned n, unsigned warps) {
+  return n <= warps ? 5 : n <= 2u * warps ? 4 : 3;
+}
+
+/* what the rest of the kernel knows of the traversal at level d */
+struct LevelState {
+  int d, td, sig_bits;
+  long long m_u, visited, edges;
+};
+
+enum NarrowEnd { NARROW_DONE, NARROW_LEAVE, NARROW_TIMEOUT, NARROW_INJECTED };
+
+/* Runs narrow levels from l.d on, whose qn vertices with qe out-edges are in
+ * the global queue.  NARROW_LEAVE: level l.d is in the global queue again,
+ * to be run otherwise. */
+template <bool SIG>
+__device__ __forceinline__ NarrowEnd narrow_levels(const BfsParams &p, NarrowState &ns,
+                                                   LevelState &l, unsigned qn, unsigned qe,
+                                                   float alpha, bool &ovf) {
+  BfsCtl *ctl = p.ctl;
+  const unsigned tid = threadIdx.x, lane = tid & 31u, wid = tid >> 5, nw = blockDim.x >> 5;
+  const unsigned gtid = blockIdx.x * blockDim.x + tid, nthreads = gridDim.x * blockDim.x;
+  const unsigned gwarp = wid * gridDim.x + blockIdx.x, nwarps = gridDim.x * nw;
+  /* the warp that waits for the barrier gets kept vertices last */
+  const unsigned kwid = wid == 0u ? nw - 1u : wid - 1u;
+  const unsigned nwords = ((unsigned)p.n + 31u) >> 5;
+  if (!SIG) { /* depths only: no level in between needs its bitmap */
+    for (unsigned i = gtid; i < nwords; i += nthreads)
+      p.fb[l.d % 3][i] = p.fb[(l.d + 2) % 3][i] = 0u;
+  }
+  if (tid < 3) ns.found[tid] = ns.edges[tid] = 0u;
+  __syncthreads();
+  bool global = true, ovf_seen = false; /* vertices of the level are in the global queue */
+  unsigned mine = 0; /* kept by this CTA */
+  int kept_levels = 0;
+  bool crowded = false;
+  int sub = 3, v = 0, a = 0, deg = 0, u = 0, su = -1, ad = 0, dg = 0;
+  for (;;) {
+    const int d = l.d, b = d & 1, c0 = d % 3, c1 = (d + 1) % 3, c2 = (d + 2) % 3;
+    ++l.td;
+    l.visited += qn;
+    l.edges += qe;
+    l.m_u -= qe;
+    if (gtid == 0) {
+      ctl->qctr[c2] = 0ull;
+      ctl->work[(d + 2) & 3] = 0u;
+      if (p.trace && d < p.trace_cap - 1) {
+        long long *rec = p.trace + 4 * (long long)d;
+        rec[0] = (long long)global_ns();
+        rec[1] = qn;
+        rec[2] = qe;
+        rec[3] = DIR_TD;
+      }
+    }
+    if (tid == 0) ns.found[c2] = ns.edges[c2] = 0u;
+    const unsigned long long gq = global ? __ldcg(&ctl->qctr[c0]) : 0ull;
+    const bool chk = SIG && !ovf_seen && !(p.deg_bits > 0 && l.sig_bits + p.deg_bits <= 63);
+    const bool share = crowded || ++kept_levels > kShareEvery;
+    const unsigned cap = share ? 0u : kKeep;
+    if (share) kept_levels = 0;
+    const NextQueue nx = {p.q[b ^ 1], p.e[b ^ 1], p.a[b ^ 1], &ctl->qctr[c1]};
+    const unsigned long long *src = b ? p.sigma_odd : p.sigma;
+    unsigned long long *dst = b ? p.sigma : p.sigma_odd;
+    /* kept vertices: the first round's loads are done */
+    unsigned i = kwid << (5 - sub);
+    if (i < mine)
+      narrow_expand<SIG>(p, ns, d, sub, v, a, deg, u, su, ad, dg, chk, cap, nx, src, dst, ovf);
+    for (i += nw << (5 - sub); i < mine; i += nw << (5 - sub)) {
+      const unsigned k = i + (lane >> sub);
+      const int j = (int)(lane & ((1u << sub) - 1u));
+      deg = k < mine ? ns.deg[b][k] : 0;
+      v = a = u = ad = dg = 0;
+      if (deg) v = ns.v[b][k], a = ns.a[b][k];
+      if (j < deg) {
+        u = __ldg(p.jr + a + j);
+        ad = __ldg(p.rp + u);
+        dg = __ldg(p.rp + u + 1) - ad;
+      }
+      narrow_expand<SIG>(p, ns, d, sub, v, a, deg, u, -1, ad, dg, chk, cap, nx, src, dst, ovf);
+    }
+    /* a share of the global queue */
+    const unsigned gn = (unsigned)(gq >> 32);
+    const int gsub = narrow_sub(gn, nwarps);
+    for (i = gwarp << (5 - gsub); i < gn; i += nwarps << (5 - gsub)) {
+      const unsigned k = i + (lane >> gsub);
+      const int j = (int)(lane & ((1u << gsub) - 1u));
+      v = a = deg = u = ad = dg = 0;
+      if (k < gn) {
+        v = __ldcg(p.q[b] + k);
+        a = __ldcg(p.a[b] + k);
+        deg = (int)((k + 1u < gn ? (unsigned)__ldcg(p.e[b] + k + 1u) : (unsigned)gq) -
+                    (unsigned)__ldcg(p.e[b] + k));
+      }
+      if (j < deg) {
+        u = __ldg(p.jr + a + j);
+        ad = __ldg(p.rp + u);
+        dg = __ldg(p.rp + u + 1) - ad;
+      }
+      narrow_expand<SIG>(p, ns, d, gsub, v, a, deg, u, -1, ad, dg, chk, cap, nx, src, dst, ovf);
+    }
+    if (p.inject_barrier_skip > 0 && blockIdx.x == 0 && d == p.inject_barrier_skip - 1)
+      return NARROW_INJECTED;
+    if (SIG && __any_sync(FULL, ovf) && lane == 0) atomicOr(&ctl->sigma_overflow, 1);
+
+    /* Barrier with a sum, as grid_barrier otherwise: a level's arrivals add
+     * 2^(kSumCount - 1), whose bit changes with the last one, and each adds
+     * its CTA's figures above.  The sum is the difference to the word after
+     * its last use; two words are used in turn, so that a CTA already at the
+     * next barrier does not change what a slower one is still to read. */
+    __syncthreads();
+    constexpr unsigned kFlip = 1u << (kSumCount - 1);
+    const unsigned found = ns.found[c1];
+    if (tid == 0) {
+      const unsigned long long add =
+          (blockIdx.x == 0 ? kFlip - (gridDim.x - 1u) : 1u) +
+          ((unsigned long long)found << kSumCount) +
+          ((unsigned long long)ns.edges[c1] << kSumEdges) +
+          (!share && found > kRound ? 1ull << kSumSpill : 0ull);
+      asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(&ctl->sum[b].word), "l"(add)
+                   : "memory");
+    }
+    /* meanwhile: the lists of the kept vertices, and the depths of their
+     * targets, some of which may be level d + 2's already */
+    mine = found < cap ? found : cap;
+    sub = narrow_sub(mine, nw - 1u);
+    {
+      const unsigned k = (kwid << (5 - sub)) + (lane >> sub);
+      const int j = (int)(lane & ((1u << sub) - 1u));
+      deg = k < mine ? ns.deg[b ^ 1][k] : 0;
+      v = a = u = ad = dg = 0;
+      su = -1;
+      if (deg) v = ns.v[b ^ 1][k], a = ns.a[b ^ 1][k];
+      if (j < deg) {
+        u = __ldg(p.jr + a + j);
+        su = __ldcg(p.S + u);
+        if (SIG) /* its count, to be added to: 3.46 -> 3.25 us per level */
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(src + u));
+        ad = __ldg(p.rp + u);
+        dg = __ldg(p.rp + u + 1) - ad;
+      }
+      if (SIG && !ovf_seen) ovf_seen = __ldcg(&ctl->sigma_overflow) != 0;
+    }
+    if (tid == 0) {
+      const unsigned long long last = ns.last[b];
+      const unsigned long long t0 = global_ns();
+      unsigned long long w;
+      unsigned spins = 0;
+      int ok = 1;
+      for (;;) {
+        asm volatile("ld.acquire.gpu.global.u64 %0, [%1];"
+                     : "=l"(w)
+                     : "l"(&ctl->sum[b].word)
+                     : "memory");
+        if (((w ^ last) & kFlip) != 0ull) break;
+        if ((++spins & 31u) == 0) {
+          if (dev::ld_volatile(&ctl->status) != 0) {
+            ok = 0;
+            break;
+          }
+          if ((long long)(global_ns() - t0) > p.timeout_ns) {
+            atomicCAS(&ctl->status, 0, (int)TBFS_ERR_TIMEOUT);
+            atomicCAS(&ctl->timeout_level, 0, d + 2);
+            ok = 0;
+            break;
+          }
+        }
+      }
+      ns.ok = ok;
+      ns.sum = w - last;
+      ns.last[b] = w;
+    }
+    __syncthreads();
+    if (!ns.ok) return NARROW_TIMEOUT;
+    const unsigned long long sum = ns.sum;
+    qn = (unsigned)(sum >> kSumCount) & ((1u << (kSumEdges - kSumCount)) - 1u);
+    qe = (unsigned)(sum >> kSumEdges) & ((1u << (kSumSpill - kSumEdges)) - 1u);
+    crowded = (sum >> kSumSpill) != 0ull;
+    global = share || crowded; /* more than kRound may be more than kKeep */
+    l.sig_bits = l.sig_bits + p.deg_bits < 64 ? l.sig_bits + p.deg_bits : 64;
+    ++l.d;
+    if (qn == 0u) return NARROW_DONE;
+    if (qn > kNarrow * gridDim.x ||
+        (p.mode != TBFS_MODE_TOP_DOWN &&
+         (float)qe * alpha > (float)(l.m_u - qe) + kBuWordCost * (float)nwords)) {
+      if (wid < (mine + 31u) / 32u) { /* level d + 1 to the global queue */
+        const unsigned k = tid;
+        const int vv[1] = {k < mine ? ns.v[b ^ 1][k] : 0};
+        const int gg[1] = {k < mine ? ns.deg[b ^ 1][k] : 0};
+        const int aa[1] = {k < mine ? ns.a[b ^ 1][k] : 0};
+        warp_append<1>(k < mine ? 1u : 0u, vv, gg, aa, nx.q, nx.e, nx.a, nx.ctr);
+      }
+      if (!grid_barrier(ctl, p.timeout_ns, d)) return NARROW_TIMEOUT;
+      if (!SIG) { /* and its bitmap */
+        for (unsigned k = gtid; k < qn; k += nthreads) {
+          const unsigned t = (unsigned)__ldcg(nx.q + k);
+          atomicOr(p.fb[c1] + (t >> 5), 1u << (t & 31u));
+        }
+        if (!grid_barrier(ctl, p.timeout_ns, d)) return NARROW_TIMEOUT;
+      }
+      return NARROW_LEAVE;
+    }
+  }
+}
+
 template <bool SHORT, bool SIG>
-__global__ void __launch_bounds__(kBlock, 1) bfs_persistent_kernel(const BfsParams p) {
+__global__ void __launch_bounds__(SHORT ? kShortBlock : kBlock, 1)
+    bfs_persistent_kernel(const BfsParams p) {
   /* a window per warp, then the frontier filter (instance <false, true>) */
   extern __shared__ __align__(16) unsigned char s_dyn[];
   ExpandWin *s_win = reinterpret_cast<ExpandWin *>(s_dyn);
@@ -885,6 +1193,12 @@ __global__ void __launch_bounds__(kBlock, 1) bfs_persistent_kernel(const BfsPara
   const unsigned nwarps = nthreads >> 5;
   BfsCtl *ctl = p.ctl;
   constexpr bool want_sigma = SIG;
+  NarrowState *ns = nullptr;
+  if constexpr (SHORT) {
+    __shared__ NarrowState s_narrow;
+    ns = &s_narrow;
+    if (threadIdx.x == 0) ns->last[0] = ns->last[1] = 0ull;
+  }
   const int root = p.inv ? __ldg(p.inv + p.root) : p.root; /* internal numbering */
 
   /* init: S = -1, counts 0, root at depth 0 with one path; depths only:
@@ -953,6 +1267,25 @@ __global__ void __launch_bounds__(kBlock, 1) bfs_persistent_kernel(const BfsPara
     if (qn == 0) {
       done = true;
       break;
+    }
+    if constexpr (SHORT) {
+      if (dir == DIR_TD && p.mode != TBFS_MODE_BOTTOM_UP && qn <= kNarrowEnter * gridDim.x &&
+          gridDim.x <= kSumGrid &&
+          (p.mode == TBFS_MODE_TOP_DOWN ||
+           !((float)qe * alpha > (float)(m_u - qe) + kBuWordCost * (float)nwords))) {
+        LevelState l = {d, td, sig_bits, m_u, visited, edges};
+        const NarrowEnd end = narrow_levels<SIG>(p, *ns, l, qn, qe, alpha, ovf);
+        if (end == NARROW_INJECTED) return;
+        d = l.d;
+        td = l.td;
+        sig_bits = l.sig_bits;
+        m_u = l.m_u;
+        visited = l.visited;
+        edges = l.edges;
+        if (end == NARROW_LEAVE) continue;
+        done = end == NARROW_DONE;
+        break;
+      }
     }
     visited += qn;
     edges += qe;
@@ -1217,14 +1550,15 @@ cudaError_t bfs_geometry(int device, LaunchGeom *out) {
   if (e != cudaSuccess) return e;
   for (int k = 0; k < 4; ++k) { /* carve out what a CTA needs, the rest is L1 */
     const void *fn = bfs_kernel((k & 1) != 0, (k & 2) != 0);
-    const size_t need = bfs_smem(kBlock, k == 2);
-    const int carve = (int)((100 * (need + 1024) + (size_t)smem_sm - 1) / (size_t)smem_sm);
+    const int most = (k & 1) ? kShortBlock : kBlock;
+    const size_t need = bfs_smem(most, k == 2);
+    const int carve = (int)((100 * (need + sizeof(NarrowState) + 1024) + (size_t)smem_sm - 1) / (size_t)smem_sm);
     e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need);
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout,
                                carve < 100 ? carve : 100);
     int fit = 0;
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, fn, kBlock, need);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, fn, most, need);
     if (e != cudaSuccess) return e;
     if (fit < 1) return cudaErrorInvalidConfiguration;
   }
@@ -1236,8 +1570,8 @@ cudaError_t bfs_geometry(int device, LaunchGeom *out) {
 }
 
 cudaError_t bfs_launch(const BfsParams &p0, const LaunchGeom &g, cudaStream_t s) {
-  /* One CTA per SM, of 256 threads per unit of ctas_per_sm.  By default 2 on
-   * short-list graphs, whose levels are many and small; 4 for depths only and
+  /* One CTA per SM, of 256 threads per unit of ctas_per_sm.  By default (and at
+   * most) 2 on short-list graphs, whose levels are many and small; 4 for depths only and
    * on large graphs regrouped by degree, whose heavy levels want every warp;
    * else 3, which leaves more L1 and costs less at every barrier (ms per BFS
    * with path counts at 3 / 4: RMAT-22 0.487 / 0.445, Erdos-Renyi of 2.5 M
@@ -1247,7 +1581,8 @@ cudaError_t bfs_launch(const BfsParams &p0, const LaunchGeom &g, cudaStream_t s)
   const bool short_lists = p.short_lists != 0, sigma = p.sigma != nullptr;
   const bool full = !sigma || (p.inv && p.nnz > kLargeEntries);
   const int want = p.ctas_per_sm > 0 ? p.ctas_per_sm : short_lists ? 2 : full ? 4 : 3;
-  const int block = want < g.per_sm ? kBlockStep * want : g.block;
+  int block = want < g.per_sm ? kBlockStep * want : g.block;
+  if (short_lists && block > kShortBlock) block = kShortBlock;
   p.filter = !short_lists && sigma && p.tile && (double)p.nnz > kHeavyEntries;
   void *args[] = {&p};
   return cudaLaunchCooperativeKernel(bfs_kernel(short_lists, sigma), dim3(g.grid), dim3(block), args,

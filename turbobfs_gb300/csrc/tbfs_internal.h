@@ -49,6 +49,13 @@ struct __align__(128) GridBarrier {
   unsigned pad0[31];
 };
 
+/* Word of a barrier that also adds up counts over the grid (bfs_engine.cu),
+ * on its own 128-byte line. */
+struct __align__(128) SumBarrier {
+  unsigned long long word;
+  unsigned pad0[30];
+};
+
 /* Device control block of one traversal; zeroed before every launch. */
 struct __align__(128) BfsCtl {
   /* slot d % 3 accumulates the queue of level d+1 ... see bfs_engine.cu */
@@ -62,6 +69,7 @@ struct __align__(128) BfsCtl {
   unsigned long long collect; /* queue of a level found bottom-up: (count << 32) | edges */
   unsigned int pad0[8];
   GridBarrier bar;
+  SumBarrier sum[2]; /* used in turn */
 };
 
 struct BfsParams {
