@@ -74,6 +74,17 @@ void carve(unsigned char *base, int n, bool sigma, InstDesc &D) {
   }
 }
 
+/* memory of this device that a kernel can write elements of `align` bytes to;
+ * outputs elsewhere (a peer's, unaligned) are copied */
+bool own_memory(const void *p, int device, size_t align) {
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return at.type == cudaMemoryTypeDevice && at.device == device && (uintptr_t)p % align == 0;
+}
+
 void fill_stats(const InstDesc &D, float ms, tbfs_stats *st) {
   memset(st, 0, sizeof(*st));
   st->levels = D.levels;
@@ -298,11 +309,14 @@ extern "C" tbfs_status tbfs_arena_bfs(tbfs_arena *a, const int32_t *roots, const
     MTRY(tbfs::dev_alloc(&a->work, tot), "arena traversal buffers");
     a->work_sigma = want_sigma;
   }
+  const bool packed = o.outputs_on_device && own_memory(S, a->device, sizeof(int)) &&
+                      (!want_sigma || own_memory(sigma, a->device, 8));
   const long long timeout = o.timeout_ns > 0 ? o.timeout_ns : 4000000000LL;
   const int cap = tbfs::kMultiMaxSlots;
   for (int32_t g0 = 0; g0 < a->g; g0 += cap) {
     const int k = std::min<int32_t>(cap, a->g - g0);
     std::vector<int> ids((size_t)k);
+    int n_most = 0;
     for (int j = 0; j < k; ++j) {
       const int i = g0 + j;
       InstDesc &D = a->inst_host[j];
@@ -317,8 +331,8 @@ extern "C" tbfs_status tbfs_arena_bfs(tbfs_arena *a, const int32_t *roots, const
       D.deg_bits = a->deg_bits[(size_t)i];
       D.root = roots[i];
       carve(a->work + a->woff[(size_t)i], D.n, want_sigma, D);
-      MTRY(cudaMemsetAsync(D.S, 0xff, (size_t)D.n * sizeof(int), s), "clear S");
-      if (D.sig) MTRY(cudaMemsetAsync(D.sig, 0, (size_t)D.n * 8, s), "clear sigma");
+      D.out = (long long)a->voff[(size_t)i];
+      n_most = std::max(n_most, D.n);
       ids[(size_t)j] = j;
     }
     MTRY(cudaMemcpyAsync(a->inst, a->inst_host, (size_t)k * sizeof(InstDesc),
@@ -326,7 +340,7 @@ extern "C" tbfs_status tbfs_arena_bfs(tbfs_arena *a, const int32_t *roots, const
          "descriptors");
     MTRY(cudaMemcpyAsync(a->slots, ids.data(), (size_t)k * sizeof(int), cudaMemcpyHostToDevice, s),
          "slots");
-    MTRY(tbfs::multi_init(a->inst, a->slots, k, s), "init");
+    MTRY(tbfs::multi_init(a->inst, a->slots, k, n_most, s), "init");
     MTRY(cudaMemsetAsync(a->ctl, 0, sizeof(MultiCtl), s), "clear control block");
     MultiParams p;
     p.inst = a->inst;
@@ -345,7 +359,11 @@ extern "C" tbfs_status tbfs_arena_bfs(tbfs_arena *a, const int32_t *roots, const
     MTRY(cudaMemcpyAsync(a->ctl_host, a->ctl, sizeof(MultiCtl), cudaMemcpyDeviceToHost, s),
          "read control block");
     /* results: the packed layout is the arena's own (no renumbering) */
-    for (int j = 0; j < k; ++j) {
+    if (packed)
+      MTRY(tbfs::multi_pack(a->inst, k, n_most, S,
+                            want_sigma ? reinterpret_cast<unsigned long long *>(sigma) : nullptr, s),
+           "pack");
+    for (int j = 0; j < k && !packed; ++j) {
       const int i = g0 + j;
       const InstDesc &D = a->inst_host[j];
       const size_t vo = (size_t)a->voff[(size_t)i];
@@ -597,8 +615,8 @@ void run_plain(tbfs_server *sv, const std::shared_ptr<Request> &r) {
     sv->cv_done.notify_all();
 }
 
-/* one step of the loop: admit, advance every instance up to max_phases
- * levels in one launch, retire the finished ones */
+/* one step of the loop: admit, advance every instance in one launch, retire the
+ * finished ones */
 tbfs_status server_step(tbfs_server *sv, bool *idle) {
   std::vector<int> admitted;
   int waiting = 0;
@@ -647,6 +665,7 @@ tbfs_status server_step(tbfs_server *sv, bool *idle) {
     *sv->wake_host = 0; /* a submit from now on ends the next launch early */
   }
   cudaStream_t s = sv->stream;
+  int n_most = 0;
   for (int i : admitted) {
     Slot &sl = sv->slots[(size_t)i];
     const Request &r = *sl.req;
@@ -662,8 +681,7 @@ tbfs_status server_step(tbfs_server *sv, bool *idle) {
     D.deg_bits = r.g->deg_bits;
     D.root = r.root;
     carve(sv->mem + sl.off, D.n, r.sigma != nullptr, D);
-    MTRY(cudaMemsetAsync(D.S, 0xff, (size_t)D.n * sizeof(int), s), "clear S");
-    if (D.sig) MTRY(cudaMemsetAsync(D.sig, 0, (size_t)D.n * 8, s), "clear sigma");
+    n_most = std::max(n_most, D.n);
   }
   int nslots = 0;
   for (int i = 0; i < sv->max_slots; ++i) {
@@ -674,6 +692,8 @@ tbfs_status server_step(tbfs_server *sv, bool *idle) {
   }
   *idle = nslots == 0;
   if (nslots == 0) return TBFS_OK;
+  std::vector<int> level0((size_t)nslots);
+  for (int i = 0; i < nslots; ++i) level0[(size_t)i] = sv->inst_host[i].levels;
   MTRY(cudaMemcpyAsync(sv->inst, sv->inst_host, (size_t)nslots * sizeof(InstDesc),
                        cudaMemcpyHostToDevice, s),
        "descriptors");
@@ -682,7 +702,8 @@ tbfs_status server_step(tbfs_server *sv, bool *idle) {
     MTRY(cudaMemcpyAsync(sv->slot_ids, sv->slot_ids_host, admitted.size() * sizeof(int),
                          cudaMemcpyHostToDevice, s),
          "slots");
-    MTRY(tbfs::multi_init(sv->inst, sv->slot_ids, (int)admitted.size(), s), "init");
+    MTRY(tbfs::multi_init(sv->inst, sv->slot_ids, (int)admitted.size(), n_most, s),
+         "init");
   }
   /* The launch runs until a query finishes (its results are delivered at
    * once and its memory freed) or, unless queries already wait for memory
@@ -708,7 +729,10 @@ tbfs_status server_step(tbfs_server *sv, bool *idle) {
   {
     std::lock_guard<std::mutex> lk(sv->mu);
     sv->launches++;
-    sv->levels_run += sv->ctl_host->phases;
+    int most = 0; /* levels that the launch took some query on */
+    for (int i = 0; i < nslots; ++i)
+      most = std::max(most, sv->inst_host[i].levels - level0[(size_t)i]);
+    sv->levels_run += most;
     sv->slot_sum += nslots;
     sv->launch_ns += std::chrono::duration_cast<std::chrono::nanoseconds>(t_deliver - t_launch).count();
   }

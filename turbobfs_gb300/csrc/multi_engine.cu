@@ -25,9 +25,17 @@
  * and the owner of each edge by a 32-ary search over the instance's
  * out-degree prefix (first round) followed by a shuffle search in a window
  * of 64 queue entries.
+ *
+ * Small levels stay out of that: an instance whose frontier fits one CTA is
+ * run by that CTA alone, level after level, with its queue in shared memory
+ * and no grid barrier (local_run), while the other CTAs advance the wide
+ * instances.  A phase is then one level of every wide instance and as many
+ * of the others as fit in its time.
  */
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <algorithm>
 
 #include "device_common.cuh"
 #include "tbfs_internal.h"
@@ -39,13 +47,73 @@ using dev::FULL;
 using dev::grid_barrier;
 
 #ifndef TBFS_MULTI_PER_SM
-#define TBFS_MULTI_PER_SM 3
+#define TBFS_MULTI_PER_SM 1
 #endif
 
-constexpr int kBlock = 256;
+constexpr int kBlock = 768;
 constexpr int kEPT = 4;                   /* consecutive edges per lane per round */
 constexpr unsigned kRoundEdges = 32 * kEPT;
 constexpr int kMaxRounds = 8;             /* rounds per item, fewer on small levels */
+
+constexpr int kInitBlock = 256;
+
+/* ---- instances run by one CTA ----
+ * A level that all CTAs share costs ~11 us, however small: plan, work prefix,
+ * queue entries, owners, lists, claims, reservation and barrier are dependent
+ * round trips to L2 or follow one.  One CTA with the queue in shared memory
+ * has two or three (list entry, depth, where the found one's list is) and two
+ * __syncthreads.  What bounds a larger level is the SM's path to L2, one
+ * scattered access per 1-3 clocks (and an atomic in ~4), so as little as
+ * possible goes there: lists are read by consecutive lanes, the queue and its
+ * counts stay in shared memory, and since nobody else touches the instance
+ * meanwhile, the vertices found by a level are the keys of a hash table whose
+ * slots add up the counts, stored once; a vertex whose kProbe slots are taken
+ * by others is claimed and counted in L2.  (A claim and an add in L2 per edge,
+ * both ends of every target's list and the source's count from L2: 9 us for
+ * a level of 2300 edges.)
+ *   A level of up to kLocalEnter edges costs less so than shared; an instance
+ * is given back when it has outgrown kLocalLeave or the queue.  (192
+ * graphs of 2^10 to 2^18 vertices: 12.5 -> 5.0 ms, of which 3.3 ms were two
+ * memsets and two copies per graph on the host; 28 queries to a server of 14
+ * such graphs: 8.3 -> 5.2 ms.  Us per level of a grid of 2^17.5 vertices,
+ * ~2300 edges: 9.6 shared, 5.7 so; of 2^14, 10.2 and 3.3.  768 threads and
+ * one CTA per SM against two of 384: 5.7 and 8.6.) */
+constexpr unsigned kLocalQueue = 2048;
+constexpr unsigned kSlotBits = 12, kSlots = 1u << kSlotBits, kProbe = 24;
+constexpr unsigned kNoKey = 0xffffffffu, kNoSlot = 0xffffu;
+constexpr unsigned kLocalEnter = 12288, kLocalLeave = 24576;
+/* A CTA gives its instance back for the next phase after this long: alone, so
+ * that no CTA waits long at the barrier; beside wide instances, about a
+ * shared level's time.  (In clocks of ~0.5 ns: the ns timer is slow to read.) */
+constexpr long long kLocalAlone = 500000, kLocalBeside = 60000;
+constexpr int kLocalMine = 16;            /* instances of one CTA in a phase */
+constexpr unsigned kLocalGrid = kMultiMaxSlots / kLocalMine + 1; /* CTAs for that */
+constexpr unsigned kIsLocal = 0x80000000u;
+
+struct LocalShared {
+  int v[2][kLocalQueue], a[2][kLocalQueue]; /* level d in [d & 1]: vertex, list start */
+  unsigned e[2][kLocalQueue];               /* exclusive prefix of out-degrees        */
+  unsigned long long cnt[2][kLocalQueue];   /* path counts                            */
+  unsigned key[kSlots], lo[kSlots], hi[kSlots]; /* vertices of the next level, counts */
+  unsigned long long ctr[3];                /* level d: (count << 32) | out-edges     */
+  int leave[2];
+  unsigned short slot[kLocalQueue];         /* of the next level's entries            */
+};
+
+/* u's slot in the table, entered if it is not there (*is_new); kNoSlot if all its
+ * slots are others'.  Entries only come during a level, so every thread that
+ * looks for u finds the same answer. */
+__device__ __forceinline__ unsigned find_slot(LocalShared &L, unsigned u, bool *is_new) {
+  unsigned s = (u * 0x9e3779b1u) >> (32 - kSlotBits);
+  for (unsigned p = 0; p < kProbe; ++p, s = (s + 1u) & (kSlots - 1u)) {
+    const unsigned k = atomicCAS(&L.key[s], kNoKey, u);
+    if (k == kNoKey || k == u) {
+      *is_new = k != u;
+      return s;
+    }
+  }
+  return kNoSlot;
+}
 
 /* Append, for every lane and every bit j of take, (v[j], out-degree dg[j])
  * to a queue: one 64-bit atomic per warp reserves (count << 32 | edge sum),
@@ -101,14 +169,242 @@ __device__ __forceinline__ unsigned lane_owner(const unsigned *e, unsigned cnt, 
   return lo;
 }
 
+/* This CTA runs instance D from level d on (qn vertices, qe out-edges) until
+ * it is finished or has outgrown a CTA, the clock t_end, or a stop request. */
+__device__ __forceinline__ void local_run(const MultiParams &P, InstDesc &D, LocalShared &L, int d,
+                                          unsigned qn, unsigned qe, unsigned ph,
+                                          long long t_end) {
+  const int t = threadIdx.x, lane = t & 31;
+  const unsigned wid = (unsigned)t >> 5;
+  const int *rp = D.rp, *jr = D.jr;
+  int *S = D.S;
+  unsigned long long *sig = D.sig;
+  for (unsigned i = t; i < qn; i += kBlock) {
+    const int v = __ldcg(D.q[d % 3] + i);
+    L.v[d & 1][i] = v;
+    L.e[d & 1][i] = __ldcg(D.e[d % 3] + i);
+    L.a[d & 1][i] = __ldg(rp + v);
+    if (sig) L.cnt[d & 1][i] = __ldcg(sig + v);
+  }
+  for (unsigned i = t; i < kSlots; i += kBlock) {
+    L.key[i] = kNoKey;
+    L.lo[i] = L.hi[i] = 0u;
+  }
+  if (t < 3) L.ctr[t] = 0ull;
+  __syncthreads();
+  const int bits = D.deg_bits;
+  const bool ovf_seen = __ldcg(&D.ovf) != 0;
+  long long visited = 0, edges = 0;
+  bool ovf = false;
+  for (;;) {
+    const int b = d & 1, c1 = (d + 1) % 3;
+    visited += qn;
+    edges += qe;
+    int stop = 0;
+    if (t == 0) {
+      L.ctr[(d + 2) % 3] = 0ull;
+      stop = dev::ld_volatile(&P.ctl->stop[ph & 1u]);
+    }
+    const bool chk = sig && !ovf_seen && !(bits > 0 && 1 + (long long)(d + 1) * bits <= 63);
+    /* a contiguous piece of the level's edges per warp, up to kEPT rounds of
+     * 32 in flight */
+    const unsigned steps = (qe + kBlock - 1u) / kBlock;
+    const unsigned lim = min(qe, (wid + 1u) * steps * 32u);
+    const bool early = steps <= 2u; /* latency counts: where the targets' lists are, unasked */
+    const unsigned *le = L.e[b];
+    unsigned base = wid * steps * 32u, i0 = 0;
+    if (base < qe) { /* largest entry with e <= base */
+      unsigned hi = qn;
+      while (hi - i0 > 1) {
+        const unsigned mid = (i0 + hi) >> 1;
+        if (le[mid] <= base) i0 = mid;
+        else hi = mid;
+      }
+    }
+    for (; base < lim; base += 32u * kEPT) {
+      int u[kEPT];
+      unsigned k[kEPT];
+      bool on[kEPT];
+#pragma unroll
+      for (int j = 0; j < kEPT; ++j) {
+        /* owner within the 32 entries from the last one's; past them (many
+         * empty lists) step by step */
+        const unsigned tj = base + 32u * j + lane;
+        on[j] = tj < lim;
+        u[j] = 0;
+        k[j] = 0;
+        if (base + 32u * j >= lim) continue; /* the whole warp */
+        const unsigned w = i0 + lane < qn ? le[i0 + lane] : 0xffffffffu;
+        unsigned o = 0;
+#pragma unroll
+        for (int h = 16; h > 0; h >>= 1)
+          if (__shfl_sync(FULL, w, (int)(o + h)) <= tj) o += h;
+        o += i0;
+        if (on[j]) {
+          while (o + 1 < qn && le[o + 1] <= tj) ++o;
+          k[j] = o;
+          u[j] = __ldg(jr + L.a[b][o] + (int)(tj - le[o]));
+        }
+        i0 = __shfl_sync(FULL, o, 31);
+      }
+      int sv[kEPT], ad[kEPT];
+      unsigned dg[kEPT];
+#pragma unroll
+      for (int j = 0; j < kEPT; ++j) {
+        sv[j] = 0;
+        ad[j] = 0;
+        dg[j] = 0u;
+        if (on[j]) {
+          sv[j] = __ldcg(S + u[j]);
+          if (early) {
+            ad[j] = __ldg(rp + u[j]);
+            dg[j] = (unsigned)__ldg(rp + u[j] + 1);
+          }
+        }
+      }
+      unsigned cnt = 0, dsum = 0, won = 0, sl[kEPT];
+#pragma unroll
+      for (int j = 0; j < kEPT; ++j) {
+        sl[j] = kNoSlot;
+        /* not reached before this level (d + 1: just claimed by another lane) */
+        on[j] = on[j] && (sv[j] == -1 || sv[j] == d + 1);
+        if (on[j]) {
+          bool is_new = false;
+          sl[j] = find_slot(L, (unsigned)u[j], &is_new);
+          if (is_new) S[u[j]] = d + 1;
+          if (sl[j] == kNoSlot) is_new = atomicCAS(S + u[j], -1, d + 1) == -1;
+          if (is_new) won |= 1u << j;
+        }
+        if (!early && ((won >> j) & 1u)) {
+          ad[j] = __ldg(rp + u[j]);
+          dg[j] = (unsigned)__ldg(rp + u[j] + 1);
+        }
+      }
+      if (sig) { /* low words of all, then the carries and high words */
+        unsigned long long x[kEPT];
+        unsigned up[kEPT];
+#pragma unroll
+        for (int j = 0; j < kEPT; ++j) {
+          up[j] = 0u;
+          x[j] = on[j] ? L.cnt[b][k[j]] : 0ull;
+          if (on[j] && sl[j] != kNoSlot) up[j] = atomicAdd(&L.lo[sl[j]], (unsigned)x[j]);
+        }
+#pragma unroll
+        for (int j = 0; j < kEPT; ++j) {
+          if (on[j] && sl[j] != kNoSlot) {
+            const unsigned carry = up[j] + (unsigned)x[j] < up[j] ? 1u : 0u;
+            const unsigned xh = (unsigned)(x[j] >> 32), add = xh + carry;
+            if (add < xh) ovf = true;
+            if (add) {
+              const unsigned old = atomicAdd(&L.hi[sl[j]], add);
+              if (old + add < old || (old + add) >> 31) ovf = true;
+            }
+          } else if (on[j]) {
+            if (chk) dev::add_chk(atomicAdd(sig + u[j], x[j]), x[j], ovf);
+            else atomicAdd(sig + u[j], x[j]);
+          }
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < kEPT; ++j) {
+        dg[j] -= (unsigned)ad[j];
+        if ((won >> j) & 1u) {
+          ++cnt;
+          dsum += dg[j];
+        }
+      }
+      if (!__any_sync(FULL, cnt)) continue;
+      unsigned ic = cnt, id = dsum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned tc = __shfl_up_sync(FULL, ic, o), td = __shfl_up_sync(FULL, id, o);
+        if (lane >= o) {
+          ic += tc;
+          id += td;
+        }
+      }
+      unsigned long long at = 0;
+      if (lane == 31) at = atomicAdd(&L.ctr[c1], ((unsigned long long)ic << 32) | id);
+      at = __shfl_sync(FULL, at, 31);
+      unsigned pos = (unsigned)(at >> 32) + ic - cnt, eo = (unsigned)at + id - dsum;
+#pragma unroll
+      for (int j = 0; j < kEPT; ++j) {
+        if ((won >> j) & 1u) {
+          if (pos < kLocalQueue) {
+            L.slot[pos] = (unsigned short)sl[j];
+            L.v[b ^ 1][pos] = u[j];
+            L.a[b ^ 1][pos] = ad[j];
+            L.e[b ^ 1][pos] = eo;
+          } else { /* more than fit: where the instance's queue has them */
+            D.q[c1][pos] = u[j];
+            D.e[c1][pos] = eo;
+          }
+          ++pos;
+          eo += dg[j];
+        }
+      }
+    }
+    if (t == 0) L.leave[b] = stop || clock64() > t_end;
+    __syncthreads();
+    ++d;
+    const unsigned long long cur = L.ctr[c1];
+    qn = (unsigned)(cur >> 32);
+    qe = (unsigned)cur;
+    /* the counts to memory, and the table empty again */
+    if (qn <= kLocalQueue) {
+      for (unsigned i = t; i < qn; i += kBlock) {
+        const unsigned s = L.slot[i];
+        const int v = L.v[b ^ 1][i];
+        if (s != kNoSlot) {
+          const unsigned long long x = ((unsigned long long)L.hi[s] << 32) | L.lo[s];
+          if (sig) sig[v] = L.cnt[b ^ 1][i] = x;
+          L.key[s] = kNoKey;
+          L.lo[s] = L.hi[s] = 0u;
+        } else if (sig) {
+          L.cnt[b ^ 1][i] = __ldcg(sig + v);
+        }
+      }
+    } else if (sig) { /* the instance leaves */
+      for (unsigned s = t; s < kSlots; s += kBlock)
+        if (L.key[s] != kNoKey) sig[L.key[s]] = ((unsigned long long)L.hi[s] << 32) | L.lo[s];
+    }
+    if (qn == 0u || qn > kLocalQueue || qe > kLocalLeave || L.leave[b]) {
+      for (unsigned i = t; i < qn && i < kLocalQueue; i += kBlock) {
+        D.q[c1][i] = L.v[b ^ 1][i];
+        D.e[c1][i] = L.e[b ^ 1][i];
+      }
+      if (__any_sync(FULL, ovf) && lane == 0) atomicExch(&D.ovf, 1);
+      if (t == 0) {
+        D.ctr[c1] = cur;
+        D.ctr[(d + 1) % 3] = 0ull;
+        D.ctr[(d + 2) % 3] = 0ull;
+        D.d = d;
+        D.levels = d;
+        D.visited = __ldcg(&D.visited) + visited;
+        D.edges = __ldcg(&D.edges) + edges;
+        if (qn == 0u) {
+          D.done = 1;
+          if (P.stop_on_done) *(volatile int *)&P.ctl->stop[ph & 1u] = 1;
+        }
+      }
+      __syncthreads(); /* before the next instance's queue */
+      return;
+    }
+    __syncthreads();
+  }
+}
+
 __global__ void __launch_bounds__(kBlock, TBFS_MULTI_PER_SM) multi_bfs_kernel(const MultiParams P) {
+  extern __shared__ __align__(16) unsigned char s_dyn[];
+  LocalShared &L = *reinterpret_cast<LocalShared *>(s_dyn);
+  __shared__ int s_mine[kLocalMine];             /* this CTA's instances */
   constexpr int kWarps = kBlock / 32;
   __shared__ unsigned s_pre[kMultiMaxSlots + 1]; /* item prefix over slots      */
   __shared__ int s_d[kMultiMaxSlots];            /* level each slot runs next   */
   __shared__ unsigned s_qn[kMultiMaxSlots], s_qe[kMultiMaxSlots];
   __shared__ unsigned long long s_wsum[kWarps];  /* per-warp edge sums          */
   __shared__ int s_wact[kWarps];
-  __shared__ unsigned s_wscan[kWarps];           /* per-warp item sums          */
+  __shared__ unsigned long long s_wscan[kWarps]; /* per-warp item sums          */
   InstDesc *I = P.inst;
   const int ns = P.nslots;
   const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
@@ -118,12 +414,15 @@ __global__ void __launch_bounds__(kBlock, TBFS_MULTI_PER_SM) multi_bfs_kernel(co
   for (int i = t; i < ns; i += kBlock) s_d[i] = __ldcg(&I[i].d);
   __syncthreads();
 
+  const bool use_local = gridDim.x >= kLocalGrid;
   unsigned ph = 0;
   for (; ph < (unsigned)P.max_phases; ++ph) {
     /* the host's "request waiting" flag (mapped host memory, a slow read):
      * issued now, used at the end of the level */
     int wake_now = 0;
     if (tid == 0 && P.wake) wake_now = *P.wake;
+    const long long t_begin = clock64();
+    if (t < kLocalMine) s_mine[t] = -1;
     /* ---- plan: identical in every CTA (reads counters finished before the
      * last barrier); block sums and scans by warp shuffles ---- */
     constexpr int kPer = (kMultiMaxSlots + kBlock - 1) / kBlock;
@@ -153,26 +452,31 @@ __global__ void __launch_bounds__(kBlock, TBFS_MULTI_PER_SM) multi_bfs_kernel(co
      * any bookkeeping of this one */
     if (stop_prev) break;
     unsigned qes[kPer];
+    bool loc[kPer];
     unsigned long long esum = 0;
     int act = 0, fin = 0;
 #pragma unroll
     for (int j = 0; j < kPer; ++j) {
       const int i = t * kPer + j;
       qes[j] = 0;
+      loc[j] = false;
       if (i < ns) {
         const int d = s_d[i];
         const bool done = dns[j];
         const unsigned long long qv = done ? 0ull : qvs[j];
         const unsigned qn = (unsigned)(qv >> 32), qe = (unsigned)qv;
-        s_qn[i] = qn;
+        loc[j] = use_local && qn && qn <= kLocalQueue && qe <= kLocalEnter;
+        s_qn[i] = loc[j] ? qn | kIsLocal : qn;
         s_qe[i] = qe;
         if (qn) {
-          act = 1;
-          qes[j] = qe;
-          esum += qe;
+          act |= loc[j] ? 1 : 2;
+          if (!loc[j]) {
+            qes[j] = qe;
+            esum += qe;
+          }
         }
-        /* bookkeeping of the instance, by CTA 0 */
-        if (blockIdx.x == 0 && !done) {
+        /* bookkeeping of a shared instance, by CTA 0 */
+        if (blockIdx.x == 0 && !done && !loc[j]) {
           if (qn) {
             I[i].ctr[(d + 2) % 3] = 0ull;
             I[i].levels = d + 1;
@@ -188,7 +492,7 @@ __global__ void __launch_bounds__(kBlock, TBFS_MULTI_PER_SM) multi_bfs_kernel(co
     if (fin && P.stop_on_done) ctl->stop[ph & 1u] = 1; /* CTA 0 only; read after the barrier */
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) esum += __shfl_xor_sync(FULL, esum, o);
-    const int wact = __any_sync(FULL, act);
+    const int wact = (__any_sync(FULL, act & 1) ? 1 : 0) | (__any_sync(FULL, act & 2) ? 2 : 0);
     if (lane == 0) {
       s_wsum[wid] = esum;
       s_wact[wid] = wact;
@@ -209,35 +513,41 @@ __global__ void __launch_bounds__(kBlock, TBFS_MULTI_PER_SM) multi_bfs_kernel(co
     const unsigned rounds = (unsigned)max(1ull, min((unsigned long long)kMaxRounds, per_warp));
     const unsigned iedges = kRoundEdges * rounds;
     unsigned items[kPer];
-    unsigned sum = 0;
+    unsigned long long sum = 0; /* (local instances << 32) | items */
 #pragma unroll
     for (int j = 0; j < kPer; ++j) {
       items[j] = (qes[j] + iedges - 1) / iedges;
-      sum += items[j];
+      sum += items[j] + (loc[j] ? 1ull << 32 : 0ull);
     }
     /* exclusive scan of the per-thread sums: within the warp by shuffles,
      * across the warps from their totals */
-    unsigned inc = sum;
+    unsigned long long inc = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const unsigned x = __shfl_up_sync(FULL, inc, o);
+      const unsigned long long x = __shfl_up_sync(FULL, inc, o);
       if (lane >= o) inc += x;
     }
     if (lane == 31) s_wscan[wid] = inc;
     __syncthreads();
-    unsigned wbase = 0, total = 0;
+    unsigned long long wbase = 0, wtot = 0;
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) {
-      const unsigned v = s_wscan[w];
+      const unsigned long long v = s_wscan[w];
       if (w < wid) wbase += v;
-      total += v;
+      wtot += v;
     }
-    unsigned run = wbase + inc - sum;
+    const unsigned total = (unsigned)wtot;
+    unsigned run = (unsigned)(wbase + inc - sum);
+    unsigned rank = (unsigned)((wbase + inc - sum) >> 32);
 #pragma unroll
     for (int j = 0; j < kPer; ++j) {
       const int i = t * kPer + j;
       if (i < ns) s_pre[i] = run;
       run += items[j];
+      if (loc[j]) { /* instance `rank` of the local ones, on CTA 1 and up */
+        if (rank % (gridDim.x - 1u) + 1u == blockIdx.x) s_mine[rank / (gridDim.x - 1u)] = i;
+        ++rank;
+      }
     }
     if (t == 0) s_pre[ns] = total;
     __syncthreads();
@@ -393,11 +703,33 @@ __global__ void __launch_bounds__(kBlock, TBFS_MULTI_PER_SM) multi_bfs_kernel(co
       if (lane == 0) nx = nwarps + atomicAdd(&ctl->work[ph & 3u], 1u);
       it = __shfl_sync(FULL, nx, 0);
     }
+    if (any_act & 1) { /* instances run by single CTAs */
+      const long long most = (any_act & 2) ? kLocalBeside : kLocalAlone;
+      const long long span = most < P.timeout_ns / 4 ? most : P.timeout_ns / 4;
+      const long long t_end = t_begin + span;
+      int mine = 0;
+      while (mine < kLocalMine && s_mine[mine] >= 0) ++mine;
+      for (int m = 0; m < mine; ++m) { /* equal parts of the time */
+        const int i = s_mine[m];
+        local_run(P, I[i], L, s_d[i], s_qn[i] & ~kIsLocal, s_qe[i], ph,
+                  t_begin + span * (m + 1) / mine);
+      }
+      /* CTA 0 has none: it watches for requests until all others arrived */
+      if (tid == 0 && P.wake) {
+        const unsigned others = gridDim.x - 1u;
+        while (!wake_now && clock64() < t_end &&
+               (dev::ld_acquire_u32(&ctl->bar.arrive) & 0x7fffffffu) != others)
+          wake_now = *P.wake;
+        if (wake_now) *(volatile int *)&ctl->stop[ph & 1u] = 1;
+      }
+    }
     /* a waiting request (host flag) ends the launch after this level */
     if (tid == 0 && wake_now) ctl->stop[ph & 1u] = 1;
     if (!grid_barrier(ctl, P.timeout_ns, (int)ph)) return;
-    for (int i = t; i < ns; i += kBlock)
-      if (s_qn[i]) s_d[i] += 1;
+    for (int i = t; i < ns; i += kBlock) {
+      if (s_qn[i] & kIsLocal) s_d[i] = __ldcg(&I[i].d);
+      else if (s_qn[i]) s_d[i] += 1;
+    }
     __syncthreads();
   }
   /* the level each instance runs next, for the following launch */
@@ -406,17 +738,35 @@ __global__ void __launch_bounds__(kBlock, TBFS_MULTI_PER_SM) multi_bfs_kernel(co
   if (tid == 0) ctl->phases = (int)ph;
 }
 
-/* new instances: depth 0 and count 1 at the root, queue {root} */
-__global__ void multi_init_kernel(InstDesc *I, const int *slots, int k) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= k) return;
-  InstDesc &D = I[slots[j]];
+/* new instances: depths -1 and counts 0, 0 and 1 at the root, queue {root}.
+ * One launch for all of them (blockIdx.y): two memsets per instance took 2.4 us
+ * of the host each, and more than a small traversal. */
+__global__ void __launch_bounds__(kInitBlock) multi_init_kernel(InstDesc *I, const int *slots) {
+  InstDesc &D = I[slots[blockIdx.y]];
   const int r = D.inv ? D.inv[D.root] : D.root;
-  D.S[r] = 0;
-  if (D.sig) D.sig[r] = 1ull;
-  D.q[0][0] = r;
-  D.e[0][0] = 0u;
-  D.ctr[0] = (1ull << 32) | (unsigned)(D.rp[r + 1] - D.rp[r]);
+  int *S = D.S;
+  unsigned long long *sig = D.sig;
+  const long long n = D.n, step = (long long)gridDim.x * kInitBlock * 4;
+  for (long long i = ((long long)blockIdx.x * kInitBlock + threadIdx.x) * 4; i < n; i += step) {
+    if (i + 4 <= n) { /* both arrays start on 256 bytes */
+      *reinterpret_cast<int4 *>(S + i) =
+          make_int4(i == r ? 0 : -1, i + 1 == r ? 0 : -1, i + 2 == r ? 0 : -1, i + 3 == r ? 0 : -1);
+      if (sig) {
+        *reinterpret_cast<ulonglong2 *>(sig + i) = make_ulonglong2(i == r, i + 1 == r);
+        *reinterpret_cast<ulonglong2 *>(sig + i + 2) = make_ulonglong2(i + 2 == r, i + 3 == r);
+      }
+    } else {
+      for (long long k = i; k < n; ++k) {
+        S[k] = k == r ? 0 : -1;
+        if (sig) sig[k] = k == r ? 1ull : 0ull;
+      }
+    }
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    D.q[0][0] = r;
+    D.e[0][0] = 0u;
+    D.ctr[0] = (1ull << 32) | (unsigned)(D.rp[r + 1] - D.rp[r]);
+  }
 }
 
 /* results in the caller's numbering: out[j] = S[inv[j]] */
@@ -429,6 +779,17 @@ __global__ void multi_gather_kernel(const int *S, const unsigned long long *sig,
   if (sig_out) sig_out[j] = sig[v];
 }
 
+/* results of all instances (blockIdx.y), each at its place in the packed outputs */
+__global__ void __launch_bounds__(kInitBlock) multi_pack_kernel(const InstDesc *I, int *S_out,
+                                                                unsigned long long *sig_out) {
+  const InstDesc &D = I[blockIdx.y];
+  const long long step = (long long)gridDim.x * kInitBlock;
+  for (long long i = (long long)blockIdx.x * kInitBlock + threadIdx.x; i < D.n; i += step) {
+    S_out[D.out + i] = D.S[i];
+    if (sig_out) sig_out[D.out + i] = D.sig[i];
+  }
+}
+
 }  // namespace
 
 cudaError_t multi_geometry(int device, LaunchGeom *out) {
@@ -438,11 +799,15 @@ cudaError_t multi_geometry(int device, LaunchGeom *out) {
   e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
   if (e != cudaSuccess) return e;
   if (!coop) return cudaErrorNotSupported;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, multi_bfs_kernel, kBlock, 0);
+  e = cudaFuncSetAttribute(multi_bfs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)sizeof(LocalShared));
+  if (e != cudaSuccess) return e;
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, multi_bfs_kernel, kBlock,
+                                                    sizeof(LocalShared));
   if (e != cudaSuccess) return e;
   if (per < 1) return cudaErrorInvalidConfiguration;
-  /* a few CTAs per SM: enough warps to cover the latency of the pushes,
-   * fewer barrier arrivals than a fully occupied grid */
+  /* one large CTA per SM: all of an SM for an instance that a CTA runs alone,
+   * few barrier arrivals for the others */
   if (per > TBFS_MULTI_PER_SM) per = TBFS_MULTI_PER_SM;
   out->block = kBlock;
   out->grid = sms * per;
@@ -452,12 +817,29 @@ cudaError_t multi_geometry(int device, LaunchGeom *out) {
 cudaError_t multi_launch(const MultiParams &p, const LaunchGeom &g, cudaStream_t s) {
   void *args[] = {const_cast<MultiParams *>(&p)};
   return cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(multi_bfs_kernel), dim3(g.grid),
-                                     dim3(g.block), args, 0, s);
+                                     dim3(g.block), args, sizeof(LocalShared), s);
 }
 
-cudaError_t multi_init(InstDesc *inst, const int *slots, int k, cudaStream_t s) {
+/* blocks (x) for the k instances of a launch, the largest of n vertices, each
+ * thread with `per` of them: as many as the largest asks for while all
+ * together are at most ~16 per SM */
+static unsigned inst_blocks(int n, int k, int per) {
+  const long long want = ((long long)n + (long long)kInitBlock * per - 1) / ((long long)kInitBlock * per);
+  const long long most = 2432 / k + 1;
+  return (unsigned)std::max(1ll, std::min(want, most));
+}
+
+cudaError_t multi_init(InstDesc *inst, const int *slots, int k, int n_most, cudaStream_t s) {
   if (k <= 0) return cudaSuccess;
-  multi_init_kernel<<<(k + 127) / 128, 128, 0, s>>>(inst, slots, k);
+  multi_init_kernel<<<dim3(inst_blocks(n_most, k, 4), (unsigned)k), kInitBlock, 0, s>>>(inst, slots);
+  return cudaGetLastError();
+}
+
+cudaError_t multi_pack(const InstDesc *inst, int k, int n_most, int *S_out,
+                       unsigned long long *sig_out, cudaStream_t s) {
+  if (k <= 0) return cudaSuccess;
+  multi_pack_kernel<<<dim3(inst_blocks(n_most, k, 1), (unsigned)k), kInitBlock, 0, s>>>(inst, S_out,
+                                                                                     sig_out);
   return cudaGetLastError();
 }
 

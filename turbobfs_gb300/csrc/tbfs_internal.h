@@ -265,7 +265,8 @@ void batch_ws_free(BatchWS *ws);
 
 /* ---- multi-instance engine (multi_engine.cu) ----
  * One descriptor per traversal (graph, root); the kernel advances every
- * unfinished descriptor by one level per phase. */
+ * unfinished descriptor by one level per phase, by as many as the phase has
+ * time for if one CTA can run it alone. */
 constexpr int kMultiMaxSlots = 1024;
 
 struct InstDesc {
@@ -287,13 +288,14 @@ struct InstDesc {
   int deg_bits;               /* bits of the largest in-degree (0: unknown):
                                  counts of level d have at most 1 + d deg_bits */
   long long visited, edges;
+  long long out;              /* first element in packed outputs (multi_pack) */
 };
 
 struct __align__(128) MultiCtl {
   unsigned work[4];
   int status, timeout_level;
-  int phases;                 /* levels run by the launch */
-  int stop[2];                /* end the launch after level ph: stop[ph % 2], written
+  int phases;                 /* phases run by the launch */
+  int stop[2];                /* end the launch after phase ph: stop[ph % 2], written
                                  during the level, read after its barrier; two slots
                                  so that a CTA already in level ph+1 cannot write
                                  the word a slower CTA is still to read for ph */
@@ -304,7 +306,7 @@ struct __align__(128) MultiCtl {
 struct MultiParams {
   InstDesc *inst;
   int nslots;                 /* descriptors (<= kMultiMaxSlots) */
-  int max_phases;             /* stop after this many levels     */
+  int max_phases;             /* stop after this many phases     */
   MultiCtl *ctl;
   long long timeout_ns;
   const volatile int *wake;   /* host-mapped flag: requests wait (null: none) */
@@ -313,8 +315,12 @@ struct MultiParams {
 
 cudaError_t multi_geometry(int device, LaunchGeom *out);
 cudaError_t multi_launch(const MultiParams &p, const LaunchGeom &g, cudaStream_t s);
-/* initialise the descriptors slots[0..k) (S = -1 and sig = 0 already set) */
-cudaError_t multi_init(InstDesc *inst, const int *slots, int k, cudaStream_t s);
+/* initialise the descriptors slots[0..k), of graphs of at most n_most vertices */
+cudaError_t multi_init(InstDesc *inst, const int *slots, int k, int n_most, cudaStream_t s);
+/* S_out[inst.out + j] = inst.S[j] for the first k descriptors; sig likewise when
+ * sig_out is set */
+cudaError_t multi_pack(const InstDesc *inst, int k, int n_most, int *S_out,
+                       unsigned long long *sig_out, cudaStream_t s);
 /* out[j] = S[inv[j]] (or S[j]) for j < n; sig likewise when sig_out is set */
 cudaError_t multi_gather(const int *S, const unsigned long long *sig, const int *inv, int n,
                          int *S_out, unsigned long long *sig_out, cudaStream_t s);
