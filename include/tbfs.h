@@ -82,8 +82,8 @@ typedef struct tbfs_options {
   /* Engine shape of the single-source traversal (tbfs_autotune sets both):
    * the most list entries a lane handles per round of a push or pull (1..6;
    * 0 = 6), and units of 256 threads per SM of the persistent launch (1..4;
-   * 0 = 3, 4 on large graphs regrouped by degree, 2 on graphs whose out-lists
-   * all have at most 16 entries). */
+   * 0 = 3, 4 on large graphs regrouped by degree; 2, at most, on graphs without
+   * long out-lists: 16 entries, 64 on smaller graphs). */
   int32_t max_ept;
   int32_t ctas_per_sm;
 } tbfs_options;

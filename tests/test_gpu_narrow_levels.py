@@ -1,6 +1,6 @@
 """Narrow levels (vertices kept in shared memory) against the exact oracle.
 
-Graphs whose out-lists hold at most 16 entries, at the sizes where the narrow
+Graphs whose out-lists hold at most 64 entries, at the sizes where the narrow
 levels can go wrong: chains (one vertex a level), even shares every 32 levels,
 a CTA with more than 64 and more than 256 finds in a level, levels that grow
 beyond what is narrow and shrink again, directed lists, counts past 2^63.
@@ -68,7 +68,22 @@ def _diamonds(k):
     return 3 * k + 1, np.array(a), np.array(b), 0
 
 
+def _random(n, degree, seed):
+    """n * degree random edges, of which every vertex keeps at most 64."""
+    rng = np.random.default_rng(seed)
+    a, b = rng.integers(0, n, n * degree), rng.integers(0, n, n * degree)
+    order = np.argsort(a, kind="stable")
+    a, b = a[order], b[order]
+    rank = np.arange(len(a)) - np.searchsorted(a, a)
+    return n, a[rank < 64], b[rank < 64], 0
+
+
 GRAPHS = {
+    "random_1000_of_7": lambda: _random(1000, 7, 1),
+    "random_3000_of_60": lambda: _random(3000, 60, 2),
+    "random_30000_of_9": lambda: _random(30000, 9, 3),
+    "tree_64_fan": lambda: _tree(64, 2, 40),
+    "tree_65_fan": lambda: _tree(65, 2, 40),
     "chain_700": lambda: _chain(700),
     "strip_3x400": lambda: _grid(3, 400),
     "grid_150x140": lambda: _grid(150, 140),

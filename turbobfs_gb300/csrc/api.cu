@@ -184,7 +184,9 @@ static tbfs_status graph_finish(tbfs_graph *g) {
       cudaError_t e = tbfs::longest_list(g->rp, g->n, &max_out);
       if (e != cudaSuccess) return cuda_fail(e, "out-degree bound", __LINE__);
     }
-    g->short_lists = max_out <= tbfs::kShortList;
+    g->max_out = max_out;
+    g->short_lists = max_out <= tbfs::kShortList ||
+                     (max_out <= tbfs::kNarrowList && g->nnz <= tbfs::kNarrowEntries);
     CUDA_TRY(tbfs::dev_alloc(&g->tile, ((size_t)tbfs::tile_count(g->n, g->nnz) + 1) * sizeof(int)));
     CUDA_TRY(tbfs::fill_tiles(g->cp, g->n, g->nnz, g->tile, 0));
     if (maxd > tbfs::kHubLen) {
@@ -699,6 +701,7 @@ static BfsParams make_params(tbfs_graph *g, int32_t root, const tbfs_options &o,
   p.ctas_per_sm = o.ctas_per_sm;
   p.deg_bits = g->deg_bits;
   p.short_lists = g->short_lists ? 1 : 0;
+  p.max_list = g->max_out;
   return p;
 }
 

@@ -44,7 +44,7 @@
  * flattened edges, stages 128 queue entries at a time in shared memory, and
  * every lane handles kEPT consecutive edges per round, so that many list
  * reads, then that many depth gathers, are in flight per lane.  On graphs
- * whose out-lists are all short (kShortList entries at most) the kernel
+ * without long out-lists (kShortList, kNarrowList) the kernel
  * instances bfs_persistent_kernel<true, .> cut small top-down levels into
  * items of kShortEntries whole queue entries instead, which need no owner
  * search (the chain of dependent L2 round trips is what a small level
@@ -70,6 +70,8 @@
  */
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <algorithm>
 
 #include "device_common.cuh"
 #include "tbfs_internal.h"
@@ -97,8 +99,8 @@ constexpr int kBlockStep = 256;    /* threads per unit of ctas_per_sm */
 constexpr int kFilterBits = 1 << 18; /* frontier filter in shared memory (32 KB) */
 constexpr int kWin = 128;          /* queue entries staged per warp window */
 constexpr int kEPT = TBFS_EPT;     /* most consecutive edges per lane/round */
-/* queue entries per item of a small level of a short-list graph: at most
- * 8 * kShortList = 128 edges, one round of at most 4 per lane */
+/* queue entries per item of a small level of a short-list graph: 128 edges, one
+ * round of at most 4 per lane, if the lists have kShortList entries */
 constexpr unsigned kShortEntries = 8;
 constexpr float kBuWordCost = 4.0f; /* a bitmap word of a bottom-up level, in list entries */
 enum { DIR_TD = 0, DIR_BU = 1 };
@@ -886,12 +888,15 @@ __device__ __forceinline__ void bu_tile(const BfsParams &p, int d, const NextQue
  * targets' lists are, are read while the barrier is waited for; and what all
  * CTAs have to know, the size of the level, comes back with the barrier.
  * Left between two barriers: one claim.
- *   Frontiers drift into few CTAs (the faster one claims first), so every
- * kShareEvery levels, and when a CTA has more than kRound, all finds of a
- * level go to the global queue, which the next one shares out evenly.  (With
- * only the finds beyond kRound sent there, such a vertex was expanded three
- * round trips after the kept ones and lost its targets to them: who had much
- * got more, and 84 % of a grid's levels used the queue.)
+ *   A CTA whose vertices have more than its share of the level's edges
+ * (keep_limit) sends its finds to the global queue, which the next level
+ * shares out evenly, so that a frontier that starts in one CTA spreads.  One
+ * that does not grow drifts into few CTAs: the faster one claims first.  So
+ * every kShareEvery levels, and when a CTA has found more than kRound, all
+ * finds of the next level go to the global queue.  (With only the finds beyond
+ * kRound sent there: such a vertex is expanded three round trips after the
+ * kept ones and loses its targets to them; who had much got more, and 84 % of
+ * a grid's levels used the queue.)
  *   Grid of 2048 x 2048 with path counts, us per level: 6.5 with every level
  * through the global queue, 3.1 so (depths only: 2.5).  What is left is the
  * claim, the fence and the barrier's two trips, ~700 clocks each, and DRAM
@@ -899,22 +904,24 @@ __device__ __forceinline__ void bu_tile(const BfsParams &p, int d, const NextQue
  * threads 4.0; sharing every 12 or 96 levels instead of 32: +2 %, +0 %. */
 constexpr unsigned kKeep = 256, kRound = 64;
 constexpr int kShareEvery = 32;
-/* mean vertices per CTA up to which a level is narrow, and starts to be */
-constexpr unsigned kNarrow = 64, kNarrowEnter = 32;
+/* out-edges of a CTA's kept vertices up to which it keeps what it finds, in a
+ * level of qe (Erdos-Renyi, 4096 vertices: one CTA ran 336 vertices, found by
+ * eight of its own, in 15 us) */
+__device__ __forceinline__ unsigned keep_limit(unsigned qe) { return 64u + 4u * qe / gridDim.x; }
+/* mean vertices per CTA up to which a level is narrow, its most out-edges;
+ * half of both to start.  Up to there a push of all edges costs less than a
+ * bottom-up level's ~6 us, so the direction rule is not asked. */
+constexpr unsigned kNarrow = 64, kNarrowEdges = 1u << 16;
 /* A barrier's 64-bit sum: arrivals, the level's vertices, their out-edges,
- * CTAs with more than kRound of them. */
-constexpr int kSumCount = 9, kSumEdges = 29, kSumSpill = 55;
-constexpr unsigned kSumGrid = 240; /* CTAs up to which no field can overflow: */
-static_assert((unsigned long long)kNarrow * kSumGrid * kShortList < 1ull << (kSumEdges - kSumCount),
-              "vertices found by a narrow level");
-static_assert((unsigned long long)kNarrow * kSumGrid * kShortList * kShortList <
-                  1ull << (kSumSpill - kSumEdges),
-              "their out-edges");
-static_assert(kSumGrid < 1u << (kSumCount - 1), "arrivals");
+ * CTAs that used the global queue, CTAs that kept more than kRound (modulo 32:
+ * missed, it costs time only).  narrow_limit keeps the others apart. */
+constexpr int kSumCount = 9, kSumEdges = 27, kSumSpill = 51, kSumCrowd = 59;
+constexpr unsigned kSumGrid = 240;
+static_assert(kSumGrid < 1u << (kSumCount - 1) && kSumGrid < 1u << (kSumCrowd - kSumSpill), "CTAs");
 
 struct NarrowState {
   int v[2][kKeep], a[2][kKeep], deg[2][kKeep]; /* kept vertices of level d in [d & 1] */
-  unsigned found[3], edges[3];   /* found for level d in [d % 3], their out-edges */
+  unsigned found[3], edges[3]; /* by this CTA for level d in [d % 3]; out-edges  */
   unsigned long long last[2];    /* the barrier words after their last use        */
   unsigned long long sum;
   int ok;
@@ -993,7 +1000,7 @@ enum NarrowEnd { NARROW_DONE, NARROW_LEAVE, NARROW_TIMEOUT, NARROW_INJECTED };
 template <bool SIG>
 __device__ __forceinline__ NarrowEnd narrow_levels(const BfsParams &p, NarrowState &ns,
                                                    LevelState &l, unsigned qn, unsigned qe,
-                                                   float alpha, bool &ovf) {
+                                                   bool &ovf) {
   BfsCtl *ctl = p.ctl;
   const unsigned tid = threadIdx.x, lane = tid & 31u, wid = tid >> 5, nw = blockDim.x >> 5;
   const unsigned gtid = blockIdx.x * blockDim.x + tid, nthreads = gridDim.x * blockDim.x;
@@ -1033,7 +1040,7 @@ __device__ __forceinline__ NarrowEnd narrow_levels(const BfsParams &p, NarrowSta
     const unsigned long long gq = global ? __ldcg(&ctl->qctr[c0]) : 0ull;
     const bool chk = SIG && !ovf_seen && !(p.deg_bits > 0 && l.sig_bits + p.deg_bits <= 63);
     const bool share = crowded || ++kept_levels > kShareEvery;
-    const unsigned cap = share ? 0u : kKeep;
+    const unsigned cap = share || (mine && ns.edges[c0] > keep_limit(qe)) ? 0u : kKeep;
     if (share) kept_levels = 0;
     const NextQueue nx = {p.q[b ^ 1], p.e[b ^ 1], p.a[b ^ 1], &ctl->qctr[c1]};
     const unsigned long long *src = b ? p.sigma_odd : p.sigma;
@@ -1087,18 +1094,19 @@ __device__ __forceinline__ NarrowEnd narrow_levels(const BfsParams &p, NarrowSta
     __syncthreads();
     constexpr unsigned kFlip = 1u << (kSumCount - 1);
     const unsigned found = ns.found[c1];
+    mine = found < cap ? found : cap;
     if (tid == 0) {
       const unsigned long long add =
           (blockIdx.x == 0 ? kFlip - (gridDim.x - 1u) : 1u) +
           ((unsigned long long)found << kSumCount) +
           ((unsigned long long)ns.edges[c1] << kSumEdges) +
-          (!share && found > kRound ? 1ull << kSumSpill : 0ull);
+          (found > cap ? 1ull << kSumSpill : 0ull) +
+          (cap && found > kRound ? 1ull << kSumCrowd : 0ull);
       asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(&ctl->sum[b].word), "l"(add)
                    : "memory");
     }
     /* meanwhile: the lists of the kept vertices, and the depths of their
      * targets, some of which may be level d + 2's already */
-    mine = found < cap ? found : cap;
     sub = narrow_sub(mine, nw - 1u);
     {
       const unsigned k = (kwid << (5 - sub)) + (lane >> sub);
@@ -1151,14 +1159,12 @@ __device__ __forceinline__ NarrowEnd narrow_levels(const BfsParams &p, NarrowSta
     const unsigned long long sum = ns.sum;
     qn = (unsigned)(sum >> kSumCount) & ((1u << (kSumEdges - kSumCount)) - 1u);
     qe = (unsigned)(sum >> kSumEdges) & ((1u << (kSumSpill - kSumEdges)) - 1u);
-    crowded = (sum >> kSumSpill) != 0ull;
-    global = share || crowded; /* more than kRound may be more than kKeep */
+    global = ((sum >> kSumSpill) & ((1u << (kSumCrowd - kSumSpill)) - 1u)) != 0ull;
+    crowded = (sum >> kSumCrowd) != 0ull;
     l.sig_bits = l.sig_bits + p.deg_bits < 64 ? l.sig_bits + p.deg_bits : 64;
     ++l.d;
     if (qn == 0u) return NARROW_DONE;
-    if (qn > kNarrow * gridDim.x ||
-        (p.mode != TBFS_MODE_TOP_DOWN &&
-         (float)qe * alpha > (float)(l.m_u - qe) + kBuWordCost * (float)nwords)) {
+    if (qn > p.narrow || qe > kNarrowEdges) {
       if (wid < (mine + 31u) / 32u) { /* level d + 1 to the global queue */
         const unsigned k = tid;
         const int vv[1] = {k < mine ? ns.v[b ^ 1][k] : 0};
@@ -1193,11 +1199,11 @@ __global__ void __launch_bounds__(SHORT ? kShortBlock : kBlock, 1)
   const unsigned nwarps = nthreads >> 5;
   BfsCtl *ctl = p.ctl;
   constexpr bool want_sigma = SIG;
-  NarrowState *ns = nullptr;
+  NarrowState *narrow = nullptr;
   if constexpr (SHORT) {
     __shared__ NarrowState s_narrow;
-    ns = &s_narrow;
-    if (threadIdx.x == 0) ns->last[0] = ns->last[1] = 0ull;
+    narrow = &s_narrow;
+    if (threadIdx.x == 0) narrow->last[0] = narrow->last[1] = 0ull;
   }
   const int root = p.inv ? __ldg(p.inv + p.root) : p.root; /* internal numbering */
 
@@ -1269,12 +1275,10 @@ __global__ void __launch_bounds__(SHORT ? kShortBlock : kBlock, 1)
       break;
     }
     if constexpr (SHORT) {
-      if (dir == DIR_TD && p.mode != TBFS_MODE_BOTTOM_UP && qn <= kNarrowEnter * gridDim.x &&
-          gridDim.x <= kSumGrid &&
-          (p.mode == TBFS_MODE_TOP_DOWN ||
-           !((float)qe * alpha > (float)(m_u - qe) + kBuWordCost * (float)nwords))) {
+      if (dir == DIR_TD && p.mode != TBFS_MODE_BOTTOM_UP && qn <= p.narrow / 2u &&
+          qe <= kNarrowEdges / 2u) {
         LevelState l = {d, td, sig_bits, m_u, visited, edges};
-        const NarrowEnd end = narrow_levels<SIG>(p, *ns, l, qn, qe, alpha, ovf);
+        const NarrowEnd end = narrow_levels<SIG>(p, *narrow, l, qn, qe, ovf);
         if (end == NARROW_INJECTED) return;
         d = l.d;
         td = l.td;
@@ -1569,6 +1573,18 @@ cudaError_t bfs_geometry(int device, LaunchGeom *out) {
   return cudaSuccess;
 }
 
+/* Most vertices of a narrow level, 0: none.  Of lists of at most m entries, so
+ * many vertices find less than 2^18, with less than 2^24 out-edges, and the
+ * fields of a barrier's sum stay apart (also if all vertices are found). */
+static unsigned narrow_limit(const BfsParams &p, int grid) {
+  const long long m = p.max_list;
+  if (m <= 0 || m > kNarrowList || grid > (int)kSumGrid) return 0;
+  const long long found = (1 << (kSumEdges - kSumCount)) - 1, edges = (1 << (kSumSpill - kSumEdges)) - 1;
+  long long most = (long long)kNarrow * grid;
+  if (p.n > found || p.n * m > edges) most = std::min({most, found / m, edges / (m * m)});
+  return (unsigned)most;
+}
+
 cudaError_t bfs_launch(const BfsParams &p0, const LaunchGeom &g, cudaStream_t s) {
   /* One CTA per SM, of 256 threads per unit of ctas_per_sm.  By default (and at
    * most) 2 on short-list graphs, whose levels are many and small; 4 for depths only and
@@ -1583,6 +1599,7 @@ cudaError_t bfs_launch(const BfsParams &p0, const LaunchGeom &g, cudaStream_t s)
   const int want = p.ctas_per_sm > 0 ? p.ctas_per_sm : short_lists ? 2 : full ? 4 : 3;
   int block = want < g.per_sm ? kBlockStep * want : g.block;
   if (short_lists && block > kShortBlock) block = kShortBlock;
+  p.narrow = short_lists ? narrow_limit(p, g.grid) : 0u;
   p.filter = !short_lists && sigma && p.tile && (double)p.nnz > kHeavyEntries;
   void *args[] = {&p};
   return cudaLaunchCooperativeKernel(bfs_kernel(short_lists, sigma), dim3(g.grid), dim3(block), args,

@@ -113,12 +113,24 @@ struct BfsParams {
   /* bits of the largest in-degree (0: unknown); bounds the path counts'
    * growth per level (bfs_engine.cu) */
   int deg_bits;
-  /* nonzero: no out-list has more than kShortList entries, so small
-   * top-down levels may give every queue entry to one lane (bfs_engine.cu) */
+  /* nonzero: the short-list instance (bfs_engine.cu) */
   int short_lists;
+  /* longest out-list (0: unknown); most vertices of a narrow level, set by the
+   * launch */
+  int max_list;
+  unsigned narrow;
 };
 
-/* longest out-list for which a lane walks a whole list alone */
+/* Longest out-list of graphs whose narrow levels stay in shared memory.  Such
+ * graphs run the short-list instance, those with lists past kShortList only up
+ * to kNarrowEntries entries: there the narrow levels gain more than its smaller
+ * CTAs lose in the wide ones (Erdos-Renyi, ms other / short-list instance:
+ * 4096 vertices of degree 8 0.058 / 0.034, 100 K of 16 0.075 / 0.060, 600 K of
+ * 8 0.133 / 0.111; 2.5 M of 14 0.34 / 0.37, depths of 1 M of 16 0.104 / 0.108). */
+constexpr int kNarrowList = 64;
+constexpr int kNarrowEntries = 6 << 20;
+
+/* longest out-list of short-list graphs of any size */
 constexpr int kShortList = 16;
 /* work of a bottom-up level is cut by in-list entries plus this per vertex */
 constexpr int kTileCost = 512;
@@ -405,7 +417,8 @@ struct tbfs_graph {
   int *tile = nullptr;   /* BfsParams::tile */
   int *hubs = nullptr;   /* segment count, then the hub segments (BfsParams::hub_seg) */
   int deg_bits = 0;      /* bits of the largest in-degree */
-  bool short_lists = false; /* no out-list longer than kShortList */
+  bool short_lists = false; /* no long out-list: kShortList, kNarrowList */
+  int max_out = 0;          /* longest out-list */
   /* the caller's TBFS_GRAPH_SYMMETRIC (flags may also carry it when the
    * lists were found to equal their transpose on upload) */
   bool declared_symmetric = false;
