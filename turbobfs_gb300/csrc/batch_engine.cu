@@ -64,13 +64,13 @@ using dev::grid_barrier;
 
 constexpr int kBlock = 256;
 constexpr int kWarps = kBlock / 32;
-constexpr int kPushRounds = 8;    /* 32-edge rounds per push work item         */
+constexpr int kPushRounds = 8;    /* most 32-edge rounds per push work item    */
 constexpr int kClear = 256;       /* queue entries per row-clearing item        */
 constexpr int kVCost = 4;         /* a vertex costs like this many list entries */
 #ifndef TBFS_BATCH_ITEM
 #define TBFS_BATCH_ITEM 512
 #endif
-constexpr long long kItemCost = TBFS_BATCH_ITEM; /* list entries + vertex costs per item */
+constexpr long long kItemCost = TBFS_BATCH_ITEM; /* most list entries + vertex costs per item */
 #ifndef TBFS_BATCH_HITS
 #define TBFS_BATCH_HITS 3
 #endif
@@ -711,26 +711,33 @@ __device__ __forceinline__ unsigned nsegs(int deg, int seg_len) {
   return (unsigned)((deg + seg_len - 1) / seg_len);
 }
 
-/* Smallest i in [0, cnt] with f(i) >= target, f nondecreasing on [0, cnt)
- * and f(cnt) taken as +infinity; 32-ary search, all 32 lanes call with the
- * same arguments. */
+/* a, b = the smallest i in [0, cnt] with f(i) >= t0 and >= t1, f nondecreasing
+ * on [0, cnt) and f(cnt) taken as +infinity; a 16-ary search by each half of
+ * the warp, all 32 lanes call with the same arguments. */
 template <class F>
-__device__ __forceinline__ unsigned warp_lower_bound(F f, unsigned cnt, long long target) {
-  const int lane = threadIdx.x & 31;
+__device__ __forceinline__ void warp_two_bounds(F f, unsigned cnt, long long t0, long long t1,
+                                                unsigned &a, unsigned &b) {
+  const int lane = threadIdx.x & 31, l = lane & 15, sh = lane & 16;
+  const long long target = sh ? t1 : t0;
   unsigned lo = 0, hi = cnt;
-  while (hi - lo > 32) {
-    const unsigned step = (hi - lo + 31) / 32;
-    const unsigned pidx = lo + lane * step;
+  while (__any_sync(FULL, hi - lo > 16)) {
+    const unsigned step = (hi - lo + 15) / 16;
+    const unsigned pidx = lo + l * step;
     const bool pred = pidx < hi && f(pidx) < target;
-    const unsigned c = __popc(__ballot_sync(FULL, pred));
-    if (c == 0) return lo;
-    const unsigned nhi = lo + c * step;
-    lo = lo + (c - 1) * step + 1;
-    hi = nhi < hi ? nhi : hi;
+    const unsigned c = __popc((__ballot_sync(FULL, pred) >> sh) & 0xffffu);
+    if (c == 0) {
+      hi = lo;
+    } else {
+      const unsigned nhi = lo + c * step;
+      lo = lo + (c - 1) * step + 1;
+      hi = nhi < hi ? nhi : hi;
+    }
   }
-  const unsigned pidx = lo + lane;
+  const unsigned pidx = lo + l;
   const bool pred = pidx < hi && f(pidx) < target;
-  return lo + __popc(__ballot_sync(FULL, pred));
+  const unsigned r = lo + __popc((__ballot_sync(FULL, pred) >> sh) & 0xffffu);
+  a = __shfl_sync(FULL, r, 0);
+  b = __shfl_sync(FULL, r, 16);
 }
 
 /* largest i < cnt with pre[i] <= t (pre nondecreasing, pre[0] = 0) */
@@ -844,7 +851,7 @@ __global__ void __launch_bounds__(kBlock, TBFS_BATCH_MINB) fm_bfs_kernel(const B
   /* work items of a phase: the first one statically (global warp index),
    * later ones from the phase's counter (after the static range) */
   const unsigned nwarps = gridDim.x * kWarps;
-  const unsigned gwarp = blockIdx.x * kWarps + wid;
+  const unsigned gwarp = wid * gridDim.x + blockIdx.x; /* a small level on all SMs */
   bool first_claim = true;
   auto claim = [&](unsigned total) -> unsigned {
     if (first_claim) {
@@ -855,6 +862,16 @@ __global__ void __launch_bounds__(kBlock, TBFS_BATCH_MINB) fm_bfs_kernel(const B
     unsigned it = 0;
     if (g.lane == 0) it = nwarps + atomicAdd(&ctl->work[ph & 3u], 1u);
     return __shfl_sync(FULL, it, 0);
+  };
+  /* Cost of an item when `cnt` vertices cost `cost` together: about two items
+   * per warp, at least one vertex per group, at most kItemCost.  A small level's
+   * time is the chain of loads of an item's vertices one after the other.  (Items
+   * of kItemCost and 256 edges throughout against this, per level or call: grid
+   * of 200 x 200, 64 roots, 90 / 17 us; Erdos-Renyi of 30 K vertices, 200 roots,
+   * 1.00 / 0.40 ms; RMAT of 200 K, 40 roots, 0.38 / 0.31 ms.) */
+  auto item_cost = [&](long long cost, unsigned cnt) -> unsigned {
+    const float c = (float)cost, v = (float)max(cnt, 1u);
+    return (unsigned)fminf(fmaxf(c / (2.0f * (float)nwarps), c / v * PER) + 1.0f, (float)kItemCost);
   };
   /* entries finished during level d go to slot (d + 1) % 4, read at the
    * start of level d + 1 */
@@ -920,7 +937,9 @@ __global__ void __launch_bounds__(kBlock, TBFS_BATCH_MINB) fm_bfs_kernel(const B
 
     if (push) {
       /* ---- phase 1: discovery over the out-edges of Q_d ---- */
-      const unsigned nA = (qe + kPushRounds * 32 - 1) / (kPushRounds * 32);
+      /* rounds of an item: few on small levels, which have items for few warps */
+      const unsigned rounds = min((qe + 32u * nwarps - 1u) / (32u * nwarps), (unsigned)kPushRounds);
+      const unsigned nA = qe ? (qe + rounds * 32 - 1) / (rounds * 32) : 0u;
       if (tid == 0) ctl->work[(ph + 2) & 3u] = 0u;
       first_claim = true;
       for (;;) {
@@ -930,15 +949,35 @@ __global__ void __launch_bounds__(kBlock, TBFS_BATCH_MINB) fm_bfs_kernel(const B
           clear_item(it - nA);
           continue;
         }
-        for (int r = 0; r < kPushRounds; ++r) {
-          const unsigned t = it * (kPushRounds * 32) + r * 32 + g.lane;
+        const unsigned *e0 = p.e[b0];
+        unsigned o0 = dev::warp_find_owner(reinterpret_cast<const int *>(e0), qn, it * rounds * 32);
+        for (unsigned r = 0; r < rounds; ++r) {
+          const unsigned tb = it * (rounds * 32) + r * 32, t = tb + g.lane;
+          if (tb >= qe) break;
           bool first = false;
           int v = 0;
           unsigned dgo = 0;
+          /* the owner among the 32 entries from the last one's; past them (many
+           * empty lists) by a search of its own */
+          const bool in = o0 + g.lane < qn;
+          const unsigned ew = in ? __ldcg(e0 + o0 + g.lane) : 0xffffffffu;
+          const int qw = in ? __ldcg(p.q[b0] + o0 + g.lane) : 0;
+          const int aw = in ? __ldg(p.rp + qw) : 0;
+          unsigned j = 0;
+#pragma unroll
+          for (int h = 16; h > 0; h >>= 1)
+            if (__shfl_sync(FULL, ew, (int)(j + h)) <= t) j += h;
+          unsigned eo = __shfl_sync(FULL, ew, (int)j);
+          int u = __shfl_sync(FULL, qw, (int)j), a = __shfl_sync(FULL, aw, (int)j);
+          unsigned o = o0 + j;
           if (t < qe) {
-            const unsigned o = upper_owner(p.e[b0], qn, t);
-            const int u = __ldcg(p.q[b0] + o);
-            v = __ldg(p.jr + __ldg(p.rp + u) + (int)(t - __ldcg(p.e[b0] + o)));
+            if (j == 31u && o + 1 < qn && __ldcg(e0 + o + 1) <= t) {
+              o = upper_owner(e0, qn, t);
+              eo = __ldcg(e0 + o);
+              u = __ldcg(p.q[b0] + o);
+              a = __ldg(p.rp + u);
+            }
+            v = __ldg(p.jr + a + (int)(t - eo));
             unsigned fr[W], sv[W];
             load_row<W>(Fd + (size_t)u * W, fr);
             load_row<W>(p.seen + (size_t)v * W, sv);
@@ -969,6 +1008,7 @@ __global__ void __launch_bounds__(kBlock, TBFS_BATCH_MINB) fm_bfs_kernel(const B
               }
             }
           }
+          o0 = __shfl_sync(FULL, o, 31);
           warp_enqueue(first, v, dgo, p.q[b1], p.e[b1], qctr1);
         }
       }
@@ -981,9 +1021,10 @@ __global__ void __launch_bounds__(kBlock, TBFS_BATCH_MINB) fm_bfs_kernel(const B
       const unsigned hn1 = (unsigned)(hv >> 32), hsegs = (unsigned)hv;
       const unsigned qe1 = (unsigned)__ldcg(qctr1);
       const unsigned *e1 = p.e[b1];
-      /* items of ~kItemCost list entries + vertex costs over the queue */
+      /* items of equal list entries + vertex costs over the queue */
       const long long cost2 = (long long)qe1 + (long long)kVCost * qn1;
-      const unsigned nA2 = (unsigned)((cost2 + kItemCost - 1) / kItemCost);
+      const unsigned icost2 = item_cost(cost2, qn1);
+      const unsigned nA2 = (unsigned)((cost2 + icost2 - 1) / icost2);
       const unsigned nB2 = (hsegs + PER - 1) / PER;
       auto qcost = [&](unsigned i) -> long long {
         return (long long)__ldcg(e1 + i) + (long long)kVCost * i;
@@ -994,8 +1035,8 @@ __global__ void __launch_bounds__(kBlock, TBFS_BATCH_MINB) fm_bfs_kernel(const B
         const unsigned it = claim(nA2 + nB2);
         if (it >= nA2 + nB2) break;
         if (it < nA2) {
-          const unsigned is = warp_lower_bound(qcost, qn1, (long long)it * kItemCost);
-          const unsigned ie = warp_lower_bound(qcost, qn1, (long long)(it + 1) * kItemCost);
+          unsigned is, ie;
+          warp_two_bounds(qcost, qn1, (long long)it * icost2, (long long)(it + 1) * icost2, is, ie);
           for (unsigned base = is; base < ie; base += PER) {
             const unsigned idx = base + g.gid;
             bool full = false;
@@ -1032,7 +1073,8 @@ __global__ void __launch_bounds__(kBlock, TBFS_BATCH_MINB) fm_bfs_kernel(const B
       /* ---- pull: every vertex not reached by all roots ---- */
       const unsigned nA = ((unsigned)p.hub_segs + PER - 1) / PER;
       const long long cost = p.nnz_in + (long long)kVCost * n;
-      const unsigned nB = (unsigned)((cost + kItemCost - 1) / kItemCost);
+      const unsigned icost = item_cost(cost, (unsigned)n);
+      const unsigned nB = (unsigned)((cost + icost - 1) / icost);
       auto vcost = [&](unsigned v) -> long long {
         return (long long)__ldg(p.cp + v) + (long long)kVCost * v;
       };
@@ -1046,12 +1088,12 @@ __global__ void __launch_bounds__(kBlock, TBFS_BATCH_MINB) fm_bfs_kernel(const B
           continue;
         }
         unsigned bcnt = 0;
-        /* hub item: one segment per group; vertex item: the vertices of
-         * ~kItemCost list entries + vertex costs, PER at a time */
+        /* hub item: one segment per group; vertex item: the vertices of icost
+         * list entries + vertex costs, PER at a time */
         unsigned vs = 0, ve = 1;
         if (it >= nA) {
-          vs = warp_lower_bound(vcost, (unsigned)n, (long long)(it - nA) * kItemCost);
-          ve = warp_lower_bound(vcost, (unsigned)n, (long long)(it - nA + 1) * kItemCost);
+          warp_two_bounds(vcost, (unsigned)n, (long long)(it - nA) * icost,
+                          (long long)(it - nA + 1) * icost, vs, ve);
         }
         for (unsigned base = vs; base < ve; base += (it < nA ? 1u : (unsigned)PER)) {
           bool take = false, full = false;
