@@ -1,6 +1,7 @@
 """Batch levels cut into items of different sizes, against the exact oracle:
 one to a few edges, a handful of vertices for all warps, runs of empty lists
-between the owners of neighbouring edges, hubs, and every row width."""
+between the owners of neighbouring edges, hubs, counts added along a push
+level's own edges (past 2^32 and 2^63 too), and every row width."""
 import numpy as np
 import pytest
 
@@ -25,7 +26,20 @@ def fan_of_leaves(fan):
                              np.concatenate([v, [fan + 1, fan + 2]]))
 
 
+def fed_diamonds(k, feeders):
+    """k diamonds in a row, 2^k paths, and into each vertex an edge from every
+    one of `feeders` vertices that nothing leads to: few edges per level, long
+    in-lists."""
+    n = 3 * k + 1
+    v = 3 * np.arange(k)
+    src = [v, v, v + 1, v + 2, n + np.tile(np.arange(feeders), n)]
+    dst = [v + 1, v + 2, v + 3, v + 3, np.repeat(np.arange(n), feeders)]
+    return graphs.from_edges(n + feeders, np.concatenate(src), np.concatenate(dst))
+
+
 GRAPHS = {
+    "fed_diamonds_20": lambda: fed_diamonds(20, 300),
+    "fed_diamonds_70": lambda: fed_diamonds(70, 300),
     "chain": lambda: graphs.from_edges(70, np.arange(69), 1 + np.arange(69)),
     "sparse_lists": lambda: sparse(5000, 9000, 1),
     "leaves_31": lambda: fan_of_leaves(31),
@@ -55,3 +69,4 @@ def test_items(gpu_available, name, k):
                     assert stats[i]["visited"] == (S0 >= 0).sum()
                     if sigma:
                         assert np.array_equal(sg[i][ovf == 0], sg0[ovf == 0])
+                        assert bool(stats[i]["sigma_overflow"]) == bool(ovf.any())

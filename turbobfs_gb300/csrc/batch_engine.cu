@@ -32,7 +32,9 @@
  *   push  for small frontiers: edge-balanced over the out-lists of the
  *         queue of F_d, atomicOr of the new bits into F_{d+1}[v] (first
  *         touch of v appends it to the next queue), then a pull of the path
- *         counts over the in-lists of the new queue only.
+ *         counts over the in-lists of the new queue only -- or, where those
+ *         lists are much longer than the level's edges, atomic adds along
+ *         these.
  *
  * Direction rule per level: push while the frontier queue's out-edges times
  * alpha are below what a pull level costs -- the in-list entries of vertices
@@ -67,6 +69,9 @@ constexpr int kWarps = kBlock / 32;
 constexpr int kPushRounds = 8;    /* most 32-edge rounds per push work item    */
 constexpr int kClear = 256;       /* queue entries per row-clearing item        */
 constexpr int kVCost = 4;         /* a vertex costs like this many list entries */
+/* a push level adds counts along its edges when the new vertices' in-lists cost
+ * this many times as much */
+constexpr float kPullBack = 6.0f;
 #ifndef TBFS_BATCH_ITEM
 #define TBFS_BATCH_ITEM 512
 #endif
@@ -166,6 +171,12 @@ struct Grp {
 __device__ __host__ __forceinline__ int bit_of_root(int r, int W) {
   const int c = r >> 1, G = 4 * W;
   return 8 * (c % G) + 2 * (c / G) + (r & 1);
+}
+
+/* and back */
+__device__ __forceinline__ int root_of_bit(int b, int W) {
+  const int c = (b >> 3) + 4 * W * ((b & 7) >> 1);
+  return 2 * c + (b & 1);
 }
 
 /* this lane's 8-bit mask (its byte) of a row held in registers */
@@ -841,6 +852,8 @@ __global__ void __launch_bounds__(kBlock, TBFS_BATCH_MINB) fm_bfs_kernel(const B
   }
   if (!grid_barrier(ctl, p.timeout_ns, -1)) return;
 
+  /* graphs with hubs: a push level may add counts along its own edges (phase 2) */
+  const bool by_push = SIG != 0 && p.nhub > 0;
   unsigned ph = 0;            /* phase counter: work slot ph % 4 */
   unsigned long long md = 0;  /* this lane's newly finished in-list entries  */
   long long m_done = 0;       /* in-list entries of vertices every root reached,
@@ -940,23 +953,13 @@ __global__ void __launch_bounds__(kBlock, TBFS_BATCH_MINB) fm_bfs_kernel(const B
       /* rounds of an item: few on small levels, which have items for few warps */
       const unsigned rounds = min((qe + 32u * nwarps - 1u) / (32u * nwarps), (unsigned)kPushRounds);
       const unsigned nA = qe ? (qe + rounds * 32 - 1) / (rounds * 32) : 0u;
-      if (tid == 0) ctl->work[(ph + 2) & 3u] = 0u;
-      first_claim = true;
-      for (;;) {
-        const unsigned it = claim(nA + nclear);
-        if (it >= nA + nclear) break;
-        if (it >= nA) {
-          clear_item(it - nA);
-          continue;
-        }
+      /* visit(valid, u, v) for every out-edge u -> v of item `it` */
+      auto push_edges = [&](unsigned it, auto &&visit) {
         const unsigned *e0 = p.e[b0];
         unsigned o0 = dev::warp_find_owner(reinterpret_cast<const int *>(e0), qn, it * rounds * 32);
         for (unsigned r = 0; r < rounds; ++r) {
           const unsigned tb = it * (rounds * 32) + r * 32, t = tb + g.lane;
           if (tb >= qe) break;
-          bool first = false;
-          int v = 0;
-          unsigned dgo = 0;
           /* the owner among the 32 entries from the last one's; past them (many
            * empty lists) by a search of its own */
           const bool in = o0 + g.lane < qn;
@@ -970,6 +973,7 @@ __global__ void __launch_bounds__(kBlock, TBFS_BATCH_MINB) fm_bfs_kernel(const B
           unsigned eo = __shfl_sync(FULL, ew, (int)j);
           int u = __shfl_sync(FULL, qw, (int)j), a = __shfl_sync(FULL, aw, (int)j);
           unsigned o = o0 + j;
+          int v = 0;
           if (t < qe) {
             if (j == 31u && o + 1 < qn && __ldcg(e0 + o + 1) <= t) {
               o = upper_owner(e0, qn, t);
@@ -978,6 +982,24 @@ __global__ void __launch_bounds__(kBlock, TBFS_BATCH_MINB) fm_bfs_kernel(const B
               a = __ldg(p.rp + u);
             }
             v = __ldg(p.jr + a + (int)(t - eo));
+          }
+          o0 = __shfl_sync(FULL, o, 31);
+          visit(t < qe, u, v);
+        }
+      };
+      if (tid == 0) ctl->work[(ph + 2) & 3u] = 0u;
+      first_claim = true;
+      for (;;) {
+        const unsigned it = claim(nA + nclear);
+        if (it >= nA + nclear) break;
+        if (it >= nA) {
+          clear_item(it - nA);
+          continue;
+        }
+        push_edges(it, [&](bool valid, int u, int v) {
+          bool first = false;
+          unsigned dgo = 0;
+          if (valid) {
             unsigned fr[W], sv[W];
             load_row<W>(Fd + (size_t)u * W, fr);
             load_row<W>(p.seen + (size_t)v * W, sv);
@@ -986,8 +1008,18 @@ __global__ void __launch_bounds__(kBlock, TBFS_BATCH_MINB) fm_bfs_kernel(const B
             for (int w = 0; w < W; ++w) {
               const unsigned m = fr[w] & ~sv[w];
               if (m) {
-                atomicOr(&F1[(size_t)v * W + w], m);
                 any = true;
+                if (SIG && by_push) { /* depth and a count of 0, once, for each new root */
+                  unsigned nw = m & ~atomicOr(&F1[(size_t)v * W + w], m);
+                  for (; nw; nw &= nw - 1u) {
+                    const size_t at = (size_t)v * RS + root_of_bit(32 * w + __ffs(nw) - 1, W);
+                    p.S_int[at] = d + 1;
+                    if (SIG == 2) reinterpret_cast<unsigned *>(p.sig_int)[at] = 0u;
+                    else p.sig_int[at] = 0ull;
+                  }
+                } else {
+                  atomicOr(&F1[(size_t)v * W + w], m);
+                }
               }
             }
             if (any) {
@@ -1008,9 +1040,8 @@ __global__ void __launch_bounds__(kBlock, TBFS_BATCH_MINB) fm_bfs_kernel(const B
               }
             }
           }
-          o0 = __shfl_sync(FULL, o, 31);
           warp_enqueue(first, v, dgo, p.q[b1], p.e[b1], qctr1);
-        }
+        });
       }
       if (!grid_barrier(ctl, p.timeout_ns, d)) return;
       ++ph;
@@ -1021,6 +1052,60 @@ __global__ void __launch_bounds__(kBlock, TBFS_BATCH_MINB) fm_bfs_kernel(const B
       const unsigned hn1 = (unsigned)(hv >> 32), hsegs = (unsigned)hv;
       const unsigned qe1 = (unsigned)__ldcg(qctr1);
       const unsigned *e1 = p.e[b1];
+      if (SIG && by_push && (float)qe1 + (float)kVCost * (float)qn1 > kPullBack * (float)qe) {
+        /* The edges of phase 1 again: each adds its source's counts to its
+         * target's, and the new vertices are finished 32 at a time.  In the
+         * first levels of a batch few edges find vertices with long in-lists
+         * (255 roots on RMAT-20: 0.53 M edges, 27.7 M entries): 517 ->
+         * 139 us; 98 roots on RMAT of 100 K 76 -> 26. */
+        const unsigned nF = (qn1 + 31u) / 32u;
+        if (tid == 0) ctl->work[(ph + 2) & 3u] = 0u;
+        first_claim = true;
+        for (;;) {
+          const unsigned it = claim(nA + nF);
+          if (it >= nA + nF) break;
+          if (it >= nA) {
+            const unsigned idx = (it - nA) * 32u + g.lane;
+            if (idx < qn1) {
+              const int v = __ldcg(p.q[b1] + idx);
+              unsigned f1[W], sn[W];
+              load_row<W>(F1 + (size_t)v * W, f1);
+              load_row<W>(p.seen + (size_t)v * W, sn);
+#pragma unroll
+              for (int w = 0; w < W; ++w) sn[w] |= f1[w];
+              store_row<W>(p.seen + (size_t)v * W, sn);
+              atomicAnd(&p.touched[v >> 5], ~(1u << (v & 31)));
+              if (row_full<W>(p, sn, f1)) md += (unsigned)(__ldg(p.cp + v + 1) - __ldg(p.cp + v));
+            }
+            continue;
+          }
+          push_edges(it, [&](bool valid, int u, int v) {
+            if (!valid) return;
+            unsigned fr[W], f1[W];
+            load_row<W>(Fd + (size_t)u * W, fr);
+            load_row<W>(F1 + (size_t)v * W, f1);
+#pragma unroll
+            for (int w = 0; w < W; ++w) {
+              for (unsigned m = fr[w] & f1[w]; m; m &= m - 1u) {
+                const int r = root_of_bit(32 * w + __ffs(m) - 1, W);
+                const size_t from = (size_t)u * RS + r, to = (size_t)v * RS + r;
+                if (SIG == 2) {
+                  unsigned *c = reinterpret_cast<unsigned *>(p.sig_int);
+                  const unsigned x = c[from], old = atomicAdd(c + to, x);
+                  if (old + x < old) p.ctl->wide = 1;
+                } else {
+                  const unsigned long long x = p.sig_int[from], old = atomicAdd(p.sig_int + to, x);
+                  if (old + x < old || ((old + x) >> 63)) atomicOr(&p.ctl->ovf[r >> 5], 1u << (r & 31));
+                }
+              }
+            }
+          });
+        }
+        flush_md(d);
+        if (!grid_barrier(ctl, p.timeout_ns, d)) return;
+        ++ph;
+        continue;
+      }
       /* items of equal list entries + vertex costs over the queue */
       const long long cost2 = (long long)qe1 + (long long)kVCost * qn1;
       const unsigned icost2 = item_cost(cost2, qn1);
