@@ -107,7 +107,14 @@ tbfs_status ensure_ws(tbfs_graph *g, int W, bool sigma, cudaStream_t s) {
 #ifndef TBFS_BATCH_SEG
 #define TBFS_BATCH_SEG 128
 #endif
-    w->seg_len = TBFS_BATCH_SEG * W; /* a hub segment: about one work item of the pull */
+    /* A hub's segment: 32 entries per lane of its group (4 W lanes), on small
+     * graphs as few as leave every group one of the list entries' equal parts,
+     * at least 4, since a pull level takes at least one segment's chain of loads
+     * (RMAT, us per call with 32 throughout / so: 8000 vertices, 200 roots 396 /
+     * 238; 4000, 16 roots 218 / 161; 30 K, 250 roots 575 / 452). */
+    const long long groups = (long long)g->geom.sms * 24 * 8 / W;
+    w->seg_len = (int)std::min<long long>(
+        TBFS_BATCH_SEG * W, std::max<long long>(16 * W, (long long)g->nnz / std::max(groups, 1ll)));
     TRY(batch_hubs(g->cp, g->n, w->seg_len, &w->hubs, &w->hub_seg, &w->nhub, &w->hub_segs, s),
         "hub list");
     w->W = W;
