@@ -3,7 +3,8 @@
 Graphs whose out-lists hold at most 64 entries, at the sizes where the narrow
 levels can go wrong: chains (one vertex a level), even shares every 32 levels,
 a CTA with more than 64 and more than 256 finds in a level, levels that grow
-beyond what is narrow and shrink again, directed lists, counts past 2^63.
+beyond what is narrow and shrink again, directed lists, counts past 2^63 (also
+bottom-up, where parents are found by their depth then).
 """
 import numpy as np
 import pytest
@@ -96,7 +97,7 @@ GRAPHS = {
 }
 
 
-@pytest.mark.parametrize("mode", ["auto", "td"])
+@pytest.mark.parametrize("mode", ["auto", "td", "bu"])
 @pytest.mark.parametrize("name", sorted(GRAPHS))
 def test_narrow_levels(gpu_available, name, mode):
     n, src, dst, root = GRAPHS[name]()

@@ -471,6 +471,8 @@ struct Counts {
   const unsigned *filter;
   bool by_depth; /* counts may be zero: parents are found by their depth d */
   int d;
+  const int *S;
+  bool own; /* no in-list has more than kOwn entries */
 };
 
 /* exact sum of counts: 64 bits and the carries out of them */
@@ -512,7 +514,10 @@ __device__ __forceinline__ void sum_exact(const BfsParams &p, const Counts &c, u
 constexpr unsigned kBigCount = ~((1u << 20) - 1u);
 static_assert(kHubLen <= 1 << 12, "fast sums must fit 32 bits");
 
-/* the counts of u[0..U) (-1: none) as 32 bits; big collects the other bits */
+/* the counts of u[0..U) (-1: none) as 32 bits; big collects the other bits.  By
+ * depth: 1 for a parent, 0 for others; only lists with a parent are then
+ * summed (a level of a grid of 2048 x 2048, all bottom-up: 590 us with every
+ * list summed, 30 so) */
 template <bool FILTER, int U>
 __device__ __forceinline__ void get_fast(const Counts &c, const int (&u)[U], unsigned (&y)[U],
                                          unsigned &big) {
@@ -520,6 +525,14 @@ __device__ __forceinline__ void get_fast(const Counts &c, const int (&u)[U], uns
   bool on[U];
 #pragma unroll
   for (int j = 0; j < U; ++j) on[j] = u[j] >= 0;
+  if (c.by_depth) {
+    int sv[U];
+#pragma unroll
+    for (int j = 0; j < U; ++j) sv[j] = on[j] ? c.S[u[j]] : -1;
+#pragma unroll
+    for (int j = 0; j < U; ++j) y[j] = sv[j] == c.d ? 1u : 0u;
+    return;
+  }
   if (FILTER) {
     unsigned f[U];
 #pragma unroll
@@ -564,7 +577,7 @@ __device__ __forceinline__ void add_fast(const Counts &c, const int (&u)[U], uns
  * length in shared memory, 300 word by word without the lookahead, 252 so
  * (against 75 for an early-exit scan and 324 for a push of the counts after
  * it). */
-constexpr unsigned kOwn = 8, kHalf = 48;
+constexpr unsigned kOwn = 8, kHalf = 48; /* kOwn > 2^3 - 1: deg_bits < 4 */
 constexpr int kWords = 4; /* words of a group */
 static_assert(kWords * 32 <= kWin, "a group's vertices must fit the window");
 
@@ -601,9 +614,10 @@ __device__ __forceinline__ void pull_range(const BfsParams &p, Found &fd, const 
           on &= ~(1u << j);
         }
         any |= len != 0u;
+        if (c.own) continue;
         /* to the window: the lists for 8 lanes from the front of v[], those
          * for a warp from its back, both by slot; bounds in lo[], hi[] */
-        const bool exact = c.by_depth || len > (unsigned)kHubLen;
+        const bool exact = len > (unsigned)kHubLen;
         const bool is_l = len > kHalf && !exact, is_m = len > kOwn && len <= kHalf && !exact;
         const unsigned mm = __ballot_sync(FULL, is_m), ml = __ballot_sync(FULL, is_l);
         if (((on >> j) & 1u) && (len > kOwn || exact)) {
@@ -729,7 +743,18 @@ __device__ __forceinline__ void pull_range(const BfsParams &p, Found &fd, const 
         x = w.s[32 * j + lane];
         redo = w.a[32 * j + lane] != 0;
       }
-      bool found = x != 0u;
+      const unsigned n_par = x; /* by depth: parents */
+      if (c.by_depth && here && x != 0u) {
+        if ((other >> j) & 1u) {
+          redo = true;
+        } else { /* a short list: the lane alone */
+          unsigned long long sum = 0ull;
+          for (unsigned k = b; k < e; ++k) sum = add_chk(sum, c.src[__ldg(p.ic + k)], ovf);
+          x = (unsigned)sum;
+          s_hi = (unsigned)(sum >> 32);
+        }
+      }
+      bool found = x != 0u || s_hi != 0u || (c.by_depth && n_par != 0u);
       for (unsigned m = __ballot_sync(FULL, redo); m; m &= m - 1u) {
         const int l = __ffs(m) - 1;
         Sum s;
@@ -758,15 +783,14 @@ __device__ __forceinline__ void pull_segment(const BfsParams &p, Found &fd, cons
                                              unsigned long long *dst, int v, int lo, int hi,
                                              bool &ovf) {
   const unsigned lane = threadIdx.x & 31;
-  unsigned acc = 0u, big = c.by_depth ? 1u : 0u;
-  if (!c.by_depth) {
-    for (unsigned k = (unsigned)lo + lane; k - lane < (unsigned)hi; k += 256u) {
-      int u[8];
+  unsigned acc = 0u, big = 0u;
+  for (unsigned k = (unsigned)lo + lane; k - lane < (unsigned)hi; k += 256u) {
+    int u[8];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) u[j] = k + 32u * j < (unsigned)hi ? __ldg(p.ic + k + 32 * j) : -1;
-      add_fast<false, 8>(c, u, acc, big);
-    }
+    for (int j = 0; j < 8; ++j) u[j] = k + 32u * j < (unsigned)hi ? __ldg(p.ic + k + 32 * j) : -1;
+    add_fast<false, 8>(c, u, acc, big);
   }
+  if (c.by_depth) big = acc;
   Sum s = {__reduce_add_sync(FULL, acc), 0u, 0u};
   bool par = s.lo != 0u;
   if (__any_sync(FULL, big != 0u)) sum_exact(p, c, (unsigned)lo, (unsigned)hi, s, par);
@@ -1256,6 +1280,7 @@ __global__ void __launch_bounds__(SHORT ? kShortBlock : kBlock, 1)
   int d = 0, dir = DIR_TD, td = 0, bu = 0;
   long long m_u = p.out_edges_total, visited = 0, edges = 0;
   const float alpha = want_sigma ? p.alpha * kSigmaAlpha : p.alpha;
+  const bool own = p.deg_bits > 0 && p.deg_bits < 4; /* in-lists of at most kOwn entries */
   bool ovf = false, done = false;
   /* Bound on the bits of the path counts of F_d: sigma(F_0) = 1, and a count
    * of F_{d+1} sums at most max-in-degree counts of F_d, so it has at most
@@ -1367,7 +1392,9 @@ __global__ void __launch_bounds__(SHORT ? kShortBlock : kBlock, 1)
       ++bu;
       if (gtid == 0) ctl->collect = 0ull;
       n_seg = (n_hub + 31u) / 32u; /* 32 segments looked at per item */
-      heavy = want_sigma && p.tile && (float)m_u > kHeavyEntries &&
+      /* lists of about one length need no items of equal cost (grid of 1100 x
+       * 1100, all bottom-up: 19.5 us per level with them, 12.8 without) */
+      heavy = want_sigma && p.tile && !own && (float)m_u > kHeavyEntries &&
               (float)m_u > kHeavyShare * (float)p.nnz;
       if (heavy && s_filter && !no_queue && qn <= kFilterBits / 4u &&
           (float)m_u > kFilterGain * (float)qn) {
@@ -1401,7 +1428,7 @@ __global__ void __launch_bounds__(SHORT ? kShortBlock : kBlock, 1)
       /* even work needs no counter */
       if (want_sigma && !heavy) n_static = (n_all / nwarps + 1u) * nwarps;
     }
-    const Counts C = {src, filter, ovf_seen, d};
+    const Counts C = {src, filter, ovf_seen, d, p.S, own};
     unsigned *wctr = &ctl->work[d & 3];
     const int lane = threadIdx.x & 31;
     /* work items: the first n_static statically (one per warp, or several),
@@ -1594,8 +1621,12 @@ cudaError_t bfs_launch(const BfsParams &p0, const LaunchGeom &g, cudaStream_t s)
    * vertices 0.366 / 0.392, of 300 K 0.073 / 0.083, RMAT of 100 K 0.058 /
    * 0.065). */
   BfsParams p = p0;
-  const bool short_lists = p.short_lists != 0, sigma = p.sigma != nullptr;
-  const bool full = !sigma || (p.inv && p.nnz > kLargeEntries);
+  /* bottom-up levels alone, large ones, want threads, not the short-list
+   * instance's registers (grid of 2048 x 2048: 32 / 28 us per level, depths) */
+  const bool pulls = p.mode == TBFS_MODE_BOTTOM_UP && p.n > 1 << 20;
+  const bool short_lists = p.short_lists != 0 && !pulls;
+  const bool sigma = p.sigma != nullptr;
+  const bool full = !sigma || pulls || (p.inv && p.nnz > kLargeEntries);
   const int want = p.ctas_per_sm > 0 ? p.ctas_per_sm : short_lists ? 2 : full ? 4 : 3;
   int block = want < g.per_sm ? kBlockStep * want : g.block;
   if (short_lists && block > kShortBlock) block = kShortBlock;
