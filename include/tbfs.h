@@ -377,11 +377,11 @@ void tbfs_server_destroy(tbfs_server *s);
  * (d_out_ptr/d_out_idx; NULL for a symmetric graph), S[n] and sigma[n]
  * (sigma may be NULL for depths only).  Scratch (frontier queues, control
  * block) is a static device array inside the library sized for at most
- * TBFS_NOALLOC_MAX_VERTICES vertices (about 36 MB held on every GPU where
+ * TBFS_NOALLOC_MAX_VERTICES vertices (about 33 MB held on every GPU where
  * the library's device code is loaded, until exit); larger n is rejected
  * with TBFS_ERR_UNSUPPORTED.  The first call on a device looks up that
  * array's device address; since CUDA loads device code lazily, on a device
- * where nothing else of the library ran yet it also commits the 36 MB (a
+ * where nothing else of the library ran yet it also commits the 33 MB (a
  * warm-up call belongs before the host framework reserves device memory,
  * and before any stream capture; without the memory the call returns
  * TBFS_ERR_OUT_OF_MEMORY).  All calls share the array: calls whose GPU work
