@@ -71,21 +71,23 @@ constexpr int kInitBlock = 256;
  * by others is claimed and counted in L2.  (A claim and an add in L2 per edge,
  * both ends of every target's list and the source's count from L2: 9 us for
  * a level of 2300 edges.)
- *   A level of up to kLocalEnter edges costs less so than shared; an instance
- * is given back when it has outgrown kLocalLeave or the queue.  (192
- * graphs of 2^10 to 2^18 vertices: 12.5 -> 5.0 ms, of which 3.3 ms were two
- * memsets and two copies per graph on the host; 28 queries to a server of 14
- * such graphs: 8.3 -> 5.2 ms.  Us per level of a grid of 2^17.5 vertices,
- * ~2300 edges: 9.6 shared, 5.7 so; of 2^14, 10.2 and 3.3.  768 threads and
- * one CTA per SM against two of 384: 5.7 and 8.6.) */
+ *   A level of up to kLocalEnter edges costs no more so than shared; an instance
+ * is given back when it has outgrown kLocalLeave or the queue.  (192 graphs of
+ * 2^10 to 2^18 vertices: 12.5 -> 5.2 ms, of which 3.3 ms were two memsets and
+ * two copies per graph on the host; 28 queries to a server of 14 such graphs:
+ * 8.3 -> 5.2 ms.  Us per level of a grid of 2^14 vertices 10.2 -> 3.3.  With
+ * three times the limits 192 graphs took 5.0 ms, but levels of a single 1024 x
+ * 1024 grid 9.7 us instead of 8.8, and large instances waited for them.) */
 constexpr unsigned kLocalQueue = 2048;
 constexpr unsigned kSlotBits = 12, kSlots = 1u << kSlotBits, kProbe = 24;
 constexpr unsigned kNoKey = 0xffffffffu, kNoSlot = 0xffffu;
-constexpr unsigned kLocalEnter = 12288, kLocalLeave = 24576;
+constexpr unsigned kLocalEnter = 4096, kLocalLeave = 6144;
 /* A CTA gives its instance back for the next phase after this long: alone, so
- * that no CTA waits long at the barrier; beside wide instances, about a
- * shared level's time.  (In clocks of ~0.5 ns: the ns timer is slow to read.) */
-constexpr long long kLocalAlone = 500000, kLocalBeside = 60000;
+ * that no CTA waits long at the barrier; beside shared instances, about the
+ * time of a shared level (of kLocalEdges edges per clock), since a large deep
+ * instance waits for it at every one of its levels.  (In clocks of ~0.5 ns: the
+ * ns timer is slow to read.) */
+constexpr long long kLocalAlone = 500000, kLocalBeside = 20000, kLocalEdges = 8;
 constexpr int kLocalMine = 16;            /* instances of one CTA in a phase */
 constexpr unsigned kLocalGrid = kMultiMaxSlots / kLocalMine + 1; /* CTAs for that */
 constexpr unsigned kIsLocal = 0x80000000u;
@@ -201,6 +203,7 @@ __device__ __forceinline__ void local_run(const MultiParams &P, InstDesc &D, Loc
     visited += qn;
     edges += qe;
     int stop = 0;
+    const long long t_level = clock64();
     if (t == 0) {
       L.ctr[(d + 2) % 3] = 0ull;
       stop = dev::ld_volatile(&P.ctl->stop[ph & 1u]);
@@ -344,7 +347,10 @@ __device__ __forceinline__ void local_run(const MultiParams &P, InstDesc &D, Loc
         }
       }
     }
-    if (t == 0) L.leave[b] = stop || clock64() > t_end;
+    if (t == 0) { /* no time for another such level */
+      const long long now = clock64();
+      L.leave[b] = stop || now + (now - t_level) > t_end;
+    }
     __syncthreads();
     ++d;
     const unsigned long long cur = L.ctr[c1];
@@ -704,7 +710,8 @@ __global__ void __launch_bounds__(kBlock, TBFS_MULTI_PER_SM) multi_bfs_kernel(co
       it = __shfl_sync(FULL, nx, 0);
     }
     if (any_act & 1) { /* instances run by single CTAs */
-      const long long most = (any_act & 2) ? kLocalBeside : kLocalAlone;
+      const long long level = kLocalBeside + (long long)(etot / kLocalEdges);
+      const long long most = (any_act & 2) && level < kLocalAlone ? level : kLocalAlone;
       const long long span = most < P.timeout_ns / 4 ? most : P.timeout_ns / 4;
       const long long t_end = t_begin + span;
       int mine = 0;
