@@ -77,7 +77,9 @@ constexpr int kInitBlock = 256;
  * two copies per graph on the host; 28 queries to a server of 14 such graphs:
  * 8.3 -> 5.2 ms.  Us per level of a grid of 2^14 vertices 10.2 -> 3.3.  With
  * three times the limits 192 graphs took 5.0 ms, but levels of a single 1024 x
- * 1024 grid 9.7 us instead of 8.8, and large instances waited for them.) */
+ * 1024 grid 9.7 us instead of 8.8, and large instances waited for them;
+ * beside shared instances half of it: 4096 x 4096 grid beside two smaller ones
+ * 12.7 -> 12.4 us per level, against 11.0 with all levels shared.) */
 constexpr unsigned kLocalQueue = 2048;
 constexpr unsigned kSlotBits = 12, kSlots = 1u << kSlotBits, kProbe = 24;
 constexpr unsigned kNoKey = 0xffffffffu, kNoSlot = 0xffffu;
@@ -421,6 +423,7 @@ __global__ void __launch_bounds__(kBlock, TBFS_MULTI_PER_SM) multi_bfs_kernel(co
   __syncthreads();
 
   const bool use_local = gridDim.x >= kLocalGrid;
+  unsigned enter = kLocalEnter;
   unsigned ph = 0;
   for (; ph < (unsigned)P.max_phases; ++ph) {
     /* the host's "request waiting" flag (mapped host memory, a slow read):
@@ -471,7 +474,7 @@ __global__ void __launch_bounds__(kBlock, TBFS_MULTI_PER_SM) multi_bfs_kernel(co
         const bool done = dns[j];
         const unsigned long long qv = done ? 0ull : qvs[j];
         const unsigned qn = (unsigned)(qv >> 32), qe = (unsigned)qv;
-        loc[j] = use_local && qn && qn <= kLocalQueue && qe <= kLocalEnter;
+        loc[j] = use_local && qn && qn <= kLocalQueue && qe <= enter;
         s_qn[i] = loc[j] ? qn | kIsLocal : qn;
         s_qe[i] = qe;
         if (qn) {
@@ -709,6 +712,8 @@ __global__ void __launch_bounds__(kBlock, TBFS_MULTI_PER_SM) multi_bfs_kernel(co
       if (lane == 0) nx = nwarps + atomicAdd(&ctl->work[ph & 3u], 1u);
       it = __shfl_sync(FULL, nx, 0);
     }
+    /* beside shared instances only levels that are done before theirs */
+    enter = (any_act & 2) ? kLocalEnter / 2 : kLocalEnter;
     if (any_act & 1) { /* instances run by single CTAs */
       const long long level = kLocalBeside + (long long)(etot / kLocalEdges);
       const long long most = (any_act & 2) && level < kLocalAlone ? level : kLocalAlone;
