@@ -194,6 +194,9 @@ static tbfs_status graph_finish(tbfs_graph *g) {
       CUDA_TRY(tbfs::hub_segments(g->cp, g->n, g->hubs, g->hubs + 2, 0));
     }
   }
+  /* the lists and tables are complete on return: a traversal may run on a
+   * non-blocking stream, which is not ordered after this one */
+  CUDA_TRY(cudaStreamSynchronize(0));
   return TBFS_OK;
 }
 
