@@ -48,3 +48,38 @@ def test_first_traversal_on_a_side_stream(gpu_available):
         r = g.bfs(1, mode=mode, stream=side.cuda_stream)
         g.close()
         assert np.array_equal(r.S, S0) and np.array_equal(r.sigma, sg0)
+
+
+@pytest.mark.parametrize("sigma", [True, False])
+def test_arena_beside_other_kernels(gpu_available, sigma):
+    """CTAs of a launch that start at different times: matrix products on another
+    stream hold SMs while arenas of instances that are done in one to a few
+    levels, and of some that are not, are traversed."""
+    import torch
+    rng = np.random.default_rng(5)
+    hs, roots = [], []
+    for i in range(400):
+        if i % 40 == 39:
+            h = graphs.grid(48, seed=i)
+        else:
+            n = int(rng.integers(1, 40))
+            m = int(rng.integers(0, 2 * n))
+            h = graphs.from_edges(n, rng.integers(0, n, m), rng.integers(0, n, m), symmetrize=True)
+        hs.append(h)
+        roots.append(int(rng.integers(0, h.n)))
+    want = [oracle.exact_bfs(h.col_ptr, h.row_idx, r) for h, r in zip(hs, roots)]
+    side = torch.cuda.Stream()
+    a_mat = torch.ones(4096, 4096, dtype=torch.bfloat16, device="cuda")
+    torch.cuda.synchronize()
+    with tb.Arena(hs) as a:
+        for _ in range(20):
+            with torch.cuda.stream(side):
+                for _ in range(60):
+                    torch.mm(a_mat, a_mat)
+            S, sg, stats = a.bfs(roots, sigma=sigma)
+            sg = a.split(sg) if sigma else [None] * len(hs)
+            for s, x, st, (S0, sg0, ovf, levels) in zip(a.split(S), sg, stats, want):
+                assert np.array_equal(s, S0)
+                assert x is None or np.array_equal(x[ovf == 0], sg0[ovf == 0])
+                assert st["levels"] == levels and st["visited"] == (S0 >= 0).sum()
+    side.synchronize()

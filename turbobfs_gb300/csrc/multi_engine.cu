@@ -173,10 +173,46 @@ __device__ __forceinline__ unsigned lane_owner(const unsigned *e, unsigned cnt, 
   return lo;
 }
 
+/* Waits until every CTA has read what it plans the phase from: `want` arrivals
+ * at ctl->planned.  An instance's queue counters, level and done flag are read
+ * by all CTAs at the start of a phase and, for an instance that one CTA runs,
+ * written by that CTA within the same phase: it may not do so before the last
+ * of the others has them (a CTA that starts late, or is held up, would plan
+ * another phase than the rest, and an instance be run twice or by nobody).
+ * The arrivals of a phase are long there when an instance's first level is
+ * done.  Bounded like the grid barrier; called by the whole CTA. */
+__device__ __forceinline__ bool plans_read(MultiCtl *ctl, unsigned want, long long timeout_ns,
+                                           unsigned ph) {
+  __shared__ int s_ok;
+  if (threadIdx.x == 0) {
+    int ok = 1;
+    const unsigned long long t0 = dev::global_ns();
+    unsigned spins = 0;
+    while ((int)(dev::ld_acquire_u32(&ctl->planned) - want) < 0) {
+      if ((++spins & 31u) != 0) continue;
+      if (dev::ld_volatile(&ctl->status) != 0) {
+        ok = 0;
+        break;
+      }
+      if ((long long)(dev::global_ns() - t0) > timeout_ns) {
+        atomicCAS(&ctl->status, 0, (int)TBFS_ERR_TIMEOUT);
+        atomicCAS(&ctl->timeout_level, 0, (int)ph + 2);
+        ok = 0;
+        break;
+      }
+    }
+    s_ok = ok;
+  }
+  __syncthreads();
+  return s_ok != 0;
+}
+
 /* This CTA runs instance D from level d on (qn vertices, qe out-edges) until
- * it is finished or has outgrown a CTA, the clock t_end, or a stop request. */
-__device__ __forceinline__ void local_run(const MultiParams &P, InstDesc &D, LocalShared &L, int d,
-                                          unsigned qn, unsigned qe, unsigned ph,
+ * it is finished or has outgrown a CTA, the clock t_end, or a stop request.
+ * planned: arrivals after which D's counters may be written (plans_read);
+ * false: they did not come in time. */
+__device__ __forceinline__ bool local_run(const MultiParams &P, InstDesc &D, LocalShared &L, int d,
+                                          unsigned qn, unsigned qe, unsigned ph, unsigned planned,
                                           long long t_end) {
   const int t = threadIdx.x, lane = t & 31;
   const unsigned wid = (unsigned)t >> 5;
@@ -382,6 +418,7 @@ __device__ __forceinline__ void local_run(const MultiParams &P, InstDesc &D, Loc
         D.e[c1][i] = L.e[b ^ 1][i];
       }
       if (__any_sync(FULL, ovf) && lane == 0) atomicExch(&D.ovf, 1);
+      if (!plans_read(P.ctl, planned, P.timeout_ns, ph)) return false;
       if (t == 0) {
         D.ctr[c1] = cur;
         D.ctr[(d + 1) % 3] = 0ull;
@@ -396,7 +433,7 @@ __device__ __forceinline__ void local_run(const MultiParams &P, InstDesc &D, Loc
         }
       }
       __syncthreads(); /* before the next instance's queue */
-      return;
+      return true;
     }
     __syncthreads();
   }
@@ -424,6 +461,7 @@ __global__ void __launch_bounds__(kBlock, TBFS_MULTI_PER_SM) multi_bfs_kernel(co
 
   const bool use_local = gridDim.x >= kLocalGrid;
   unsigned enter = kLocalEnter;
+  unsigned planned = 0; /* arrivals at ctl->planned up to this phase */
   unsigned ph = 0;
   for (; ph < (unsigned)P.max_phases; ++ph) {
     /* the host's "request waiting" flag (mapped host memory, a slow read):
@@ -433,7 +471,9 @@ __global__ void __launch_bounds__(kBlock, TBFS_MULTI_PER_SM) multi_bfs_kernel(co
     const long long t_begin = clock64();
     if (t < kLocalMine) s_mine[t] = -1;
     /* ---- plan: identical in every CTA (reads counters finished before the
-     * last barrier); block sums and scans by warp shuffles ---- */
+     * last barrier: a shared instance's of this level are only added to, and
+     * those of an instance run by one CTA are written once all CTAs have read
+     * them, plans_read); block sums and scans by warp shuffles ---- */
     constexpr int kPer = (kMultiMaxSlots + kBlock - 1) / kBlock;
     /* every read of the plan in one round trip: the previous level's stop
      * word, each slot's done flag and queue counter, and (CTA 0) the totals
@@ -515,6 +555,12 @@ __global__ void __launch_bounds__(kBlock, TBFS_MULTI_PER_SM) multi_bfs_kernel(co
       any_act |= s_wact[w];
     }
     if (!any_act) break;
+    if (any_act & 1) { /* this CTA has read them */
+      planned += gridDim.x;
+      if (t == 0)
+        asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(&ctl->planned), "r"(1u)
+                     : "memory");
+    }
     /* rounds per item: enough items for every warp on small levels */
     const unsigned nwarps = gridDim.x * kWarps;
     const unsigned long long per_warp =
@@ -723,8 +769,9 @@ __global__ void __launch_bounds__(kBlock, TBFS_MULTI_PER_SM) multi_bfs_kernel(co
       while (mine < kLocalMine && s_mine[mine] >= 0) ++mine;
       for (int m = 0; m < mine; ++m) { /* equal parts of the time */
         const int i = s_mine[m];
-        local_run(P, I[i], L, s_d[i], s_qn[i] & ~kIsLocal, s_qe[i], ph,
-                  t_begin + span * (m + 1) / mine);
+        if (!local_run(P, I[i], L, s_d[i], s_qn[i] & ~kIsLocal, s_qe[i], ph, planned,
+                       t_begin + span * (m + 1) / mine))
+          return;
       }
       /* CTA 0 has none: it watches for requests until all others arrived */
       if (tid == 0 && P.wake) {

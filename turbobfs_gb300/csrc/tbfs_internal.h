@@ -311,7 +311,9 @@ struct __align__(128) MultiCtl {
                                  during the level, read after its barrier; two slots
                                  so that a CTA already in level ph+1 cannot write
                                  the word a slower CTA is still to read for ph */
-  int pad0[23];
+  unsigned planned;           /* CTAs that have read the inputs of their plan, summed over
+                                 the phases with instances run by one CTA */
+  int pad0[22];
   GridBarrier bar;
 };
 
