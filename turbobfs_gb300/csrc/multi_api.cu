@@ -31,7 +31,6 @@
 #include "tbfs_internal.h"
 
 using tbfs::InstDesc;
-using tbfs::LaunchGeom;
 using tbfs::MultiCtl;
 using tbfs::MultiParams;
 
@@ -128,7 +127,7 @@ struct tbfs_arena {
   InstDesc *inst = nullptr, *inst_host = nullptr;
   int *slots = nullptr;
   MultiCtl *ctl = nullptr, *ctl_host = nullptr;
-  LaunchGeom geom;
+  tbfs::MultiGeom geom;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 };
 
@@ -351,7 +350,7 @@ extern "C" tbfs_status tbfs_arena_bfs(tbfs_arena *a, const int32_t *roots, const
     p.wake = nullptr;
     p.stop_on_done = 0;
     MTRY(cudaEventRecord(a->ev0, s), "event");
-    MTRY(tbfs::multi_launch(p, a->geom, s), "multi launch");
+    MTRY(tbfs::multi_launch(p, a->geom, tbfs::multi_local(n_most), s), "multi launch");
     MTRY(cudaEventRecord(a->ev1, s), "event");
     MTRY(cudaMemcpyAsync(a->inst_host, a->inst, (size_t)k * sizeof(InstDesc),
                          cudaMemcpyDeviceToHost, s),
@@ -476,7 +475,7 @@ struct tbfs_server {
   InstDesc *inst = nullptr, *inst_host = nullptr;
   int *slot_ids = nullptr, *slot_ids_host = nullptr;
   MultiCtl *ctl = nullptr, *ctl_host = nullptr;
-  LaunchGeom geom;
+  tbfs::MultiGeom geom;
   cudaStream_t stream = nullptr;
   /* set by submit, read by the running launch at every level boundary */
   volatile int *wake_host = nullptr;
@@ -683,12 +682,14 @@ tbfs_status server_step(tbfs_server *sv, bool *idle) {
     carve(sv->mem + sl.off, D.n, r.sigma != nullptr, D);
     n_most = std::max(n_most, D.n);
   }
-  int nslots = 0;
+  int nslots = 0, n_run = 0; /* n_run: vertices of the largest instance that runs */
   for (int i = 0; i < sv->max_slots; ++i) {
-    if (sv->slots[(size_t)i].busy)
+    if (sv->slots[(size_t)i].busy) {
       nslots = i + 1;
-    else
+      n_run = std::max(n_run, sv->inst_host[i].n);
+    } else {
       sv->inst_host[i].done = 1; /* empty */
+    }
   }
   *idle = nslots == 0;
   if (nslots == 0) return TBFS_OK;
@@ -718,7 +719,7 @@ tbfs_status server_step(tbfs_server *sv, bool *idle) {
   p.stop_on_done = 1;
   const auto t_launch = std::chrono::steady_clock::now();
   MTRY(cudaMemsetAsync(sv->ctl, 0, sizeof(MultiCtl), s), "clear control block");
-  MTRY(tbfs::multi_launch(p, sv->geom, s), "multi launch");
+  MTRY(tbfs::multi_launch(p, sv->geom, tbfs::multi_local(n_run), s), "multi launch");
   MTRY(cudaMemcpyAsync(sv->inst_host, sv->inst, (size_t)nslots * sizeof(InstDesc),
                        cudaMemcpyDeviceToHost, s),
        "read descriptors");

@@ -46,11 +46,11 @@ namespace {
 using dev::FULL;
 using dev::grid_barrier;
 
-#ifndef TBFS_MULTI_PER_SM
-#define TBFS_MULTI_PER_SM 1
-#endif
-
-constexpr int kBlock = 768;
+/* Two instances of the kernel.  With one large CTA per SM a CTA can run an
+ * instance alone (below); with three of 256 threads, and an L1 not given away to
+ * the tables for that, the levels that all CTAs share are faster.  multi_local
+ * has the rule. */
+constexpr int kLocalBlock = 768, kSharedBlock = 256, kSharedPerSm = 3;
 constexpr int kEPT = 4;                   /* consecutive edges per lane per round */
 constexpr unsigned kRoundEdges = 32 * kEPT;
 constexpr int kMaxRounds = 8;             /* rounds per item, fewer on small levels */
@@ -93,6 +93,15 @@ constexpr long long kLocalAlone = 500000, kLocalBeside = 20000, kLocalEdges = 8;
 constexpr int kLocalMine = 16;            /* instances of one CTA in a phase */
 constexpr unsigned kLocalGrid = kMultiMaxSlots / kLocalMine + 1; /* CTAs for that */
 constexpr unsigned kIsLocal = 0x80000000u;
+/* Vertices of a launch's largest unfinished instance up to which the kernel with
+ * one-CTA instances runs it (multi_local).  The levels of larger ones are mostly
+ * shared, and the small ones beside them wait for those; a server whose large
+ * queries take 10 % longer is that much nearer to saturation.  Us per shared
+ * level of one grid, kernel without / with: 512 x 512 9.3 / 5.2, 1024 x 1024 8.8 /
+ * 8.1, 1448 x 1448 9.0 / 8.9, 2048 x 2048 10.0 / 10.4, 4096 x 4096 10.3 / 11.5;
+ * 64 graphs of up to 4096 x 4096 served at 400 queries/s, p50 / p99 14 / 100 ms
+ * without and, all in the kernel with, 15-25 / 137-632. */
+constexpr int kLocalVertices = 1 << 20;
 
 struct LocalShared {
   int v[2][kLocalQueue], a[2][kLocalQueue]; /* level d in [d & 1]: vertex, list start */
@@ -219,14 +228,14 @@ __device__ __forceinline__ bool local_run(const MultiParams &P, InstDesc &D, Loc
   const int *rp = D.rp, *jr = D.jr;
   int *S = D.S;
   unsigned long long *sig = D.sig;
-  for (unsigned i = t; i < qn; i += kBlock) {
+  for (unsigned i = t; i < qn; i += kLocalBlock) {
     const int v = __ldcg(D.q[d % 3] + i);
     L.v[d & 1][i] = v;
     L.e[d & 1][i] = __ldcg(D.e[d % 3] + i);
     L.a[d & 1][i] = __ldg(rp + v);
     if (sig) L.cnt[d & 1][i] = __ldcg(sig + v);
   }
-  for (unsigned i = t; i < kSlots; i += kBlock) {
+  for (unsigned i = t; i < kSlots; i += kLocalBlock) {
     L.key[i] = kNoKey;
     L.lo[i] = L.hi[i] = 0u;
   }
@@ -249,7 +258,7 @@ __device__ __forceinline__ bool local_run(const MultiParams &P, InstDesc &D, Loc
     const bool chk = sig && !ovf_seen && !(bits > 0 && 1 + (long long)(d + 1) * bits <= 63);
     /* a contiguous piece of the level's edges per warp, up to kEPT rounds of
      * 32 in flight */
-    const unsigned steps = (qe + kBlock - 1u) / kBlock;
+    const unsigned steps = (qe + kLocalBlock - 1u) / kLocalBlock;
     const unsigned lim = min(qe, (wid + 1u) * steps * 32u);
     const bool early = steps <= 2u; /* latency counts: where the targets' lists are, unasked */
     const unsigned *le = L.e[b];
@@ -396,7 +405,7 @@ __device__ __forceinline__ bool local_run(const MultiParams &P, InstDesc &D, Loc
     qe = (unsigned)cur;
     /* the counts to memory, and the table empty again */
     if (qn <= kLocalQueue) {
-      for (unsigned i = t; i < qn; i += kBlock) {
+      for (unsigned i = t; i < qn; i += kLocalBlock) {
         const unsigned s = L.slot[i];
         const int v = L.v[b ^ 1][i];
         if (s != kNoSlot) {
@@ -409,11 +418,11 @@ __device__ __forceinline__ bool local_run(const MultiParams &P, InstDesc &D, Loc
         }
       }
     } else if (sig) { /* the instance leaves */
-      for (unsigned s = t; s < kSlots; s += kBlock)
+      for (unsigned s = t; s < kSlots; s += kLocalBlock)
         if (L.key[s] != kNoKey) sig[L.key[s]] = ((unsigned long long)L.hi[s] << 32) | L.lo[s];
     }
     if (qn == 0u || qn > kLocalQueue || qe > kLocalLeave || L.leave[b]) {
-      for (unsigned i = t; i < qn && i < kLocalQueue; i += kBlock) {
+      for (unsigned i = t; i < qn && i < kLocalQueue; i += kLocalBlock) {
         D.q[c1][i] = L.v[b ^ 1][i];
         D.e[c1][i] = L.e[b ^ 1][i];
       }
@@ -439,10 +448,12 @@ __device__ __forceinline__ bool local_run(const MultiParams &P, InstDesc &D, Loc
   }
 }
 
-__global__ void __launch_bounds__(kBlock, TBFS_MULTI_PER_SM) multi_bfs_kernel(const MultiParams P) {
+template <bool LOCAL>
+__global__ void __launch_bounds__(LOCAL ? kLocalBlock : kSharedBlock, LOCAL ? 1 : kSharedPerSm)
+    multi_bfs_kernel(const MultiParams P) {
+  constexpr int kBlock = LOCAL ? kLocalBlock : kSharedBlock;
   extern __shared__ __align__(16) unsigned char s_dyn[];
-  LocalShared &L = *reinterpret_cast<LocalShared *>(s_dyn);
-  __shared__ int s_mine[kLocalMine];             /* this CTA's instances */
+  __shared__ int s_mine[LOCAL ? kLocalMine : 1]; /* this CTA's instances */
   constexpr int kWarps = kBlock / 32;
   __shared__ unsigned s_pre[kMultiMaxSlots + 1]; /* item prefix over slots      */
   __shared__ int s_d[kMultiMaxSlots];            /* level each slot runs next   */
@@ -459,7 +470,7 @@ __global__ void __launch_bounds__(kBlock, TBFS_MULTI_PER_SM) multi_bfs_kernel(co
   for (int i = t; i < ns; i += kBlock) s_d[i] = __ldcg(&I[i].d);
   __syncthreads();
 
-  const bool use_local = gridDim.x >= kLocalGrid;
+  const bool use_local = LOCAL && gridDim.x >= kLocalGrid;
   unsigned enter = kLocalEnter;
   unsigned planned = 0; /* arrivals at ctl->planned up to this phase */
   unsigned ph = 0;
@@ -469,7 +480,7 @@ __global__ void __launch_bounds__(kBlock, TBFS_MULTI_PER_SM) multi_bfs_kernel(co
     int wake_now = 0;
     if (tid == 0 && P.wake) wake_now = *P.wake;
     const long long t_begin = clock64();
-    if (t < kLocalMine) s_mine[t] = -1;
+    if (LOCAL && t < kLocalMine) s_mine[t] = -1;
     /* ---- plan: identical in every CTA (reads counters finished before the
      * last barrier: a shared instance's of this level are only added to, and
      * those of an instance run by one CTA are written once all CTAs have read
@@ -555,7 +566,7 @@ __global__ void __launch_bounds__(kBlock, TBFS_MULTI_PER_SM) multi_bfs_kernel(co
       any_act |= s_wact[w];
     }
     if (!any_act) break;
-    if (any_act & 1) { /* this CTA has read them */
+    if (LOCAL && (any_act & 1)) { /* this CTA has read them */
       planned += gridDim.x;
       if (t == 0)
         asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(&ctl->planned), "r"(1u)
@@ -599,7 +610,7 @@ __global__ void __launch_bounds__(kBlock, TBFS_MULTI_PER_SM) multi_bfs_kernel(co
       const int i = t * kPer + j;
       if (i < ns) s_pre[i] = run;
       run += items[j];
-      if (loc[j]) { /* instance `rank` of the local ones, on CTA 1 and up */
+      if (LOCAL && loc[j]) { /* instance `rank` of the local ones, on CTA 1 and up */
         if (rank % (gridDim.x - 1u) + 1u == blockIdx.x) s_mine[rank / (gridDim.x - 1u)] = i;
         ++rank;
       }
@@ -760,7 +771,8 @@ __global__ void __launch_bounds__(kBlock, TBFS_MULTI_PER_SM) multi_bfs_kernel(co
     }
     /* beside shared instances only levels that are done before theirs */
     enter = (any_act & 2) ? kLocalEnter / 2 : kLocalEnter;
-    if (any_act & 1) { /* instances run by single CTAs */
+    if (LOCAL && (any_act & 1)) { /* instances run by single CTAs */
+      LocalShared &L = *reinterpret_cast<LocalShared *>(s_dyn);
       const long long level = kLocalBeside + (long long)(etot / kLocalEdges);
       const long long most = (any_act & 2) && level < kLocalAlone ? level : kLocalAlone;
       const long long span = most < P.timeout_ns / 4 ? most : P.timeout_ns / 4;
@@ -786,7 +798,7 @@ __global__ void __launch_bounds__(kBlock, TBFS_MULTI_PER_SM) multi_bfs_kernel(co
     if (tid == 0 && wake_now) ctl->stop[ph & 1u] = 1;
     if (!grid_barrier(ctl, P.timeout_ns, (int)ph)) return;
     for (int i = t; i < ns; i += kBlock) {
-      if (s_qn[i] & kIsLocal) s_d[i] = __ldcg(&I[i].d);
+      if (LOCAL && (s_qn[i] & kIsLocal)) s_d[i] = __ldcg(&I[i].d);
       else if (s_qn[i]) s_d[i] += 1;
     }
     __syncthreads();
@@ -851,32 +863,41 @@ __global__ void __launch_bounds__(kInitBlock) multi_pack_kernel(const InstDesc *
 
 }  // namespace
 
-cudaError_t multi_geometry(int device, LaunchGeom *out) {
-  int sms = 0, coop = 0, per = 0;
+static const void *multi_kernel(bool local) {
+  return local ? reinterpret_cast<const void *>(multi_bfs_kernel<true>)
+               : reinterpret_cast<const void *>(multi_bfs_kernel<false>);
+}
+
+static size_t multi_smem(bool local) { return local ? sizeof(LocalShared) : 0; }
+
+bool multi_local(int n_most) { return n_most <= kLocalVertices; }
+
+cudaError_t multi_geometry(int device, MultiGeom *out) {
+  int sms = 0, coop = 0;
   cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   if (e != cudaSuccess) return e;
   e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
   if (e != cudaSuccess) return e;
   if (!coop) return cudaErrorNotSupported;
-  e = cudaFuncSetAttribute(multi_bfs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)sizeof(LocalShared));
-  if (e != cudaSuccess) return e;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, multi_bfs_kernel, kBlock,
-                                                    sizeof(LocalShared));
-  if (e != cudaSuccess) return e;
-  if (per < 1) return cudaErrorInvalidConfiguration;
-  /* one large CTA per SM: all of an SM for an instance that a CTA runs alone,
-   * few barrier arrivals for the others */
-  if (per > TBFS_MULTI_PER_SM) per = TBFS_MULTI_PER_SM;
-  out->block = kBlock;
-  out->grid = sms * per;
-  return cudaSuccess;
+  e = cudaFuncSetAttribute(multi_kernel(true), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)multi_smem(true));
+  for (int local = 0; local < 2 && e == cudaSuccess; ++local) {
+    const int block = local ? kLocalBlock : kSharedBlock, most = local ? 1 : kSharedPerSm;
+    int per = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, multi_kernel(local != 0), block,
+                                                      multi_smem(local != 0));
+    if (e == cudaSuccess && per < 1) e = cudaErrorInvalidConfiguration;
+    out->shape[local].block = block;
+    out->shape[local].grid = sms * std::min(per, most);
+  }
+  return e;
 }
 
-cudaError_t multi_launch(const MultiParams &p, const LaunchGeom &g, cudaStream_t s) {
+cudaError_t multi_launch(const MultiParams &p, const MultiGeom &g, bool local, cudaStream_t s) {
   void *args[] = {const_cast<MultiParams *>(&p)};
-  return cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(multi_bfs_kernel), dim3(g.grid),
-                                     dim3(g.block), args, sizeof(LocalShared), s);
+  const LaunchGeom &shape = g.shape[local ? 1 : 0];
+  return cudaLaunchCooperativeKernel(multi_kernel(local), dim3(shape.grid), dim3(shape.block), args,
+                                     multi_smem(local), s);
 }
 
 /* blocks (x) for the k instances of a launch, the largest of n vertices, each

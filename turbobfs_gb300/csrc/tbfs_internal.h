@@ -327,8 +327,15 @@ struct MultiParams {
   int stop_on_done;           /* end the launch after a level that finished an instance */
 };
 
-cudaError_t multi_geometry(int device, LaunchGeom *out);
-cudaError_t multi_launch(const MultiParams &p, const LaunchGeom &g, cudaStream_t s);
+struct MultiGeom {
+  LaunchGeom shape[2]; /* all instances shared by all CTAs; small ones run by one CTA */
+};
+
+cudaError_t multi_geometry(int device, MultiGeom *out);
+/* whether a launch whose largest unfinished instance has n_most vertices runs
+ * its small instances on one CTA each */
+bool multi_local(int n_most);
+cudaError_t multi_launch(const MultiParams &p, const MultiGeom &g, bool local, cudaStream_t s);
 /* initialise the descriptors slots[0..k), of graphs of at most n_most vertices */
 cudaError_t multi_init(InstDesc *inst, const int *slots, int k, int n_most, cudaStream_t s);
 /* S_out[inst.out + j] = inst.S[j] for the first k descriptors; sig likewise when
