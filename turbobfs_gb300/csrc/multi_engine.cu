@@ -71,19 +71,20 @@ constexpr int kInitBlock = 256;
  * by others is claimed and counted in L2.  (A claim and an add in L2 per edge,
  * both ends of every target's list and the source's count from L2: 9 us for
  * a level of 2300 edges.)
- *   A level of up to kLocalEnter edges costs no more so than shared; an instance
- * is given back when it has outgrown kLocalLeave or the queue.  (192 graphs of
- * 2^10 to 2^18 vertices: 12.5 -> 5.2 ms, of which 3.3 ms were two memsets and
- * two copies per graph on the host; 28 queries to a server of 14 such graphs:
- * 8.3 -> 5.2 ms.  Us per level of a grid of 2^14 vertices 10.2 -> 3.3.  With
- * three times the limits 192 graphs took 5.0 ms, but levels of a single 1024 x
- * 1024 grid 9.7 us instead of 8.8, and large instances waited for them;
- * beside shared instances half of it: 4096 x 4096 grid beside two smaller ones
- * 12.7 -> 12.4 us per level, against 11.0 with all levels shared.) */
+ *   A level of up to kLocalEnter edges costs no more so than shared, twice as many
+ * beside more than kFew other instances, since a shared level is longer then; an
+ * instance is given back when it has outgrown half as many again, or the queue.
+ * (192 graphs of 2^10 to 2^18 vertices: 12.5 -> 5.2 ms, of which 3.3 ms were two
+ * memsets and two copies per graph on the host; 28 queries to a server of 14 such
+ * graphs: 8.3 -> 5.2 ms.  Us per level of a grid of 2^14 vertices 10.2 -> 3.3.
+ * Limits of 4096 alone / of 8192 alone / halved beside shared instances, ms: a
+ * 1024 x 1024 grid 9.4 / 10.2 / 9.7, six of 700 x 700 9.6 / 5.9 / 8.5, 192 other
+ * graphs of up to 2^18 vertices 5.3 / 5.3 / 11.0, 64 of up to 2^20 13.6 / 11.6 /
+ * 16.2, 512 of them 37.6 / 26.4 / 36.1.) */
 constexpr unsigned kLocalQueue = 2048;
 constexpr unsigned kSlotBits = 12, kSlots = 1u << kSlotBits, kProbe = 24;
 constexpr unsigned kNoKey = 0xffffffffu, kNoSlot = 0xffffu;
-constexpr unsigned kLocalEnter = 4096, kLocalLeave = 6144;
+constexpr unsigned kLocalEnter = 4096, kFew = 4;
 /* A CTA gives its instance back for the next phase after this long: alone, so
  * that no CTA waits long at the barrier; beside shared instances, about the
  * time of a shared level (of kLocalEdges edges per clock), since a large deep
@@ -217,12 +218,13 @@ __device__ __forceinline__ bool plans_read(MultiCtl *ctl, unsigned want, long lo
 }
 
 /* This CTA runs instance D from level d on (qn vertices, qe out-edges) until
- * it is finished or has outgrown a CTA, the clock t_end, or a stop request.
+ * it is finished or has outgrown a CTA (`most` edges), the clock t_end, or a
+ * stop request.
  * planned: arrivals after which D's counters may be written (plans_read);
  * false: they did not come in time. */
 __device__ __forceinline__ bool local_run(const MultiParams &P, InstDesc &D, LocalShared &L, int d,
-                                          unsigned qn, unsigned qe, unsigned ph, unsigned planned,
-                                          long long t_end) {
+                                          unsigned qn, unsigned qe, unsigned most, unsigned ph,
+                                          unsigned planned, long long t_end) {
   const int t = threadIdx.x, lane = t & 31;
   const unsigned wid = (unsigned)t >> 5;
   const int *rp = D.rp, *jr = D.jr;
@@ -421,7 +423,7 @@ __device__ __forceinline__ bool local_run(const MultiParams &P, InstDesc &D, Loc
       for (unsigned s = t; s < kSlots; s += kLocalBlock)
         if (L.key[s] != kNoKey) sig[L.key[s]] = ((unsigned long long)L.hi[s] << 32) | L.lo[s];
     }
-    if (qn == 0u || qn > kLocalQueue || qe > kLocalLeave || L.leave[b]) {
+    if (qn == 0u || qn > kLocalQueue || qe > most || L.leave[b]) {
       for (unsigned i = t; i < qn && i < kLocalQueue; i += kLocalBlock) {
         D.q[c1][i] = L.v[b ^ 1][i];
         D.e[c1][i] = L.e[b ^ 1][i];
@@ -579,11 +581,11 @@ __global__ void __launch_bounds__(LOCAL ? kLocalBlock : kSharedBlock, LOCAL ? 1 
     const unsigned rounds = (unsigned)max(1ull, min((unsigned long long)kMaxRounds, per_warp));
     const unsigned iedges = kRoundEdges * rounds;
     unsigned items[kPer];
-    unsigned long long sum = 0; /* (local instances << 32) | items */
+    unsigned long long sum = 0; /* instances shared << 48 | run by one CTA << 32 | items */
 #pragma unroll
     for (int j = 0; j < kPer; ++j) {
       items[j] = (qes[j] + iedges - 1) / iedges;
-      sum += items[j] + (loc[j] ? 1ull << 32 : 0ull);
+      sum += items[j] + (loc[j] ? 1ull << 32 : 0ull) + (items[j] ? 1ull << 48 : 0ull);
     }
     /* exclusive scan of the per-thread sums: within the warp by shuffles,
      * across the warps from their totals */
@@ -604,7 +606,7 @@ __global__ void __launch_bounds__(LOCAL ? kLocalBlock : kSharedBlock, LOCAL ? 1 
     }
     const unsigned total = (unsigned)wtot;
     unsigned run = (unsigned)(wbase + inc - sum);
-    unsigned rank = (unsigned)((wbase + inc - sum) >> 32);
+    unsigned rank = (unsigned)((wbase + inc - sum) >> 32) & 0xffffu;
 #pragma unroll
     for (int j = 0; j < kPer; ++j) {
       const int i = t * kPer + j;
@@ -769,8 +771,6 @@ __global__ void __launch_bounds__(LOCAL ? kLocalBlock : kSharedBlock, LOCAL ? 1 
       if (lane == 0) nx = nwarps + atomicAdd(&ctl->work[ph & 3u], 1u);
       it = __shfl_sync(FULL, nx, 0);
     }
-    /* beside shared instances only levels that are done before theirs */
-    enter = (any_act & 2) ? kLocalEnter / 2 : kLocalEnter;
     if (LOCAL && (any_act & 1)) { /* instances run by single CTAs */
       LocalShared &L = *reinterpret_cast<LocalShared *>(s_dyn);
       const long long level = kLocalBeside + (long long)(etot / kLocalEdges);
@@ -781,7 +781,8 @@ __global__ void __launch_bounds__(LOCAL ? kLocalBlock : kSharedBlock, LOCAL ? 1 
       while (mine < kLocalMine && s_mine[mine] >= 0) ++mine;
       for (int m = 0; m < mine; ++m) { /* equal parts of the time */
         const int i = s_mine[m];
-        if (!local_run(P, I[i], L, s_d[i], s_qn[i] & ~kIsLocal, s_qe[i], ph, planned,
+        if (!local_run(P, I[i], L, s_d[i], s_qn[i] & ~kIsLocal, s_qe[i], enter + enter / 2,
+                       ph, planned,
                        t_begin + span * (m + 1) / mine))
           return;
       }
@@ -794,6 +795,8 @@ __global__ void __launch_bounds__(LOCAL ? kLocalBlock : kSharedBlock, LOCAL ? 1 
         if (wake_now) *(volatile int *)&ctl->stop[ph & 1u] = 1;
       }
     }
+    enter = (unsigned)(wtot >> 48) + ((unsigned)(wtot >> 32) & 0xffffu) > kFew ? 2 * kLocalEnter
+                                                                               : kLocalEnter;
     /* a waiting request (host flag) ends the launch after this level */
     if (tid == 0 && wake_now) ctl->stop[ph & 1u] = 1;
     if (!grid_barrier(ctl, P.timeout_ns, (int)ph)) return;
