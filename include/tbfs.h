@@ -277,8 +277,9 @@ tbfs_status tbfs_graph_degree_stats(tbfs_graph *g, int32_t kind, tbfs_degree_sta
  * direction parameters, then every combination of a grid of those at the
  * chosen shape) and writes them into *opt, leaving its other fields as they
  * are.  With cache_path (a text file; NULL: no cache) the result is stored
- * under a key made of the graph's degree-profile shape, and a later call on
- * a graph with the same key returns the stored values without timing
+ * under a key made of the graph's degree-profile shape and the engine's
+ * version (values that another version stored are not used), and a later call
+ * on a graph with the same key returns the stored values without timing
  * (*from_cache = 1). */
 tbfs_status tbfs_autotune(tbfs_graph *g, const int32_t *roots, int32_t k, const char *cache_path,
                           tbfs_options *opt, int32_t *from_cache);

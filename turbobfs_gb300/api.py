@@ -308,8 +308,9 @@ class Graph:
         return out
 
     def autotune(self, roots, cache: str | None = None, **kw) -> dict:
-        """Tuned {'alpha', 'beta', 'pull_ratio', 'from_cache'} for this graph
-        (timed on ``roots``; cached per degree profile in ``cache``)."""
+        """Tuned {'alpha', 'beta', 'max_ept', 'ctas_per_sm', 'from_cache'} for
+        this graph (timed on ``roots``; cached per degree profile in ``cache``).
+        'pull_ratio' is kept in the result and has no effect (always 1)."""
         roots = _i32(roots)
         o = make_options("auto", True, **kw)
         fc = ctypes.c_int32()

@@ -174,7 +174,18 @@ std::string profile_key(const tbfs_graph *g, const int64_t *hist, int64_t maxd) 
   return std::string(buf) + (g->separate_out ? "_dir" : "_sym");
 }
 
-/* a cache line: "key alpha beta pull_ratio [max_ept ctas_per_sm]" */
+/* The key of the single-source engine's settings: the profile, the kernel
+ * instance it runs (graphs with and without long out-lists, whose limit lies
+ * within a profile's range of entries) and the meaning of the settings, counted
+ * up when that changes, so that values stored for another meaning are not found.
+ * 2: alpha is scaled for traversals with path counts, ctas_per_sm is in units of
+ * 256 threads. */
+std::string engine_key(const tbfs_graph *g, const int64_t *hist, int64_t maxd) {
+  return profile_key(g, hist, maxd) + (g->short_lists ? "_short" : "") + "_v2";
+}
+
+/* a cache line: "key alpha beta pull_ratio [max_ept ctas_per_sm]"; pull_ratio
+ * has no effect and stays 1 */
 struct Tuned {
   float a = 15.0f, b = 2.0f, pr = 1.0f;
   int ept = 0, ctas = 0;
@@ -378,7 +389,7 @@ extern "C" tbfs_status tbfs_autotune(tbfs_graph *g, const int32_t *roots, int32_
   int64_t hist[tbfs::kBuckets], maxd = 0;
   tbfs_status st = tbfs_graph_degree_profile(g, hist, &maxd, nullptr);
   if (st != TBFS_OK) return st;
-  const std::string key = tbfs::profile_key(g, hist, maxd);
+  const std::string key = tbfs::engine_key(g, hist, maxd);
   tbfs::Tuned best;
   if (from_cache) *from_cache = 0;
   if (tbfs::cache_lookup(cache_path, key, &best)) {
