@@ -882,9 +882,16 @@ __global__ void __launch_bounds__(kBlock, TBFS_BATCH_MINB) fm_bfs_kernel(const B
    * of kItemCost and 256 edges throughout against this, per level or call: grid
    * of 200 x 200, 64 roots, 90 / 17 us; Erdos-Renyi of 30 K vertices, 200 roots,
    * 1.00 / 0.40 ms; RMAT of 200 K, 40 roots, 0.38 / 0.31 ms.) */
+  const float per_warp = 1.0f / (2.0f * (float)nwarps);
   auto item_cost = [&](long long cost, unsigned cnt) -> unsigned {
     const float c = (float)cost, v = (float)max(cnt, 1u);
-    return (unsigned)fminf(fmaxf(c / (2.0f * (float)nwarps), c / v * PER) + 1.0f, (float)kItemCost);
+    return (unsigned)fminf(fmaxf(c * per_warp, __fdividef(c, v) * PER) + 1.0f, (float)kItemCost);
+  };
+  /* items of that cost; a 64-bit division is a fifth of a microsecond of a small
+   * level */
+  auto items_of = [&](long long cost, unsigned icost) -> unsigned {
+    const long long c = cost + icost - 1;
+    return (c >> 32) == 0 ? (unsigned)c / icost : (unsigned)(c / icost);
   };
   /* entries finished during level d go to slot (d + 1) % 4, read at the
    * start of level d + 1 */
@@ -951,8 +958,11 @@ __global__ void __launch_bounds__(kBlock, TBFS_BATCH_MINB) fm_bfs_kernel(const B
     if (push) {
       /* ---- phase 1: discovery over the out-edges of Q_d ---- */
       /* rounds of an item: few on small levels, which have items for few warps */
-      const unsigned rounds = min((qe + 32u * nwarps - 1u) / (32u * nwarps), (unsigned)kPushRounds);
-      const unsigned nA = qe ? (qe + rounds * 32 - 1) / (rounds * 32) : 0u;
+      const unsigned rounds =
+          qe <= 32u * nwarps
+              ? 1u
+              : min((qe + 32u * nwarps - 1u) / (32u * nwarps), (unsigned)kPushRounds);
+      const unsigned nA = rounds == 1u ? (qe + 31u) / 32u : (qe + rounds * 32 - 1) / (rounds * 32);
       /* visit(valid, u, v) for every out-edge u -> v of item `it` */
       auto push_edges = [&](unsigned it, auto &&visit) {
         const unsigned *e0 = p.e[b0];
@@ -1116,7 +1126,7 @@ __global__ void __launch_bounds__(kBlock, TBFS_BATCH_MINB) fm_bfs_kernel(const B
       /* items of equal list entries + vertex costs over the queue */
       const long long cost2 = (long long)qe1 + (long long)kVCost * qn1;
       const unsigned icost2 = item_cost(cost2, qn1);
-      const unsigned nA2 = (unsigned)((cost2 + icost2 - 1) / icost2);
+      const unsigned nA2 = items_of(cost2, icost2);
       const unsigned nB2 = (hsegs + PER - 1) / PER;
       auto qcost = [&](unsigned i) -> long long {
         return (long long)__ldcg(e1 + i) + (long long)kVCost * i;
@@ -1166,7 +1176,7 @@ __global__ void __launch_bounds__(kBlock, TBFS_BATCH_MINB) fm_bfs_kernel(const B
       const unsigned nA = ((unsigned)p.hub_segs + PER - 1) / PER;
       const long long cost = p.nnz_in + (long long)kVCost * n;
       const unsigned icost = item_cost(cost, (unsigned)n);
-      const unsigned nB = (unsigned)((cost + icost - 1) / icost);
+      const unsigned nB = items_of(cost, icost);
       auto vcost = [&](unsigned v) -> long long {
         return (long long)__ldg(p.cp + v) + (long long)kVCost * v;
       };
