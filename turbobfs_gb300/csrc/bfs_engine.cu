@@ -1443,11 +1443,6 @@ __global__ void __launch_bounds__(SHORT ? kShortBlock : kBlock, 1)
       if (first < qn) run_short_item<SIG>(p, d, A, first, max_ept, nx, bm_next, win, ovf);
     }
     while (item < n_all) {
-      /* the next item: static, or claimed now and looked at when this one is
-       * done */
-      unsigned nxt = item + nwarps;
-      const bool claim = nxt >= n_static;
-      if (claim && n_all > n_static && lane == 0) nxt = n_static + atomicAdd(wctr, 1u);
       if (dir == DIR_TD) {
         run_expand_item<SIG>(p, d, A, item, nx, bm_next, win, ovf);
       } else if (item < n_seg) {
@@ -1465,8 +1460,17 @@ __global__ void __launch_bounds__(SHORT ? kShortBlock : kBlock, 1)
           pull_range<false>(p, fd, C, dst, v, e < p.n ? e : p.n, win, ovf);
         }
       }
-      if (claim && n_all <= n_static) break;
-      item = claim ? __shfl_sync(FULL, nxt, 0) : nxt;
+      /* The next item: static, or claimed once this one is done.  Claimed beside
+       * it, the counter's round trip is hidden, but a warp that is slow with its
+       * item keeps the next one from the others, and a level has one to four items
+       * per warp (us, claimed beside / after: depths bottom-up on Erdos-Renyi of
+       * 2 M of 6 689 / 573, RMAT-22 423 / 417, top-down 1616 / 1547). */
+      item += nwarps;
+      if (item >= n_static) {
+        if (n_all <= n_static) break;
+        if (lane == 0) item = n_static + atomicAdd(wctr, 1u);
+        item = __shfl_sync(FULL, item, 0);
+      }
     }
     if (dir == DIR_BU) {
       const unsigned fn = __reduce_add_sync(FULL, fd.n), fe = __reduce_add_sync(FULL, fd.e);
