@@ -119,9 +119,18 @@ constexpr float kHeavyShare = 0.25f; /* ... and of all entries: else words of
 /* entries per frontier vertex from which a frontier filter pays: every CTA
  * reads the whole queue to fill its own */
 constexpr float kFilterGain = 300.0f;
-/* what leaving bottom-up costs a traversal with path counts besides a pass over
- * the depths (a barrier and the round trips around it), in list entries */
-constexpr float kLeaveCost = 4e5f;
+/* Leaving bottom-up with path counts, in list entries (~270 K take a
+ * microsecond): a bottom-up level reads every vertex's depth and no queue, which
+ * together cost more than a top-down one by kScanVertex per vertex less
+ * kQueueCost (narrow levels: plus kNarrowGain); leaving costs one pass over the
+ * depths, that collects the queue, and kLeaveCost.  A level's excess alone seldom
+ * pays for that, but the tail of a deep graph has many: they are added up, and
+ * the traversal leaves once they would have.  (RMAT of 2^22 and a chain of 2000,
+ * us per level of the chain: 13.9 bottom-up, 7.5 top-down, RMAT of 2^20 8.3 and
+ * 7.1, of 2^16 6.4 and 6.6.  With one level's excess compared, as little as
+ * kLeaveCost unexplored entries kept every level of the tail bottom-up.) */
+constexpr float kScanVertex = 0.48f, kQueueCost = 1.8e5f, kNarrowGain = 9e5f;
+constexpr float kLeaveCost = 2.2e5f;
 
 /* Shared memory of a warp that expands: a window of queue entries. */
 struct ExpandWin {
@@ -1289,6 +1298,7 @@ __global__ void __launch_bounds__(SHORT ? kShortBlock : kBlock, 1)
    * is not waited for); so do pushes once an overflow has been recorded,
    * since the flag is per traversal. */
   int sig_bits = 1;
+  float excess = 0.0f; /* of bottom-up levels over top-down ones, in list entries */
   for (;;) {
     const unsigned long long cur = __ldcg(&ctl->qctr[d % 3]);
     /* read with the counter, so that both loads are in flight together */
@@ -1334,12 +1344,21 @@ __global__ void __launch_bounds__(SHORT ? kShortBlock : kBlock, 1)
        * to bottom-up levels three times as costly as top-down ones */
       dir = DIR_BU;
     } else if (dir == DIR_BU) {
-      /* leave when a bottom-up level costs more than the top-down one and
-       * the pass that collects its queue, unless the frontier is large */
-      if ((float)qn * p.beta <= (float)p.n &&
-          (!want_sigma || (float)qe * alpha + kLeaveCost < (float)m_u))
-        dir = DIR_TD;
+      /* leave unless the frontier is large; with path counts when the bottom-up
+       * levels cost more, summed up, than top-down ones and the pass that
+       * collects the queue */
+      if ((float)qn * p.beta <= (float)p.n) {
+        if (want_sigma) {
+          const float scan = kScanVertex * (float)p.n;
+          const float fixed = SHORT && p.narrow ? kNarrowGain : -kQueueCost;
+          excess = fmaxf(0.0f, excess + (float)m_u + scan + fixed - (float)qe * alpha);
+          if (excess > kLeaveCost + kQueueCost + fixed + scan) dir = DIR_TD;
+        } else {
+          dir = DIR_TD;
+        }
+      }
     }
+    if (dir == DIR_TD) excess = 0.0f;
     if (gtid == 0 && p.trace && d < p.trace_cap - 1) {
       long long *rec = p.trace + 4 * (long long)d;
       rec[0] = (long long)global_ns();
