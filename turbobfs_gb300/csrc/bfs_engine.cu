@@ -95,6 +95,7 @@ constexpr int kBlock = 1024;       /* threads of a full CTA, one CTA per SM */
  * barrier's acquire drops L1, so a spilled value costs a round trip to L2) */
 constexpr int kShortBlock = 512;
 constexpr long long kLargeEntries = 48 << 20;
+constexpr int kLargeVertices = 400000;
 constexpr int kBlockStep = 256;    /* threads per unit of ctas_per_sm */
 constexpr int kFilterBits = 1 << 18; /* frontier filter in shared memory (32 KB) */
 constexpr int kWin = 128;          /* queue entries staged per warp window */
@@ -1606,7 +1607,9 @@ cudaError_t bfs_geometry(int device, LaunchGeom *out) {
     const void *fn = bfs_kernel((k & 1) != 0, (k & 2) != 0);
     const int most = (k & 1) ? kShortBlock : kBlock;
     const size_t need = bfs_smem(most, k == 2);
-    const int carve = (int)((100 * (need + sizeof(NarrowState) + 1024) + (size_t)smem_sm - 1) / (size_t)smem_sm);
+    /* without the filter: a launch with one takes its part of L1 */
+    const size_t held = bfs_smem(most, false) + sizeof(NarrowState) + 1024;
+    const int carve = (int)((100 * held + (size_t)smem_sm - 1) / (size_t)smem_sm);
     e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need);
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout,
@@ -1637,24 +1640,29 @@ static unsigned narrow_limit(const BfsParams &p, int grid) {
 
 cudaError_t bfs_launch(const BfsParams &p0, const LaunchGeom &g, cudaStream_t s) {
   /* One CTA per SM, of 256 threads per unit of ctas_per_sm.  By default (and at
-   * most) 2 on short-list graphs, whose levels are many and small; 4 for depths only and
-   * on large graphs regrouped by degree, whose heavy levels want every warp;
-   * else 3, which leaves more L1 and costs less at every barrier (ms per BFS
-   * with path counts at 3 / 4: RMAT-22 0.487 / 0.445, Erdos-Renyi of 2.5 M
-   * vertices 0.366 / 0.392, of 300 K 0.073 / 0.083, RMAT of 100 K 0.058 /
-   * 0.065). */
+   * most) 2 on short-list graphs, whose levels are many and small; 4 for depths
+   * only and bottom-up levels, if only possible ones from kLargeVertices, which
+   * want every warp; else 3, which leaves more L1 and costs less at every barrier (us
+   * per BFS with path counts at 3 / 4: RMAT 2^17 of 16 57 / 61, 2^18 of 16 67 /
+   * 71, of 32 106 / 110, 2^19 of 8 98 / 93, of 24 98 / 88, 2^20 of 16 137 / 129,
+   * 2^21 of 16 191 / 184, 2^22 of 32 468 / 417; Erdos-Renyi of 300 K of 30 81 / 85,
+   * of 2 M of 20 257 / 255; bottom-up only, directed, 1 M of 8 538 / 487). */
   BfsParams p = p0;
   /* bottom-up levels alone, large ones, want threads, not the short-list
    * instance's registers (grid of 2048 x 2048: 32 / 28 us per level, depths) */
   const bool pulls = p.mode == TBFS_MODE_BOTTOM_UP && p.n > 1 << 20;
   const bool short_lists = p.short_lists != 0 && !pulls;
   const bool sigma = p.sigma != nullptr;
-  const bool full = !sigma || pulls || (p.inv && p.nnz > kLargeEntries);
+  const bool full = !sigma || p.mode == TBFS_MODE_BOTTOM_UP ||
+                    (p.mode == TBFS_MODE_AUTO && p.n > kLargeVertices);
   const int want = p.ctas_per_sm > 0 ? p.ctas_per_sm : short_lists ? 2 : full ? 4 : 3;
   int block = want < g.per_sm ? kBlockStep * want : g.block;
   if (short_lists && block > kShortBlock) block = kShortBlock;
   p.narrow = short_lists ? narrow_limit(p, g.grid) : 0u;
-  p.filter = !short_lists && sigma && p.tile && (double)p.nnz > kHeavyEntries;
+  /* The frontier filter pays where the gathers it saves miss L1 even so: its 32
+   * KB come off that.  (us per BFS with / without: RMAT 2^18 of 24 87 / 82, 2^19
+   * of 8 97 / 92, 2^20 of 16 137 / 134, 2^21 of 16 191 / 189, of 32 218 / 224.) */
+  p.filter = !short_lists && sigma && p.tile && p.nnz > kLargeEntries;
   void *args[] = {&p};
   return cudaLaunchCooperativeKernel(bfs_kernel(short_lists, sigma), dim3(g.grid), dim3(block), args,
                                      bfs_smem(block, p.filter), s);
