@@ -1285,7 +1285,7 @@ __global__ void __launch_bounds__(SHORT ? kShortBlock : kBlock, 1)
     const unsigned deg = (unsigned)(__ldg(p.rp + root + 1) - a);
     ctl->qctr[0] = (1ull << 32) | deg;
   }
-  if (!grid_barrier(ctl, p.timeout_ns, -1)) return;
+  const bool started = grid_barrier(ctl, p.timeout_ns, -1);
 
   int d = 0, dir = DIR_TD, td = 0, bu = 0;
   long long m_u = p.out_edges_total, visited = 0, edges = 0;
@@ -1300,7 +1300,7 @@ __global__ void __launch_bounds__(SHORT ? kShortBlock : kBlock, 1)
    * since the flag is per traversal. */
   int sig_bits = 1;
   float excess = 0.0f; /* of bottom-up levels over top-down ones, in list entries */
-  for (;;) {
+  while (started) {
     const unsigned long long cur = __ldcg(&ctl->qctr[d % 3]);
     /* read with the counter, so that both loads are in flight together */
     const bool ovf_seen = want_sigma && __ldcg(&ctl->sigma_overflow) != 0;
@@ -1315,7 +1315,6 @@ __global__ void __launch_bounds__(SHORT ? kShortBlock : kBlock, 1)
           qe <= kNarrowEdges / 2u) {
         LevelState l = {d, td, sig_bits, m_u, visited, edges};
         const NarrowEnd end = narrow_levels<SIG>(p, *narrow, l, qn, qe, ovf);
-        if (end == NARROW_INJECTED) return;
         d = l.d;
         td = l.td;
         sig_bits = l.sig_bits;
@@ -1497,7 +1496,7 @@ __global__ void __launch_bounds__(SHORT ? kShortBlock : kBlock, 1)
       if (lane == 0 && fn) atomicAdd(nx.ctr, ((unsigned long long)fn << 32) | fe);
     }
     /* test hook: CTA 0 leaves without arriving; the others' waits expire */
-    if (p.inject_barrier_skip > 0 && blockIdx.x == 0 && d == p.inject_barrier_skip - 1) return;
+    if (p.inject_barrier_skip > 0 && blockIdx.x == 0 && d == p.inject_barrier_skip - 1) break;
     if (want_sigma) { /* overflow recorded now: seen by every CTA after the barrier */
       const bool any_ovf = __any_sync(FULL, ovf);
       if (any_ovf && (threadIdx.x & 31) == 0) atomicOr(&ctl->sigma_overflow, 1);
@@ -1511,7 +1510,9 @@ __global__ void __launch_bounds__(SHORT ? kShortBlock : kBlock, 1)
    * into the caller's numbering, kOut vertices per thread and round so that
    * their dependent loads (id, depth, count of the depth's parity) overlap;
    * coalesced stores.  Otherwise: counts of odd depths join the others, and
-   * kNoList becomes -1. */
+   * kNoList becomes -1, also when the traversal was given up and the arrays are
+   * the caller's (a CTA still in the last level sees an unvisited vertex with an
+   * empty list). */
   constexpr int kOut = 4;
   if (done && p.perm) {
     for (unsigned i0 = gtid; i0 < (unsigned)p.n; i0 += kOut * nthreads) {
@@ -1538,7 +1539,7 @@ __global__ void __launch_bounds__(SHORT ? kShortBlock : kBlock, 1)
         }
       }
     }
-  } else if (done && want_sigma) {
+  } else if (!p.perm && want_sigma) {
     for (unsigned i0 = gtid; i0 < (unsigned)p.n; i0 += kOut * nthreads) {
       bool odd[kOut];
       unsigned long long x[kOut];
