@@ -68,31 +68,47 @@ __global__ void degree_profile_kernel(const int *cp, int n, unsigned long long *
 }
 
 /* tile[i] = first vertex v with ptr[v] + kTileVertex * v >= i * kTileCost, for
- * i <= tiles (n where there is none) */
+ * i <= tiles (n where there is none).  Each by its own search: with a thread per
+ * vertex that wrote the pieces beginning at it, one thread wrote all of a hub's
+ * list (a star of 2^20 vertices: 75 us). */
 __global__ void tile_kernel(const int *ptr, int n, int tiles, int *tile) {
-  for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v <= n;
-       v += (long long)gridDim.x * blockDim.x) {
-    const long long at = ptr[v] + (long long)kTileVertex * v;
-    const long long before = v > 0 ? ptr[v - 1] + (long long)kTileVertex * (v - 1) : -1;
-    long long i = before < 0 ? 0 : before / kTileCost + 1;
-    for (; i <= tiles && i * kTileCost <= at; ++i) tile[i] = (int)v;
-    if (v == n)
-      for (; i <= tiles; ++i) tile[i] = n;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i <= tiles;
+       i += (long long)gridDim.x * blockDim.x) {
+    const long long want = i * kTileCost;
+    int lo = 0, hi = n;
+    while (lo < hi) {
+      const int mid = lo + ((hi - lo) >> 1);
+      if (__ldg(ptr + mid) + (long long)kTileVertex * mid < want) lo = mid + 1;
+      else hi = mid;
+    }
+    tile[i] = lo;
   }
 }
 
 /* (list, first entry) of every kHubLen-entry segment of the lists longer
  * than that */
 __global__ void hub_segments_kernel(const int *ptr, int n, int *count, int *seg) {
-  for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n;
-       v += (long long)gridDim.x * blockDim.x) {
-    const int b = ptr[v], len = ptr[v + 1] - b;
-    if (len <= kHubLen) continue;
-    const int k = (len + kHubLen - 1) / kHubLen;
-    const int at = atomicAdd(count, k);
-    for (int j = 0; j < k; ++j) {
-      seg[2 * (at + j)] = (int)v;
-      seg[2 * (at + j) + 1] = b + j * kHubLen;
+  const int lane = threadIdx.x & 31;
+  for (long long v0 = (long long)blockIdx.x * blockDim.x + threadIdx.x - lane; v0 < n;
+       v0 += (long long)gridDim.x * blockDim.x) {
+    const long long v = v0 + lane;
+    int b = 0, k = 0, at = 0;
+    if (v < n) {
+      b = ptr[v];
+      const int len = ptr[v + 1] - b;
+      if (len > kHubLen) {
+        k = (len + kHubLen - 1) / kHubLen;
+        at = atomicAdd(count, k);
+      }
+    }
+    for (unsigned m = __ballot_sync(0xffffffffu, k > 0); m; m &= m - 1u) {
+      const int l = __ffs(m) - 1; /* the warp writes one list's segments */
+      const int bl = __shfl_sync(0xffffffffu, b, l), kl = __shfl_sync(0xffffffffu, k, l);
+      const int al = __shfl_sync(0xffffffffu, at, l);
+      for (int j = lane; j < kl; j += 32) {
+        seg[2 * (al + j)] = (int)v0 + l;
+        seg[2 * (al + j) + 1] = bl + j * kHubLen;
+      }
     }
   }
 }
@@ -239,7 +255,7 @@ cudaError_t longest_list(const int *ptr, int n, int *out) {
 
 cudaError_t fill_tiles(const int *ptr, int n, int64_t nnz, int *tile, cudaStream_t s) {
   const int tiles = (int)tile_count(n, nnz);
-  const int blocks = (int)std::min<long long>(((long long)n + 255) / 256, 4096);
+  const int blocks = std::min(tiles / 256 + 1, 4096);
   tile_kernel<<<blocks, 256, 0, s>>>(ptr, n, tiles, tile);
   return cudaGetLastError();
 }
