@@ -80,10 +80,12 @@ typedef struct tbfs_options {
    * paths in the pass that finds it. */
   float pull_ratio;
   /* Engine shape of the single-source traversal (tbfs_autotune sets both):
-   * the most list entries a lane handles per round of a push or pull (1..6;
-   * 0 = 6), and units of 256 threads per SM of the persistent launch (1..4;
-   * 0 = 3, 4 on large graphs regrouped by degree; 2, at most, on graphs without
-   * long out-lists: 16 entries, 64 on smaller graphs). */
+   * the most list entries a lane handles per round of a top-down level (1..6;
+   * 0 = 6; no effect on bottom-up levels, nor on the narrow levels of graphs
+   * without long out-lists), and units of 256 threads per SM of the persistent
+   * launch (1..4; 0 = 3, or 4 for depths only, bottom-up only and, AUTO, from
+   * 400 K vertices; 2, at most, on graphs without long out-lists: 16 entries, 64
+   * on smaller graphs). */
   int32_t max_ept;
   int32_t ctas_per_sm;
 } tbfs_options;
@@ -357,6 +359,8 @@ tbfs_status tbfs_server_submit(tbfs_server *s, tbfs_graph *g, int32_t root, int3
                                int64_t *sigma, uint64_t *ticket);
 tbfs_status tbfs_server_wait(tbfs_server *s, uint64_t ticket, tbfs_stats *stats,
                              double *latency_ms);
+/* Launches of the multi-instance engine so far; levels: for every launch, the
+ * most levels that it took any one query on, summed; completed queries. */
 tbfs_status tbfs_server_counters(tbfs_server *s, int64_t *launches, int64_t *levels,
                                  int64_t *completed);
 /* Where the server's time went (host wall clock, ms, cumulative): its

@@ -55,9 +55,11 @@
  * "Direction-optimizing breadth-first search", SC 2012): a level runs
  * bottom-up when alpha times the frontier's out-edges exceed the unexplored
  * edges plus the cost of visiting every vertex's word; a frontier of more
- * than n/beta vertices does not leave bottom-up.  The comparisons are in fp32:
- * every thread evaluates them at every level, and fp64 issues slowly on
- * this part (in fp64 they cost about 0.7 us per level).
+ * than n/beta vertices does not leave bottom-up, a smaller one does at once
+ * without path counts, and with them when the levels' excess has paid for it
+ * (kLeaveCost).  The comparisons are in fp32: every thread evaluates them at
+ * every level, and fp64 issues slowly on this part (in fp64 they cost about 0.7
+ * us per level).
  *
  * Memory model.  Queues and counters are read with ld.global.cg (L2).
  * Depth and path-count gathers use ordinary (L1-cacheable) loads: every
@@ -94,8 +96,9 @@ constexpr int kBlock = 1024;       /* threads of a full CTA, one CTA per SM */
 /* ... on short-list graphs: levels that are latency alone want registers (a
  * barrier's acquire drops L1, so a spilled value costs a round trip to L2) */
 constexpr int kShortBlock = 512;
-constexpr long long kLargeEntries = 48 << 20;
-constexpr int kLargeVertices = 400000;
+constexpr long long kLargeEntries = 48 << 20; /* list entries from which a frontier
+                                                 filter is used (bfs_launch) */
+constexpr int kLargeVertices = 400000; /* vertices from which AUTO takes all threads */
 constexpr int kBlockStep = 256;    /* threads per unit of ctas_per_sm */
 constexpr int kFilterBits = 1 << 18; /* frontier filter in shared memory (32 KB) */
 constexpr int kWin = 128;          /* queue entries staged per warp window */

@@ -30,7 +30,8 @@
  * run by that CTA alone, level after level, with its queue in shared memory
  * and no grid barrier (local_run), while the other CTAs advance the wide
  * instances.  A phase is then one level of every wide instance and as many
- * of the others as fit in its time.
+ * of the others as fit in its time.  Launches with a large instance run a kernel
+ * without that (multi_local).
  */
 #include <cuda_runtime.h>
 #include <stdint.h>

@@ -278,7 +278,7 @@ void batch_ws_free(BatchWS *ws);
 /* ---- multi-instance engine (multi_engine.cu) ----
  * One descriptor per traversal (graph, root); the kernel advances every
  * unfinished descriptor by one level per phase, by as many as the phase has
- * time for if one CTA can run it alone. */
+ * time for if one CTA can run it alone (launches without large instances). */
 constexpr int kMultiMaxSlots = 1024;
 
 struct InstDesc {
