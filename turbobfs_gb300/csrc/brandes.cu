@@ -572,7 +572,7 @@ extern "C" tbfs_status tbfs_brandes(tbfs_graph *g, const int32_t *roots, int32_t
   BTRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, tbfs::sweep_kernel, tbfs::kBlock, 0),
        "occupancy");
 #ifndef TBFS_SWEEP_PER_SM
-#define TBFS_SWEEP_PER_SM 4 /* 32 registers: 4 CTAs of 256 per SM measured 11 % faster than 2 */
+#define TBFS_SWEEP_PER_SM 4 /* 4 CTAs of 256 per SM measured 11 % faster than 2 */
 #endif
   if (per > TBFS_SWEEP_PER_SM) per = TBFS_SWEEP_PER_SM;
   const unsigned grid = (unsigned)(sms * (per > 0 ? per : 1));
