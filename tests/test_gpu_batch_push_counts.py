@@ -1,7 +1,7 @@
-"""Push levels of a batch whose counts are added along the level's own edges:
-the new vertices are finished, with counts of 0, in a phase before, one to
-several rounds of them per item, for every row width, against the exact
-oracle."""
+"""Push levels of a batch whose counts are added along the level's own edges: the
+new vertices' counts start at 0, written with the discovery at the first level
+and in a phase of its own (one to several rounds of vertices per item) at later
+ones, for every row width, against the exact oracle."""
 import numpy as np
 import pytest
 
@@ -13,27 +13,32 @@ pytestmark = pytest.mark.gpu
 
 
 def wide_fan(fan, out, feeders):
-    """0 and 1 -> fan vertices, each with `out` edges into a second layer of
+    """2 -> 0 and 1 -> fan vertices, each with `out` edges into a second layer of
     fan // 3, and `feeders` vertices that nothing leads to with an edge to each of
     the fan's first: long in-lists there, few edges that find them."""
-    v = 2 + np.arange(fan)
-    second = 2 + fan + np.arange(fan // 3)
+    v = 3 + np.arange(fan)
+    second = 3 + fan + np.arange(fan // 3)
     rng = np.random.default_rng(fan)
-    feed = 2 + fan + fan // 3 + np.arange(feeders)
-    src = [np.zeros(fan, np.int64), np.ones(fan // 2, np.int64), np.repeat(v, out),
-           np.repeat(feed, 40)]
-    dst = [v, v[:fan // 2], second[rng.integers(0, fan // 3, fan * out)],
+    feed = 3 + fan + fan // 3 + np.arange(feeders)
+    src = [np.array([2, 2]), np.zeros(fan, np.int64), np.ones(fan // 2, np.int64),
+           np.repeat(v, out), np.repeat(feed, 40)]
+    dst = [np.array([0, 1]), v, v[:fan // 2], second[rng.integers(0, fan // 3, fan * out)],
            np.tile(v[:40], feeders)]
-    return graphs.from_edges(2 + fan + fan // 3 + feeders, np.concatenate(src), np.concatenate(dst))
+    return graphs.from_edges(3 + fan + fan // 3 + feeders, np.concatenate(src), np.concatenate(dst))
 
 
-@pytest.mark.parametrize("k", [2, 33, 70, 200])  # rows of 1, 2, 4 and 8 words
+@pytest.mark.parametrize("k", [3, 33, 70, 200])  # rows of 1, 2, 4 and 8 words
 @pytest.mark.parametrize("fan", [50, 1000, 30000, 130000])
-def test_counts_along_edges(gpu_available, fan, k):
+@pytest.mark.parametrize("level", ["first", "later"])
+def test_counts_along_edges(gpu_available, level, fan, k):
     h = wide_fan(fan, 12, 3000)
     rng = np.random.default_rng(k)
-    roots = np.concatenate([[0, 1], rng.integers(0, h.n, k - 2)]).astype(np.int32)
-    pick = [0, 1] + list(range(2, k, 13))
+    if level == "first":
+        roots = np.concatenate([[0, 1, 2], rng.integers(0, h.n, k - 3)])
+    else:  # the others lead nowhere: the fan is found at the second level
+        roots = np.concatenate([[2, 2, 2], 3 + fan + rng.integers(0, fan // 3, k - 3)])
+    roots = roots.astype(np.int32)
+    pick = [0, 1, 2] + list(range(3, k, 13))
     want = {i: oracle.exact_bfs(h.col_ptr, h.row_idx, int(roots[i])) for i in pick}
     with tb.Graph.from_host_csc(h) as g:
         for mode in ("td", "auto"):

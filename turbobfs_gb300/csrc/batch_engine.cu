@@ -957,6 +957,7 @@ __global__ void __launch_bounds__(kBlock, TBFS_BATCH_MINB) fm_bfs_kernel(const B
 
     if (push) {
       /* ---- phase 1: discovery over the out-edges of Q_d ---- */
+      const bool zero_now = by_push && d == 0; /* see phase 2 */
       /* rounds of an item: few on small levels, which have items for few warps */
       const unsigned rounds =
           qe <= 32u * nwarps
@@ -1018,8 +1019,18 @@ __global__ void __launch_bounds__(kBlock, TBFS_BATCH_MINB) fm_bfs_kernel(const B
             for (int w = 0; w < W; ++w) {
               const unsigned m = fr[w] & ~sv[w];
               if (m) {
-                atomicOr(&F1[(size_t)v * W + w], m);
                 any = true;
+                if (SIG && zero_now) { /* depth and a count of 0, once, for each new root */
+                  unsigned nw = m & ~atomicOr(&F1[(size_t)v * W + w], m);
+                  for (; nw; nw &= nw - 1u) {
+                    const size_t at = (size_t)v * RS + root_of_bit(32 * w + __ffs(nw) - 1, W);
+                    p.S_int[at] = d + 1;
+                    if (SIG == 2) reinterpret_cast<unsigned *>(p.sig_int)[at] = 0u;
+                    else p.sig_int[at] = 0ull;
+                  }
+                } else {
+                  atomicOr(&F1[(size_t)v * W + w], m);
+                }
               }
             }
             if (any) {
@@ -1055,47 +1066,54 @@ __global__ void __launch_bounds__(kBlock, TBFS_BATCH_MINB) fm_bfs_kernel(const B
       if (SIG && by_push && (float)qe1 + (float)kVCost * (float)qn1 > kPullBack * (float)qe) {
         /* The edges of phase 1 again: each adds its source's counts to its
          * target's.  In the first levels of a batch few edges find vertices with
-         * long in-lists (255 roots on RMAT-20: 0.53 M edges, 27.7 M entries): 517
-         * -> 139 us; 98 roots on RMAT of 100 K 76 -> 26.  Before, in a phase of its
-         * own, the new vertices are finished, their new roots with a count of 0.
-         * (With those written in phase 1 by the lanes whose bits were new, there is
-         * one barrier less, but every push level of a graph with hubs waits for
-         * the bits' old values: a chain of 1000 behind RMAT of 64 K, 64 roots, 11.8
-         * -> 14.8 ms.) */
-        const unsigned iv = PER * min(max(qn1 / (2u * PER * nwarps), 1u), 8u);
-        const unsigned nF = (qn1 + iv - 1u) / iv;
+         * long in-lists (255 roots on RMAT-20: 0.53 M edges, 27.7 M entries): 528
+         * -> 141 us; 98 roots on RMAT of 100 K 92 -> 28.  The new roots' counts
+         * are 0 before: written in phase 1 by the lanes whose bits were new at the
+         * first level, which is nearly always such a one; later, where few are and
+         * every push level would wait for the bits' old values (a chain of 1000
+         * behind RMAT of 64 K, 64 roots, 11.8 -> 14.8 ms), in a phase of its own. */
+        if (!zero_now) {
+          const unsigned iv = PER * min(max(qn1 / (2u * PER * nwarps), 1u), 8u);
+          const unsigned nZ = (qn1 + iv - 1u) / iv;
+          if (tid == 0) ctl->work[(ph + 2) & 3u] = 0u;
+          first_claim = true;
+          for (;;) {
+            const unsigned it = claim(nZ);
+            if (it >= nZ) break;
+            for (unsigned base = it * iv; base < qn1 && base < (it + 1u) * iv; base += PER) {
+              if (base + g.gid >= qn1) continue;
+              const int v = __ldcg(p.q[b1] + base + g.gid);
+              unsigned f1[W];
+              load_row<W>(F1 + (size_t)v * W, f1);
+              const unsigned long long none[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+              write_new<W, SIG>(p, d, v, lane_bits<W>(f1, g), none, g);
+            }
+          }
+          if (!grid_barrier(ctl, p.timeout_ns, d)) return;
+          ++ph;
+        }
+        /* and the new vertices are finished, 32 at a time */
+        const unsigned nF = (qn1 + 31u) / 32u;
         if (tid == 0) ctl->work[(ph + 2) & 3u] = 0u;
         first_claim = true;
         for (;;) {
-          const unsigned it = claim(nF);
-          if (it >= nF) break;
-          for (unsigned base = it * iv; base < qn1 && base < (it + 1u) * iv; base += PER) {
-            const unsigned idx = base + g.gid;
+          const unsigned it = claim(nA + nF);
+          if (it >= nA + nF) break;
+          if (it >= nA) {
+            const unsigned idx = (it - nA) * 32u + g.lane;
             if (idx < qn1) {
               const int v = __ldcg(p.q[b1] + idx);
               unsigned f1[W], sn[W];
               load_row<W>(F1 + (size_t)v * W, f1);
               load_row<W>(p.seen + (size_t)v * W, sn);
-              const unsigned long long none[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-              write_new<W, SIG>(p, d, v, lane_bits<W>(f1, g), none, g);
-              if (g.gl < W) {
-                const unsigned nw = pick<W>(f1, g.gl);
-                if (nw) p.seen[(size_t)v * W + g.gl] = pick<W>(sn, g.gl) | nw;
-              }
-              if (g.gl == 0) {
-                atomicAnd(&p.touched[v >> 5], ~(1u << (v & 31)));
-                if (row_full<W>(p, sn, f1)) md += (unsigned)(__ldg(p.cp + v + 1) - __ldg(p.cp + v));
-              }
+#pragma unroll
+              for (int w = 0; w < W; ++w) sn[w] |= f1[w];
+              store_row<W>(p.seen + (size_t)v * W, sn);
+              atomicAnd(&p.touched[v >> 5], ~(1u << (v & 31)));
+              if (row_full<W>(p, sn, f1)) md += (unsigned)(__ldg(p.cp + v + 1) - __ldg(p.cp + v));
             }
+            continue;
           }
-        }
-        if (!grid_barrier(ctl, p.timeout_ns, d)) return;
-        ++ph;
-        if (tid == 0) ctl->work[(ph + 2) & 3u] = 0u;
-        first_claim = true;
-        for (;;) {
-          const unsigned it = claim(nA);
-          if (it >= nA) break;
           push_edges(it, [&](bool valid, int u, int v) {
             if (!valid) return;
             unsigned fr[W], f1[W];
